@@ -893,14 +893,49 @@ __global__ void k_copy_direct(WaveArgs a, const float4* __restrict__ rad,
     direct[a.pix0 + p] = rad[p];
 }
 
-template <class T>
-T* carve(char*& cur, uint64_t count) {
-  T* p = reinterpret_cast<T*>(cur);
-  cur += ((count * sizeof(T) + 255) / 256) * 256;
-  return p;
+}  // namespace
+
+cudaError_t Scratch::take(ajg_ctx* ctx, uint64_t bytes, cudaStream_t st) {
+  bytes = std::max<uint64_t>(bytes, 16);
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(st, &cap);
+  if (bytes > kScratchKeep || cap != cudaStreamCaptureStatusNone) {
+    const cudaError_t e = cudaMallocAsync((void**)&p, bytes, st);
+    own = st;
+    owned = e == cudaSuccess;
+    return e;
+  }
+  if (ctx->scratch.bytes < bytes) {
+    scratch_drop(ctx);
+    const uint64_t want = std::max<uint64_t>(bytes, 8ull << 20);
+    const cudaError_t e = cudaMalloc(&ctx->scratch.ptr, want);
+    if (e != cudaSuccess) {
+      ctx->scratch = Buffer{};
+      cudaGetLastError();
+      return e;
+    }
+    ctx->scratch.bytes = want;
+  }
+  p = static_cast<char*>(ctx->scratch.ptr);
+  return cudaSuccess;
 }
 
-}  // namespace
+bool scratch_drop(ajg_ctx* ctx) {
+  if (!ctx->scratch.ptr) return false;
+  cudaStreamSynchronize(ctx->stream);
+  cudaFree(ctx->scratch.ptr);
+  ctx->scratch = Buffer{};
+  return true;
+}
+
+bool device_malloc(ajg_ctx* ctx, void** p, uint64_t bytes) {
+  if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+  cudaGetLastError();
+  if (scratch_drop(ctx) && cudaMalloc(p, bytes) == cudaSuccess) return true;
+  cudaGetLastError();
+  *p = nullptr;
+  return false;
+}
 
 int resident_grid(const void* fn, int threads) {
   static std::mutex mu;
@@ -981,7 +1016,7 @@ static int ensure_arena(ajg_ctx* ctx, uint64_t P, int nt, char** base) {
     for (auto& b : ctx->arena) cudaFree(b.ptr);
     ctx->arena.clear();
     Buffer b;
-    if (cudaMalloc(&b.ptr, need) != cudaSuccess)
+    if (!device_malloc(ctx, &b.ptr, need))
       return fail(ctx, AJG_ERR_OOM, "device allocation failed (wave arena)");
     b.bytes = need;
     ctx->arena.push_back(b);
@@ -1405,8 +1440,18 @@ void enqueue_resolve(const float4* fsum, const float4* fcomp,
       fsum, fcomp, fsum64, w, h, fold_x ? 1 : 0, fold_y ? 1 : 0, out);
 }
 
+int reserve_wave(ajg_scene* sc, const ajg_camera& cam,
+                 const ajg_render_params& prm, uint64_t npix) {
+  int rc = check_render(sc->ctx, sc->d, cam, prm);
+  if (rc) return rc;
+  const int nt = (int)sc->d.num_lights + 1;
+  char* base = nullptr;
+  return ensure_arena(sc->ctx, job_wave_paths(sc->ctx, npix * prm.spp, nt), nt,
+                      &base);
+}
+
 int render_impl(ajg_scene* sc, const ajg_camera& cam,
-                const ajg_render_params& prm, float4* d_out,
+                const ajg_render_params& prm, float4* d_out, void* film,
                 uint64_t li_begin, uint64_t li_end, float* d_li,
                 cudaStream_t st) {
   ajg_ctx* ctx = sc->ctx;
@@ -1424,25 +1469,19 @@ int render_impl(ajg_scene* sc, const ajg_camera& cam,
 
   // film accumulators: per pixel a float32 sum and Kahan compensation, or a
   // float64 sum
-  const bool fp64 = (prm.flags & AJG_RENDER_FP64_FILM) != 0;
   float4 *fsum = nullptr, *fcomp = nullptr;
   double* fsum64 = nullptr;
   if (d_out) {
-    if (fp64) {
-      if (cudaMallocAsync((void**)&fsum64, npix_all * 32, st) != cudaSuccess)
-        return fail(ctx, AJG_ERR_OOM, "device allocation failed (film)");
-      cudaMemsetAsync(fsum64, 0, npix_all * 32, st);
+    if (prm.flags & AJG_RENDER_FP64_FILM) {
+      fsum64 = static_cast<double*>(film);
     } else {
-      if (cudaMallocAsync((void**)&fsum, npix_all * 32, st) != cudaSuccess)
-        return fail(ctx, AJG_ERR_OOM, "device allocation failed (film)");
+      fsum = static_cast<float4*>(film);
       fcomp = fsum + npix_all;
-      cudaMemsetAsync(fsum, 0, npix_all * 32, st);
     }
+    cudaMemsetAsync(film, 0, npix_all * 32, st);
   }
   run_waves(sc, cam, prm, w, P, fsum, fcomp, fsum64, d_out, li_begin, li_end,
             d_li, st, true);
-  if (fsum) cudaFreeAsync(fsum, st);
-  if (fsum64) cudaFreeAsync(fsum64, st);
   return AJG_OK;
 }
 
@@ -1483,12 +1522,9 @@ int render_in_scratch(ajg_scene* sc, const ajg_camera& cam,
   return AJG_OK;
 }
 
-int sppm_camera_pass(ajg_scene* sc, const ajg_camera& cam, int fmd,
-                     uint64_t seed, VisPointD* vp, float4* direct,
-                     cudaStream_t st) {
-  ajg_ctx* ctx = sc->ctx;
-  // TracerVP is TraceMIS without roulette that stops at a visible point:
-  // min = max bounces = fmd, sample 0 of each pixel (SetSeed(x + y W))
+// TracerVP is TraceMIS without roulette that stops at a visible point:
+// min = max bounces = fmd, sample 0 of each pixel (SetSeed(x + y W))
+static ajg_render_params sppm_camera_params(int fmd, uint64_t seed) {
   ajg_render_params prm{};
   prm.spp = 1;
   prm.min_bounces = fmd;
@@ -1496,6 +1532,19 @@ int sppm_camera_pass(ajg_scene* sc, const ajg_camera& cam, int fmd,
   prm.cont_prob = 1.f;
   prm.use_mis = 1;
   prm.seed = seed;
+  return prm;
+}
+
+int sppm_reserve(ajg_scene* sc, const ajg_camera& cam, int fmd) {
+  return reserve_wave(sc, cam, sppm_camera_params(fmd, 0),
+                      (uint64_t)cam.width * cam.height);
+}
+
+int sppm_camera_pass(ajg_scene* sc, const ajg_camera& cam, int fmd,
+                     uint64_t seed, VisPointD* vp, float4* direct,
+                     cudaStream_t st) {
+  ajg_ctx* ctx = sc->ctx;
+  const ajg_render_params prm = sppm_camera_params(fmd, seed);
   int rc = check_render(ctx, sc->d, cam, prm);
   if (rc) return rc;
   const int nt = (int)sc->d.num_lights + 1;

@@ -756,13 +756,16 @@ __global__ void k_lum(const float* __restrict__ mats, uint32_t m,
 }
 
 struct Arena {
+  ajg_ctx* ctx;
   std::vector<void*> ptrs;
+  explicit Arena(ajg_ctx* c) : ctx(c) {}
   cudaError_t err = cudaSuccess;
   template <class T>
   T* get(uint64_t count) {
     void* p = nullptr;
     if (err != cudaSuccess) return nullptr;
-    err = cudaMalloc(&p, count * sizeof(T) > 0 ? count * sizeof(T) : 16);
+    if (!device_malloc(ctx, &p, count * sizeof(T) > 0 ? count * sizeof(T) : 16))
+      err = cudaErrorMemoryAllocation;
     if (err != cudaSuccess) return nullptr;
     ptrs.push_back(p);
     return static_cast<T*>(p);
@@ -820,7 +823,7 @@ int build_scene(ajg_ctx* ctx, ajg_scene* s, const float* h_tris,
   // persistent scene buffers
   auto keep = [&](size_t bytes) -> void* {
     void* p = nullptr;
-    if (cudaMalloc(&p, bytes > 0 ? bytes : 16) != cudaSuccess) return nullptr;
+    if (!device_malloc(ctx, &p, bytes > 0 ? bytes : 16)) return nullptr;
     s->allocations.push_back(p);
     s->info.device_bytes += bytes;
     return p;
@@ -851,7 +854,7 @@ int build_scene(ajg_ctx* ctx, ajg_scene* s, const float* h_tris,
       !ploc_nodes || !perm_keep)
     return set_err(ctx, AJG_ERR_OOM, "device allocation failed (scene)");
 
-  Arena tmp;
+  Arena tmp(ctx);
   float* d_tris = tmp.get<float>(n * 9);
   int32_t* d_mat = tmp.get<int32_t>(n);
   int32_t* d_flags = tmp.get<int32_t>(n);

@@ -288,6 +288,9 @@ struct PendingTiming {
   int64_t snap;  // the traversal counters' snapshot after it (-1: none)
 };
 constexpr int kLaunchLogCap = 65536;
+// A host ray query of at least kSplitRays rays runs in kQueryParts parts.
+constexpr int kQueryParts = 4;
+constexpr uint64_t kSplitRays = 1ull << 18;
 
 }  // namespace ajg
 
@@ -329,7 +332,9 @@ struct ajg_ctx {
   std::mutex mu;
   std::string last_error;
   uint32_t* d_error = nullptr;            // device error flag
-  uint32_t* d_fetch = nullptr;            // ray counter of query launches
+  uint32_t* h_error = nullptr;            // its pinned host copy (per call)
+  uint32_t* d_fetch = nullptr;            // [kQueryParts] ray counters of
+                                          // query launches
   ajg::TraceCounters* d_counters = nullptr;  // [2]: closest, any
   unsigned long long paths_total = 0;
   unsigned long long kernel_launches = 0;
@@ -347,6 +352,7 @@ struct ajg_ctx {
   // wavefront arena (grown on demand, reused across renders)
   std::vector<ajg::Buffer> arena;
   uint64_t arena_paths = 0;
+  ajg::Buffer scratch;  // see ajg::Scratch
 };
 
 struct ajg_scene {
@@ -364,6 +370,45 @@ struct ajg_scene {
 };
 
 namespace ajg {
+// Device scratch of one call: film accumulators, results on their way to the
+// host, query batches, SPPM state.  The context keeps one block of at most
+// kScratchKeep bytes for it, grown on demand and freed with the context: a
+// stream-ordered allocation whose memory went back to the system at the last
+// synchronisation costs about 100 us a buffer (a first 128x128 preview after
+// one: 789 -> 573 us; SPPM with 26 buffers, 10.8 -> 8.4 ms).  The block belongs to the call
+// that holds the context's mutex, and all its uses are ordered on the
+// context's stream.  A larger scratch, and one taken while the stream is
+// being captured (the graph then owns it), is allocated in stream order for
+// the call alone.
+constexpr uint64_t kScratchKeep = 4ull << 30;
+struct Scratch {
+  char* p = nullptr;
+  cudaStream_t own = nullptr;  // the stream of a scratch of its own
+  bool owned = false;
+  cudaError_t take(ajg_ctx* ctx, uint64_t bytes, cudaStream_t st);
+  Scratch() = default;
+  Scratch(const Scratch&) = delete;
+  ~Scratch() {
+    if (owned) cudaFreeAsync(p, own);
+  }
+};
+// Frees the kept block (no call may be using it: the context's mutex is
+// held, before Scratch::take); false when there is none.
+bool scratch_drop(ajg_ctx* ctx);
+// cudaMalloc, giving the kept scratch back first where memory is short
+// (conditions as for scratch_drop).
+bool device_malloc(ajg_ctx* ctx, void** p, uint64_t bytes);
+// The next `count` T of a scratch, 256-byte aligned, and their size there.
+template <class T>
+T* carve(char*& cur, uint64_t count) {
+  T* p = reinterpret_cast<T*>(cur);
+  cur += ((count * sizeof(T) + 255) / 256) * 256;
+  return p;
+}
+template <class T>
+constexpr uint64_t carve_bytes(uint64_t count) {
+  return ((count * sizeof(T) + 255) / 256) * 256;
+}
 // Brackets one launch of a given kind with events when profiling.
 struct KernelTimer {
   ajg_ctx* ctx;
@@ -469,13 +514,17 @@ int resident_grid(const void* fn, int threads);
 // SPPM's camera pass (TracerVP, sppm.cpp:35-101) through the path-tracing
 // wave: one path per pixel (sample 0), no roulette, depth `fmd`; fills
 // vp[npix] (kNoVisPoint where none) and the direct light direct[npix].
+// sppm_reserve makes its wave arena.
+int sppm_reserve(ajg_scene* sc, const ajg_camera& cam, int fmd);
 int sppm_camera_pass(ajg_scene* sc, const ajg_camera& cam, int fmd,
                      uint64_t seed, VisPointD* vp, float4* direct,
                      cudaStream_t st);
-// SPPMRenderer::Render on `st`: the footprint film (d_out, [h][w] float4, or
-// null) and ComputePixelRadiance per pixel (d_rad, [h][w][3], or null).
+// SPPMRenderer::Render on `st`: the footprint film (d_out, [h][w] float4,
+// when want_film) and ComputePixelRadiance per pixel (d_rad, [h][w][3], when
+// want_rad), both in `scratch`.
 int sppm_render(ajg_scene* sc, const ajg_camera& cam,
-                const ajg_sppm_params& p, float4* d_out, float* d_rad,
+                const ajg_sppm_params& p, bool want_film, bool want_rad,
+                Scratch& scratch, float4** d_out, float** d_rad,
                 cudaStream_t st);
 // Resolves a window-sized film into (sum rgb, sum w) per target pixel.
 void enqueue_resolve(const float4* fsum, const float4* fcomp,
@@ -485,8 +534,12 @@ int check_render(ajg_ctx* ctx, const DeviceScene& s, const ajg_camera& cam,
                  const ajg_render_params& prm);
 JobParams make_job_params(const ajg_scene* sc, const ajg_camera& cam,
                           const ajg_render_params& prm);
+// The wave arena of a render of `npix` pixels (before any scratch is taken).
+int reserve_wave(ajg_scene* sc, const ajg_camera& cam,
+                 const ajg_render_params& prm, uint64_t npix);
+// `film`: 32 bytes per pixel of accumulators (renders with d_out).
 int render_impl(ajg_scene* sc, const ajg_camera& cam,
-                const ajg_render_params& prm, float4* d_out,
+                const ajg_render_params& prm, float4* d_out, void* film,
                 uint64_t li_begin, uint64_t li_end, float* d_li,
                 cudaStream_t st);
 // The same render over caller-provided scratch (film accumulators first,

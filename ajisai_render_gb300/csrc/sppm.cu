@@ -731,24 +731,11 @@ __global__ void k_fill_f(float* p, uint64_t n, float v) {
     p[i] = v;
 }
 
-template <class T>
-struct Dev {
-  T* p = nullptr;
-  cudaStream_t s = nullptr;
-  cudaError_t alloc(uint64_t count, cudaStream_t st) {
-    s = st;
-    return cudaMallocAsync((void**)&p, std::max<uint64_t>(16, count * sizeof(T)),
-                           st);
-  }
-  ~Dev() {
-    if (p) cudaFreeAsync(p, s);
-  }
-};
-
 }  // namespace
 
 int sppm_render(ajg_scene* sc, const ajg_camera& cam, const ajg_sppm_params& p,
-                float4* d_out, float* d_rad, cudaStream_t st) {
+                bool want_film, bool want_rad, Scratch& scratch,
+                float4** out_film, float** out_rad, cudaStream_t st) {
   ajg_ctx* ctx = sc->ctx;
   const DeviceScene& s = sc->d;
   const uint64_t npix = (uint64_t)cam.width * cam.height;
@@ -801,31 +788,6 @@ int sppm_render(ajg_scene* sc, const ajg_camera& cam, const ajg_sppm_params& p,
     a.lpdf = table[0];
   }
 
-  Dev<VisPointD> vp;
-  Dev<float4> direct, phi, tau, film;
-  Dev<float> radius, N, maxr;
-  Dev<uint32_t> M, counts, offsets, cursor, items, bits;
-  Dev<float4> spheres;
-  const uint32_t cap = (uint32_t)std::min<uint64_t>(8 * npix, 0xffffffffull);
-  cudaError_t e = cudaSuccess;
-  auto A = [&](cudaError_t r) {
-    if (e == cudaSuccess) e = r;
-  };
-  A(vp.alloc(npix, st));
-  A(direct.alloc(npix, st));
-  A(phi.alloc(npix, st));
-  A(tau.alloc(npix, st));
-  A(film.alloc(2 * npix, st));
-  A(radius.alloc(npix, st));
-  A(N.alloc(npix, st));
-  A(maxr.alloc(1, st));
-  A(M.alloc(npix, st));
-  A(counts.alloc(kEntries, st));
-  A(offsets.alloc(kEntries + 1, st));
-  A(cursor.alloc(kEntries, st));
-  A(items.alloc(cap, st));
-  A(spheres.alloc(cap, st));
-  A(bits.alloc(1, st));
   // the photon queue, in equal chunks of at most the context's wave size
   // whose deposits (one per depth from 2 on) fit the record buffer
   const uint64_t dep_depths = p.photon_max_depth > 1 ? p.photon_max_depth - 1 : 0;
@@ -836,67 +798,97 @@ int sppm_render(ajg_scene* sc, const ajg_camera& cam, const ajg_sppm_params& p,
   const uint64_t n_chunks = (p.photons_per_iteration + chunk - 1) / chunk;
   if (n_chunks) chunk = (p.photons_per_iteration + n_chunks - 1) / n_chunks;
   const uint64_t dep_cap = chunk * dep_depths;
-  Dev<float4> qro, qrd, qcoef;
-  Dev<ajg_hit> qhits;
-  Dev<uint32_t> qcounts;
-  A(qro.alloc(2 * chunk, st));
-  A(qrd.alloc(2 * chunk, st));
-  A(qcoef.alloc(2 * chunk, st));
-  A(qhits.alloc(chunk, st));
   // zeroed per chunk: the depths' queue counters, the deposit count, the
   // entries' deposit counts
   const uint64_t n_counts = 2 * ((uint64_t)p.photon_max_depth + 2);
-  A(qcounts.alloc(n_counts + 1 + kEntries, st));
-  Dev<float4> drec;
-  Dev<uint32_t> doff, dsorted;
-  Dev<unsigned long long> dunits;
-  Dev<EntryVal> totals;
-  A(drec.alloc(3 * dep_cap, st));
-  A(doff.alloc(kEntries + 1, st));
-  A(dunits.alloc(kEntries + 1, st));
-  A(dsorted.alloc(dep_cap, st));
-  A(totals.alloc(kEntryBlocks, st));
-  if (e != cudaSuccess)
-    return fail(ctx, AJG_ERR_OOM, "device allocation failed (SPPM buffers)");
+  const uint32_t cap = (uint32_t)std::min<uint64_t>(8 * npix, 0xffffffffull);
 
-  int rc = sppm_camera_pass(sc, cam, p.forward_max_depth, p.seed, vp.p,
-                            direct.p, st);
+  // the camera pass's wave arena first, then everything else
+  int rc = sppm_reserve(sc, cam, p.forward_max_depth);
+  if (rc) return rc;
+  VisPointD* vp = nullptr;
+  float4 *direct, *phi, *tau, *film, *spheres, *qro, *qrd, *qcoef, *drec;
+  float4* d_out = nullptr;
+  float* d_rad = nullptr;
+  float *radius, *N, *maxr;
+  uint32_t *M, *counts, *offsets, *cursor, *items, *bits, *qcounts, *doff, *dsorted;
+  unsigned long long* dunits;
+  ajg_hit* qhits;
+  EntryVal* totals;
+  auto layout = [&](char* cur) {
+    vp = carve<VisPointD>(cur, npix);
+    direct = carve<float4>(cur, npix);
+    phi = carve<float4>(cur, npix);
+    tau = carve<float4>(cur, npix);
+    film = carve<float4>(cur, 2 * npix);
+    radius = carve<float>(cur, npix);
+    N = carve<float>(cur, npix);
+    maxr = carve<float>(cur, 1);
+    M = carve<uint32_t>(cur, npix);
+    counts = carve<uint32_t>(cur, kEntries);
+    offsets = carve<uint32_t>(cur, kEntries + 1);
+    cursor = carve<uint32_t>(cur, kEntries);
+    items = carve<uint32_t>(cur, cap);
+    spheres = carve<float4>(cur, cap);
+    bits = carve<uint32_t>(cur, 1);
+    qro = carve<float4>(cur, 2 * chunk);
+    qrd = carve<float4>(cur, 2 * chunk);
+    qcoef = carve<float4>(cur, 2 * chunk);
+    qhits = carve<ajg_hit>(cur, chunk);
+    qcounts = carve<uint32_t>(cur, n_counts + 1 + kEntries);
+    drec = carve<float4>(cur, 3 * dep_cap);
+    doff = carve<uint32_t>(cur, kEntries + 1);
+    dunits = carve<unsigned long long>(cur, kEntries + 1);
+    dsorted = carve<uint32_t>(cur, dep_cap);
+    totals = carve<EntryVal>(cur, kEntryBlocks);
+    if (want_film) d_out = carve<float4>(cur, npix);
+    if (want_rad) d_rad = carve<float>(cur, 3 * npix);
+    return cur;
+  };
+  const uint64_t bytes = (uint64_t)(uintptr_t)layout(nullptr);
+  if (scratch.take(ctx, bytes, st) != cudaSuccess)
+    return fail(ctx, AJG_ERR_OOM, "device allocation failed (SPPM buffers)");
+  layout(scratch.p);
+  *out_film = d_out;
+  *out_rad = d_rad;
+
+  rc = sppm_camera_pass(sc, cam, p.forward_max_depth, p.seed, vp, direct, st);
   if (rc) return rc;
 
   const int gs = kSMs * 8;
-  cudaMemsetAsync(phi.p, 0, npix * sizeof(float4), st);
-  cudaMemsetAsync(tau.p, 0, npix * sizeof(float4), st);
-  cudaMemsetAsync(N.p, 0, npix * sizeof(float), st);
-  cudaMemsetAsync(M.p, 0, npix * sizeof(uint32_t), st);
-  k_fill_f<<<grid_for(npix, 256, gs), 256, 0, st>>>(radius.p, npix, init_radius);
-  k_fill_f<<<1, 32, 0, st>>>(maxr.p, 1, init_radius);
-  const SppmPixels px{vp.p, direct.p, radius.p, N.p, M.p, phi.p, tau.p};
-  const Grid g{counts.p, offsets.p, cursor.p, items.p, spheres.p, cap, maxr.p};
+  cudaMemsetAsync(phi, 0, npix * sizeof(float4), st);
+  cudaMemsetAsync(tau, 0, npix * sizeof(float4), st);
+  cudaMemsetAsync(N, 0, npix * sizeof(float), st);
+  cudaMemsetAsync(M, 0, npix * sizeof(uint32_t), st);
+  k_fill_f<<<grid_for(npix, 256, gs), 256, 0, st>>>(radius, npix, init_radius);
+  k_fill_f<<<1, 32, 0, st>>>(maxr, 1, init_radius);
+  const SppmPixels px{vp, direct, radius, N, M, phi, tau};
+  const Grid g{counts, offsets, cursor, items, spheres, cap, maxr};
   PhotonQ q{};
-  q.ro[0] = qro.p;
-  q.ro[1] = qro.p + chunk;
-  q.rd[0] = qrd.p;
-  q.rd[1] = qrd.p + chunk;
-  q.coef[0] = qcoef.p;
-  q.coef[1] = qcoef.p + chunk;
-  q.hits = qhits.p;
-  q.counts = qcounts.p;
+  q.ro[0] = qro;
+  q.ro[1] = qro + chunk;
+  q.rd[0] = qrd;
+  q.rd[1] = qrd + chunk;
+  q.coef[0] = qcoef;
+  q.coef[1] = qcoef + chunk;
+  q.hits = qhits;
+  q.counts = qcounts;
   q.cap = (uint32_t)chunk;
   Deposits dp{};
-  dp.rec = drec.p;
-  dp.count = qcounts.p + n_counts;
+  dp.rec = drec;
+  dp.count = qcounts + n_counts;
   dp.hist = dp.count + 1;
-  dp.offsets = doff.p;
-  dp.units = dunits.p;
-  dp.sorted = dsorted.p;
+  dp.offsets = doff;
+  dp.units = dunits;
+  dp.sorted = dsorted;
   dp.cap = (uint32_t)dep_cap;
   const int gd = resident_grid((const void*)k_deposit, kThreads);
   for (uint32_t it = 0; it < p.iterations; ++it) {
     a.it = it;
-    cudaMemsetAsync(counts.p, 0, kEntries * sizeof(uint32_t), st);
+    cudaMemsetAsync(counts, 0, kEntries * sizeof(uint32_t), st);
     k_grid_count<<<grid_for(npix, 256, gs), 256, 0, st>>>(a, px, g, ctx->d_error);
-    k_entry_totals<false><<<kEntryBlocks, kEntryThreads, 0, st>>>(g, dp, totals.p);
-    k_entry_scan<false><<<kEntryBlocks, kEntryThreads, 0, st>>>(g, dp, totals.p);
+    k_entry_totals<false><<<kEntryBlocks, kEntryThreads, 0, st>>>(g, dp, totals);
+    k_entry_scan<false><<<kEntryBlocks, kEntryThreads, 0, st>>>(g, dp, totals);
     k_grid_fill<<<grid_for(npix, 256, gs), 256, 0, st>>>(a, px, g, ctx->d_error);
     for (uint64_t i0 = 0; i0 < p.photons_per_iteration; i0 += chunk) {
       const uint32_t n =
@@ -920,24 +912,24 @@ int sppm_render(ajg_scene* sc, const ajg_camera& cam, const ajg_sppm_params& p,
             a, g, q, dp, depth, ctx->d_error);
       }
       if (dep_depths) {
-        k_entry_totals<true><<<kEntryBlocks, kEntryThreads, 0, st>>>(g, dp, totals.p);
-        k_entry_scan<true><<<kEntryBlocks, kEntryThreads, 0, st>>>(g, dp, totals.p);
+        k_entry_totals<true><<<kEntryBlocks, kEntryThreads, 0, st>>>(g, dp, totals);
+        k_entry_scan<true><<<kEntryBlocks, kEntryThreads, 0, st>>>(g, dp, totals);
         k_deposit_sort<<<grid_for(dep_cap, 256, gs), 256, 0, st>>>(dp);
         k_deposit<<<gd, kThreads, 0, st>>>(a, px, g, dp);
       }
       ctx->paths_total += n;
     }
-    cudaMemsetAsync(bits.p, 0, sizeof(uint32_t), st);
-    k_max_radius<<<grid_for(npix, 256, gs), 256, 0, st>>>(a, px, bits.p);
+    cudaMemsetAsync(bits, 0, sizeof(uint32_t), st);
+    k_max_radius<<<grid_for(npix, 256, gs), 256, 0, st>>>(a, px, bits);
     k_update<<<grid_for(npix, 256, gs), 256, 0, st>>>(a, px, p.update_alpha,
-                                                      bits.p, maxr.p);
+                                                      bits, maxr);
   }
   const uint64_t photon_n =
       (uint64_t)p.iterations * (uint64_t)p.photons_per_iteration;
   k_final<<<grid_for(npix, 256, gs), 256, 0, st>>>(
-      a, px, p.iterations, photon_n, film.p, film.p + npix, d_rad);
+      a, px, p.iterations, photon_n, film, film + npix, d_rad);
   if (d_out)
-    enqueue_resolve(film.p, film.p + npix, nullptr, cam.width, cam.height,
+    enqueue_resolve(film, film + npix, nullptr, cam.width, cam.height,
                     true, true, d_out, st);
   const cudaError_t le = cudaGetLastError();
   if (le != cudaSuccess) return fail(ctx, AJG_ERR_CUDA, cudaGetErrorString(le));
