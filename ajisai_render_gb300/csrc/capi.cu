@@ -552,7 +552,14 @@ int ajg_scene_create_flat_ex(ajg_ctx* ctx, const float* tris,
   if (opts) o = *opts;
   if (o.tri_test > AJG_TRI_WATERTIGHT)
     return fail(ctx, AJG_ERR_INVALID, "unknown triangle test");
-  for (uint64_t i = 0; i < n; ++i) {
+  // one branch-free pass says whether any triangle is refused, the ordered
+  // one which error the first such triangle has
+  uint32_t bad = 0;
+  const uint32_t no_normals = corner_normals ? 0u : (uint32_t)AJG_MESH_HAS_NORMALS;
+  for (uint64_t i = 0; i < n; ++i)
+    bad |= (uint32_t)((uint32_t)tri_material[i] >= num_materials) |
+           ((uint32_t)tri_flags[i] & (~7u | no_normals));
+  for (uint64_t i = 0; bad && i < n; ++i) {
     if (tri_material[i] < 0 || (uint32_t)tri_material[i] >= num_materials)
       return fail(ctx, AJG_ERR_INVALID, "triangle material index out of range");
     if ((tri_flags[i] & AJG_MESH_HAS_NORMALS) && !corner_normals)
@@ -609,40 +616,50 @@ int ajg_scene_create_flat_ex(ajg_ctx* ctx, const float* tris,
     lum[m] = make_float4(host_lum(materials[m].base_color), 0, 0, 0);
     mat_mask |= 1u << materials[m].type;
   }
-  auto keep = [&](size_t bytes) -> void* {
-    void* p = nullptr;
-    if (!device_malloc(ctx, &p, bytes > 0 ? bytes : 16)) return nullptr;
-    s->allocations.push_back(p);
-    s->info.device_bytes += bytes;
-    return p;
+  // the tables: one allocation, the small ones staged for one copy
+  const size_t n_mat = s->host_materials.size();
+  const size_t n_light = std::max<size_t>(1, s->host_lights.size());
+  const size_t n_pts = num_area ? emit_pts.size() : 0;
+  float *d_mat, *d_light, *d_pts;
+  float4* d_lum;
+  int32_t* d_tri_emit = nullptr;
+  size_t staged = 0;
+  auto layout = [&](char* base) {
+    char* cur = base;
+    d_mat = carve<float>(cur, n_mat);
+    d_light = carve<float>(cur, n_light);
+    d_lum = carve<float4>(cur, num_materials);
+    d_pts = carve<float>(cur, n_pts);
+    staged = (size_t)(cur - base);
+    if (num_area) d_tri_emit = carve<int32_t>(cur, n);
+    return (size_t)(cur - base);
   };
-  float* d_mat = (float*)keep(s->host_materials.size() * sizeof(float));
-  float* d_light = (float*)keep(std::max<size_t>(1, s->host_lights.size()) *
-                                sizeof(float));
-  float4* d_lum = (float4*)keep(num_materials * sizeof(float4));
-  int32_t* d_tri_emit =
-      num_area ? (int32_t*)keep(n * sizeof(int32_t)) : nullptr;
-  float* d_pts = num_area ? (float*)keep(emit_pts.size() * sizeof(float)) : nullptr;
-  if (!d_mat || !d_light || !d_lum || (num_area && (!d_tri_emit || !d_pts))) {
+  const size_t total = layout(nullptr);
+  std::vector<char> stage(staged);
+  void* block = nullptr;
+  if (!device_malloc(ctx, &block, total)) {
     ajg_scene_release(s);
     return fail(ctx, AJG_ERR_OOM, "device allocation failed (scene tables)");
   }
-  cudaMemcpy(d_mat, s->host_materials.data(),
-             s->host_materials.size() * sizeof(float), cudaMemcpyHostToDevice);
+  s->allocations.push_back(block);
+  s->info.device_bytes += n_mat * sizeof(float) + n_light * sizeof(float) +
+                          num_materials * sizeof(float4) + n_pts * sizeof(float) +
+                          (num_area ? n * sizeof(int32_t) : 0);
+  layout(stage.data());
+  std::memcpy(d_mat, s->host_materials.data(), n_mat * sizeof(float));
   if (nl_all)
-    cudaMemcpy(d_light, s->host_lights.data(),
-               s->host_lights.size() * sizeof(float), cudaMemcpyHostToDevice);
-  if (num_area) {
-    cudaMemcpy(d_tri_emit, tri_emit.data(), n * sizeof(int32_t),
-               cudaMemcpyHostToDevice);
-    cudaMemcpy(d_pts, emit_pts.data(), emit_pts.size() * sizeof(float),
-               cudaMemcpyHostToDevice);
-  }
+    std::memcpy(d_light, s->host_lights.data(), s->host_lights.size() * sizeof(float));
+  std::memcpy(d_lum, lum.data(), num_materials * sizeof(float4));
+  if (n_pts) std::memcpy(d_pts, emit_pts.data(), n_pts * sizeof(float));
+  layout(static_cast<char*>(block));
+  cudaMemcpyAsync(block, stage.data(), staged, cudaMemcpyHostToDevice, ctx->stream);
+  if (num_area)
+    cudaMemcpyAsync(d_tri_emit, tri_emit.data(), n * sizeof(int32_t),
+                    cudaMemcpyHostToDevice, ctx->stream);
+  if (!num_area) d_pts = nullptr;
   s->d.tri_emit = d_tri_emit;
   s->d.emit_pts = d_pts;
   s->d.num_area = num_area;
-  cudaMemcpy(d_lum, lum.data(), num_materials * sizeof(float4),
-             cudaMemcpyHostToDevice);
   s->d.materials = d_mat;
   s->d.lights = d_light;
   s->d.mat_lum = d_lum;

@@ -18,6 +18,7 @@
 #include <cfloat>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "scan.cuh"
@@ -29,8 +30,11 @@ namespace {
 constexpr int kBuckets = 1024;
 constexpr int kRadixThreads = 256;
 constexpr int kRadixWarps = kRadixThreads / 32;
-constexpr int kKeysPerWarp = 512;
-constexpr int kRadixTile = kRadixWarps * kKeysPerWarp;  // 4096
+// Keys a warp ranks in order, 32 at a time: 512 amortise the digit tables of
+// a large sort; up to kSmallSort keys 64 spread the sort over eight times the
+// blocks (10,214 keys: 16 -> 5 us a pass).
+constexpr int kKeysPerWarp = 512, kKeysPerWarpSmall = 64;
+constexpr uint64_t kSmallSort = 1ull << 18;
 constexpr int kClusterThreads = 256;
 
 struct PNode {  // reference Node: bound, primitive_count, first_child
@@ -103,9 +107,11 @@ __global__ void k_morton(const float* __restrict__ tris, uint64_t n, F3 w2g,
   }
 }
 
+template <int KPW>
 __global__ void k_radix_hist(const uint32_t* __restrict__ keys, uint64_t n,
                              int bit, uint32_t* __restrict__ hist,
                              uint32_t nb) {
+  constexpr int kRadixTile = kRadixWarps * KPW;
   __shared__ uint32_t h[kBuckets];
   for (int d = threadIdx.x; d < kBuckets; d += blockDim.x) h[d] = 0;
   __syncthreads();
@@ -119,8 +125,9 @@ __global__ void k_radix_hist(const uint32_t* __restrict__ keys, uint64_t n,
     hist[(uint64_t)d * nb + blockIdx.x] = h[d];
 }
 
-// Stable scatter: warp w owns keys [t0 + w*512, t0 + (w+1)*512) and walks
+// Stable scatter: warp w owns keys [t0 + w*KPW, t0 + (w+1)*KPW) and walks
 // them in order, 32 at a time; lanes with equal digits rank by lane.
+template <int KPW>
 __global__ void __launch_bounds__(kRadixThreads)
     k_radix_scatter(const uint32_t* __restrict__ keys_in,
                     const int32_t* __restrict__ vals_in,
@@ -130,6 +137,7 @@ __global__ void __launch_bounds__(kRadixThreads)
                     int compat, const uint32_t* __restrict__ compat_base,
                     int32_t* __restrict__ owner, uint32_t* __restrict__ pos_of,
                     uint32_t* __restrict__ err) {
+  constexpr int kKeysPerWarp = KPW, kRadixTile = kRadixWarps * KPW;
   __shared__ uint32_t wh[kRadixWarps][kBuckets];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (int k = threadIdx.x; k < kRadixWarps * kBuckets; k += blockDim.x)
@@ -212,99 +220,435 @@ __global__ void k_compat_base(const uint32_t* __restrict__ offsets,
 
 __global__ void k_leaf_init(const float* __restrict__ tris,
                             const int32_t* __restrict__ perm,
-                            PNode* __restrict__ nodes, uint64_t begin,
-                            uint64_t n) {
+                            PNode* __restrict__ nodes, uint64_t n) {
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x) {
     F3 lo, hi;
     tri_box(tris + 9 * (uint64_t)perm[i], lo, hi);
-    nodes[begin + i].a = make_float4(lo.x, lo.y, lo.z, __int_as_float((int)i));
-    nodes[begin + i].b = make_float4(hi.x, hi.y, hi.z, __int_as_float(1));
+    nodes[i].a = make_float4(lo.x, lo.y, lo.z, __int_as_float((int)i));
+    nodes[i].b = make_float4(hi.x, hi.y, hi.z, __int_as_float(1));
   }
 }
 
-// Nearest neighbour within [i-r, i+r] (ploc_aggregate.cpp:408-459): scan in
-// ascending index order with a strict comparison.
-__global__ void __launch_bounds__(kClusterThreads)
-    k_neighbors(const PNode* __restrict__ in, uint32_t begin, uint32_t end,
-                int r, uint32_t* __restrict__ nb) {
-  extern __shared__ float sb[];
-  const uint32_t i0 = begin + blockIdx.x * kClusterThreads;
-  const uint32_t lo_idx = i0 > begin + (uint32_t)r ? i0 - r : begin;
-  const uint64_t hi_lim = (uint64_t)i0 + kClusterThreads + r;
-  const uint32_t hi_idx = hi_lim < end ? (uint32_t)hi_lim : end;
-  const uint32_t cnt = hi_idx - lo_idx;
-  for (uint32_t k = threadIdx.x; k < cnt; k += blockDim.x) {
-    float4 a = in[lo_idx + k].a, b = in[lo_idx + k].b;
-    sb[6 * k + 0] = a.x;
-    sb[6 * k + 1] = a.y;
-    sb[6 * k + 2] = a.z;
-    sb[6 * k + 3] = b.x;
-    sb[6 * k + 4] = b.y;
-    sb[6 * k + 5] = b.z;
+// SAH-optimal collapse into 4-wide nodes (the dynamic program of Ylitie,
+// Karras, Laine, "Efficient incoherent ray traversal on GPUs through
+// compressed wide BVHs", HPG 2017, with one triangle per leaf): cost[n].i
+// (i = 1..4 slots) is the least sum of wide-node surface areas with which
+// the subtree of binary node n fills at most i children of a wide node --
+// one slot holding n itself (a leaf, or a wide node of its own: its area
+// plus its children's best use of 4 slots), or its two children sharing
+// the slots.  Leaves cost 0 in every slot count (a leaf's triangle test is
+// the same whatever the tree).  choice[n] packs the decisions: byte 0 the
+// left child's share of a wide node's 4 slots, byte i-1 (i = 2..4) for i
+// slots 0 (n itself) or (left share << 4 | slots used).  A node's entry is
+// computed when the clustering places it (its children were placed before).
+#ifndef AJG_SAH_COLLAPSE
+#define AJG_SAH_COLLAPSE 1
+#endif
+struct SahTable {
+  float4* cost;      // [2n-1], null: not wanted
+  uint32_t* choice;  // [2n-1]
+};
+__device__ __forceinline__ void sah_node(const SahTable& t, uint32_t at,
+                                         const PNode& x) {
+  if (!t.cost) return;
+  if (__float_as_int(x.b.w) != 0) {  // leaf
+    t.cost[at] = make_float4(0.f, 0.f, 0.f, 0.f);
+    t.choice[at] = 0u;
+    return;
   }
-  __syncthreads();
-  const uint32_t i = i0 + threadIdx.x;
-  if (i >= end) return;
-  const uint32_t s0 = i > begin + (uint32_t)r ? i - r : begin;
-  const uint64_t e_lim = (uint64_t)i + r + 1;
-  const uint32_t s1 = e_lim < end ? (uint32_t)e_lim : end;
-  const float* mi = sb + 6 * (i - lo_idx);
-  const F3 ilo = mk3(mi[0], mi[1], mi[2]), ihi = mk3(mi[3], mi[4], mi[5]);
+  const uint32_t f = (uint32_t)__float_as_int(x.a.w);
+  const float4 L = t.cost[f], R = t.cost[f + 1];
+  const float l[5] = {0.f, L.x, L.y, L.z, L.w};
+  const float r[5] = {0.f, R.x, R.y, R.z, R.w};
+  float dist[5];
+  uint32_t dk[5];
+#pragma unroll
+  for (int j = 2; j <= 4; ++j) {
+    dist[j] = __int_as_float(0x7f800000);
+    dk[j] = 1;
+#pragma unroll
+    for (int k = 1; k < j; ++k) {
+      const float v = l[k] + r[j - k];
+      if (v < dist[j]) {
+        dist[j] = v;
+        dk[j] = (uint32_t)k;
+      }
+    }
+  }
+  float c[5];
+  uint32_t kind[5] = {0u, 0u, 0u, 0u, 0u};
+  c[1] = area(xyz(x.a), xyz(x.b)) + dist[4];
+#pragma unroll
+  for (int i = 2; i <= 4; ++i) {
+    if (dist[i] < c[i - 1]) {
+      c[i] = dist[i];
+      kind[i] = (dk[i] << 4) | (uint32_t)i;
+    } else {
+      c[i] = c[i - 1];
+      kind[i] = kind[i - 1];
+    }
+  }
+  t.cost[at] = make_float4(c[1], c[2], c[3], c[4]);
+  t.choice[at] = dk[4] | (kind[2] << 8) | (kind[3] << 16) | (kind[4] << 24);
+}
+
+// Cluster (ploc_aggregate.cpp:400-511), driven by device state: an iteration
+// over `cnt` clusters finds neighbours (k_neighbors), pairs them
+// (k_pairs: the merges per tile, and the last block to finish scans the
+// tiles and writes the next iteration's state) and writes the next clusters
+// and the pairs' nodes (k_cluster).  The active clusters are compact (two
+// alternating arrays); a node goes to its place in the final array once,
+// when it becomes a child: at `end` - 2 x merges, as the reference fills its
+// array from the back.  The host enqueues a guess of iterations and reads
+// the state once; kernels past the end of the work do nothing.  Once at most
+// kTail clusters are left, one block runs all the iterations that remain
+// (k_cluster_tail): they are short and most of the iterations.  kTail: one
+// SM's neighbour search over 2,048 clusters of 32 candidates takes as long as
+// the three launches it replaces (7 us), over 1,024 half of that.  Launch
+// and synchronisation bound before: five launches, a copy and a wait per
+// iteration (10,214 triangles, load to first picks: 3.00 -> 1.06 ms;
+// 1,310,722 triangles, load to a 640x360 first image: 12.08 -> 7.27 ms).
+struct PlocState {
+  uint32_t cnt;    // clusters
+  uint32_t end;    // final nodes at and above `end` are placed
+  uint32_t iters;  // iterations done
+  uint32_t buf;    // the cluster array in use
+  uint32_t stuck;  // an iteration merged no pair
+};
+constexpr uint32_t kTail = 1024;
+constexpr int kLevels = 64;  // levels of the wide collapse enqueued at most
+constexpr int kTailThreads = 1024;
+constexpr int kPairItems = 4;
+constexpr uint32_t kPairTile = kClusterThreads * kPairItems;
+
+__global__ void k_ploc_start(PlocState* s, uint32_t n, uint32_t* ticket) {
+  s[0] = PlocState{n, 2 * n - 1, 0, 0, 0};
+  *ticket = 0;
+}
+__device__ __forceinline__ bool ploc_idle(const PlocState& s) {
+  return s.cnt <= kTail || s.stuck;
+}
+
+// Nearest neighbour of box k within [s0, s1) of `box` (SoA, `stride` floats a
+// plane; ploc_aggregate.cpp:408-459): in ascending order with a strict
+// comparison.  0xffffffff: none.
+__device__ __forceinline__ uint32_t nearest(const float* box, uint32_t stride,
+                                            uint32_t k, uint32_t s0,
+                                            uint32_t s1) {
+  const F3 ilo = mk3(box[k], box[stride + k], box[2 * stride + k]);
+  const F3 ihi = mk3(box[3 * stride + k], box[4 * stride + k], box[5 * stride + k]);
   float best = FLT_MAX;
   uint32_t bj = 0xffffffffu;
   for (uint32_t j = s0; j < s1; ++j) {
-    if (j == i) continue;
-    const float* mj = sb + 6 * (j - lo_idx);
+    if (j == k) continue;
     F3 lo, hi;
-    join(ilo, ihi, mk3(mj[0], mj[1], mj[2]), mk3(mj[3], mj[4], mj[5]), lo, hi);
-    float d = area(lo, hi);
+    join(ilo, ihi, mk3(box[j], box[stride + j], box[2 * stride + j]),
+         mk3(box[3 * stride + j], box[4 * stride + j], box[5 * stride + j]), lo,
+         hi);
+    const float d = area(lo, hi);
     if (d < best) {
       best = d;
       bj = j;
     }
   }
-  nb[i] = bj;
+  return bj;
 }
 
-__global__ void k_merge_flags(const uint32_t* __restrict__ nb, uint32_t begin,
-                              uint32_t end, uint32_t* __restrict__ flags) {
-  for (uint32_t i = begin + blockIdx.x * blockDim.x + threadIdx.x; i < end;
-       i += gridDim.x * blockDim.x) {
-    uint32_t j = nb[i];
-    flags[i - begin] = (j != 0xffffffffu && i < j && nb[j] == i) ? 1u : 0u;
+__global__ void __launch_bounds__(kClusterThreads)
+    k_neighbors(const PlocState* __restrict__ st, const PNode* __restrict__ a,
+                const PNode* __restrict__ b, int r, uint32_t* __restrict__ nb) {
+  extern __shared__ float sb[];
+  const PlocState s = *st;
+  if (ploc_idle(s)) return;
+  const PNode* __restrict__ in = s.buf ? b : a;
+  const uint32_t stride = kClusterThreads + 2 * (uint32_t)r;
+  for (uint32_t i0 = blockIdx.x * kClusterThreads; i0 < s.cnt;
+       i0 += gridDim.x * kClusterThreads) {
+    const uint32_t lo_idx = i0 > (uint32_t)r ? i0 - r : 0u;
+    const uint32_t hi_idx = min(i0 + kClusterThreads + (uint32_t)r, s.cnt);
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < hi_idx - lo_idx; k += blockDim.x) {
+      const float4 lo = in[lo_idx + k].a, hi = in[lo_idx + k].b;
+      sb[k] = lo.x;
+      sb[stride + k] = lo.y;
+      sb[2 * stride + k] = lo.z;
+      sb[3 * stride + k] = hi.x;
+      sb[4 * stride + k] = hi.y;
+      sb[5 * stride + k] = hi.z;
+    }
+    __syncthreads();
+    const uint32_t i = i0 + threadIdx.x;
+    if (i >= s.cnt) continue;
+    const uint32_t s0 = i > (uint32_t)r ? i - r : 0u;
+    const uint32_t s1 = min(i + (uint32_t)r + 1, s.cnt);
+    const uint32_t j = nearest(sb, stride, i - lo_idx, s0 - lo_idx, s1 - lo_idx);
+    nb[i] = j == 0xffffffffu ? j : j + lo_idx;
   }
 }
 
-// ploc_aggregate.cpp:481-501
-__global__ void k_cluster_scatter(const PNode* __restrict__ in,
-                                  PNode* __restrict__ out,
-                                  const uint32_t* __restrict__ nb,
-                                  const uint32_t* __restrict__ mi,
-                                  uint32_t begin, uint32_t end,
-                                  uint32_t unmerged_begin,
-                                  uint32_t children_begin) {
-  for (uint32_t i = begin + blockIdx.x * blockDim.x + threadIdx.x; i < end;
-       i += gridDim.x * blockDim.x) {
-    const uint32_t j = nb[i];
-    if (j != 0xffffffffu && nb[j] == i) {
-      if (i < j) {
-        const uint32_t fc = children_begin + (mi[i - begin] - 1) * 2;
-        const PNode ni = in[i], nj = in[j];
-        F3 lo, hi;
-        join(xyz(nj.a), xyz(nj.b), xyz(ni.a), xyz(ni.b), lo, hi);
-        PNode p;
-        p.a = make_float4(lo.x, lo.y, lo.z, __int_as_float((int)fc));
-        p.b = make_float4(hi.x, hi.y, hi.z, __int_as_float(0));
-        out[unmerged_begin + j - begin - mi[j - begin]] = p;
-        out[fc + 0] = ni;
-        out[fc + 1] = nj;
+// mate[i]: the cluster i merges with, or i itself.
+__global__ void __launch_bounds__(kClusterThreads)
+    k_pairs(PlocState* st, int cur, const uint32_t* __restrict__ nb,
+            uint32_t* __restrict__ mate, uint32_t* tile_sum, uint32_t* ticket) {
+  __shared__ uint32_t s_warp[kClusterThreads / 32];
+  __shared__ uint32_t s_run;
+  const PlocState s = st[cur];
+  if (ploc_idle(s)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) st[cur ^ 1] = s;
+    return;
+  }
+  const uint32_t tiles = (s.cnt + kPairTile - 1) / kPairTile;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+    uint32_t c = 0;
+#pragma unroll
+    for (int k = 0; k < kPairItems; ++k) {
+      const uint32_t i = t * kPairTile + k * kClusterThreads + threadIdx.x;
+      if (i < s.cnt) {
+        const uint32_t j = nb[i];
+        const bool mutual = j != 0xffffffffu && nb[j] == i;
+        mate[i] = mutual ? j : i;
+        c += mutual && i < j;
       }
-    } else {
-      out[unmerged_begin + i - begin - mi[i - begin]] = in[i];
+    }
+    c = __reduce_add_sync(0xffffffffu, c);
+    __syncthreads();
+    if (lane == 0) s_warp[warp] = c;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      uint32_t sum = 0;
+      for (int w = 0; w < kClusterThreads / 32; ++w) sum += s_warp[w];
+      tile_sum[t] = sum;
+    }
+  }
+  // the last block scans the tiles' merges in place (exclusive)
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_run = atomicAdd(ticket, 1u);
+  __syncthreads();
+  if (s_run != gridDim.x - 1) return;
+  __threadfence();
+  uint32_t run = 0;
+  for (uint32_t t0 = 0; t0 < tiles; t0 += kClusterThreads) {
+    const uint32_t t = t0 + threadIdx.x;
+    const uint32_t own = t < tiles ? __ldcg(&tile_sum[t]) : 0u;
+    uint32_t x = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    __syncthreads();
+    if (lane == 31) s_warp[warp] = x;
+    __syncthreads();
+    uint32_t before = run, all = 0;
+    for (int w = 0; w < kClusterThreads / 32; ++w) {
+      if (w < warp) before += s_warp[w];
+      all += s_warp[w];
+    }
+    if (t < tiles) tile_sum[t] = before + x - own;
+    run += all;
+  }
+  if (threadIdx.x == 0) {
+    PlocState next = s;
+    next.stuck = run == 0;
+    next.iters = s.iters + 1;
+    next.cnt = s.cnt - run;
+    next.end = s.end - 2 * run;
+    next.buf = s.buf ^ 1;
+    st[cur ^ 1] = next;
+    *ticket = 0;
+  }
+}
+
+// The parent of clusters i < j whose nodes go to fc and fc + 1
+// (ploc_aggregate.cpp:481-501).
+__device__ __forceinline__ PNode merged_node(const PNode& ni, const PNode& nj,
+                                             uint32_t fc) {
+  F3 lo, hi;
+  join(xyz(nj.a), xyz(nj.b), xyz(ni.a), xyz(ni.b), lo, hi);
+  PNode p;
+  p.a = make_float4(lo.x, lo.y, lo.z, __int_as_float((int)fc));
+  p.b = make_float4(hi.x, hi.y, hi.z, __int_as_float(0));
+  return p;
+}
+
+__global__ void __launch_bounds__(kClusterThreads)
+    k_cluster(const PlocState* __restrict__ st, int cur, PNode* a, PNode* b,
+              const uint32_t* __restrict__ mate,
+              const uint32_t* __restrict__ tile_sum, PNode* __restrict__ nodes,
+              SahTable sah) {
+  __shared__ uint32_t s_warp[kPairItems][kClusterThreads / 32];
+  const PlocState s = st[cur];
+  if (ploc_idle(s)) return;
+  const uint32_t first = st[cur ^ 1].end;  // this iteration's nodes start here
+  if (st[cur ^ 1].stuck) return;
+  const PNode* in = s.buf ? b : a;
+  PNode* out = s.buf ? a : b;
+  const uint32_t tiles = (s.cnt + kPairTile - 1) / kPairTile;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned le = 0xffffffffu >> (31 - lane);
+  for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+    uint32_t m[kPairItems], in_warp[kPairItems];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kPairItems; ++k) {
+      const uint32_t i = t * kPairTile + k * kClusterThreads + threadIdx.x;
+      m[k] = i < s.cnt ? mate[i] : i;
+      const unsigned bal = __ballot_sync(0xffffffffu, m[k] > i);
+      in_warp[k] = __popc(bal & le);
+      if (lane == 0) s_warp[k][warp] = __popc(bal);
+    }
+    __syncthreads();
+    uint32_t run = tile_sum[t];
+#pragma unroll
+    for (int k = 0; k < kPairItems; ++k) {
+      const uint32_t i = t * kPairTile + k * kClusterThreads + threadIdx.x;
+      uint32_t before = run;
+      for (int w = 0; w < kClusterThreads / 32; ++w) {
+        if (w < warp) before += s_warp[k][w];
+        run += s_warp[k][w];
+      }
+      if (i >= s.cnt) continue;
+      const uint32_t mi = before + in_warp[k];  // merges up to and with i
+      const uint32_t j = m[k];
+      if (j == i) {
+        out[i - mi] = in[i];
+      } else if (j > i) {
+        const uint32_t fc = first + (mi - 1) * 2;
+        uint32_t mj = mi;  // merges up to and with j (at most r further)
+        for (uint32_t k2 = i + 1; k2 <= j; ++k2) mj += mate[k2] > k2;
+        const PNode ni = in[i], nj = in[j];
+        out[j - mj] = merged_node(ni, nj, fc);
+        nodes[fc] = ni;
+        nodes[fc + 1] = nj;
+        sah_node(sah, fc, ni);
+        sah_node(sah, fc + 1, nj);
+      }
     }
   }
 }
+
+// The iterations over at most kTail clusters, in one block: clusters in
+// shared memory, a barrier where the other kernels end.  Runs no more
+// iterations than there are clusters (each merges a pair or stops).
+struct TailMem {
+  float box[6][kTail];
+  int first[kTail], count[kTail];
+  uint32_t nb[kTail], mi[kTail];
+  uint32_t warp[kTailThreads / 32];
+};
+__global__ void __launch_bounds__(kTailThreads)
+    k_cluster_tail(PlocState* st, int cur, const PNode* a, const PNode* b,
+                   int r, PNode* nodes, SahTable sah) {
+  extern __shared__ char tail_smem[];
+  TailMem& m = *reinterpret_cast<TailMem*>(tail_smem);
+  PlocState s = st[cur];
+  if (s.cnt > kTail || s.stuck) return;
+  const PNode* in = s.buf ? b : a;
+  constexpr int kPer = kTail / kTailThreads;
+  const uint32_t tid = threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5;
+  auto put = [&](uint32_t k, const PNode& x) {
+    m.box[0][k] = x.a.x;
+    m.box[1][k] = x.a.y;
+    m.box[2][k] = x.a.z;
+    m.box[3][k] = x.b.x;
+    m.box[4][k] = x.b.y;
+    m.box[5][k] = x.b.z;
+    m.first[k] = __float_as_int(x.a.w);
+    m.count[k] = __float_as_int(x.b.w);
+  };
+  auto get = [&](uint32_t k) {
+    PNode x;
+    x.a = make_float4(m.box[0][k], m.box[1][k], m.box[2][k],
+                      __int_as_float(m.first[k]));
+    x.b = make_float4(m.box[3][k], m.box[4][k], m.box[5][k],
+                      __int_as_float(m.count[k]));
+    return x;
+  };
+  for (uint32_t k = tid; k < s.cnt; k += kTailThreads) put(k, in[k]);
+  __syncthreads();
+  while (s.cnt > 1) {
+    for (uint32_t i = tid; i < s.cnt; i += kTailThreads) {
+      const uint32_t s0 = i > (uint32_t)r ? i - r : 0u;
+      m.nb[i] = nearest(&m.box[0][0], kTail, i, s0, min(i + (uint32_t)r + 1, s.cnt));
+    }
+    __syncthreads();
+    // merges up to and with each cluster (a thread holds kPer in a row)
+    uint32_t mate[kPer], sum = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const uint32_t i = tid * kPer + k;
+      mate[k] = i;
+      if (i < s.cnt) {
+        const uint32_t j = m.nb[i];
+        if (j != 0xffffffffu && m.nb[j] == i) mate[k] = j;
+      }
+      sum += mate[k] > i;
+    }
+    uint32_t x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) m.warp[warp] = x;
+    __syncthreads();
+    uint32_t before = 0, merged = 0;
+    {
+      const uint32_t w = m.warp[lane];
+      before = __reduce_add_sync(0xffffffffu, lane < warp ? w : 0u);
+      merged = __reduce_add_sync(0xffffffffu, w);
+    }
+    uint32_t run = before + x - sum;
+    PNode own[kPer], other[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const uint32_t i = tid * kPer + k;
+      if (i >= s.cnt) continue;
+      run += mate[k] > i;
+      m.mi[i] = run;
+      own[k] = get(i);
+      if (mate[k] > i) other[k] = get(mate[k]);
+    }
+    __syncthreads();
+    if (merged == 0) {
+      s.stuck = 1;
+      break;
+    }
+    s.end -= 2 * merged;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const uint32_t i = tid * kPer + k;
+      if (i >= s.cnt) continue;
+      const uint32_t mi = m.mi[i], j = mate[k];
+      if (j == i) {
+        put(i - mi, own[k]);
+      } else if (j > i) {
+        const uint32_t fc = s.end + (mi - 1) * 2;
+        nodes[fc] = own[k];
+        nodes[fc + 1] = other[k];
+        sah_node(sah, fc, own[k]);
+        sah_node(sah, fc + 1, other[k]);
+        put(j - m.mi[j], merged_node(own[k], other[k], fc));
+      }
+    }
+    s.cnt -= merged;
+    ++s.iters;
+    __syncthreads();
+  }
+  if (tid == 0) {
+    if (s.cnt == 1) {
+      const PNode root = get(0);
+      nodes[0] = root;
+      sah_node(sah, 0, root);
+    }
+    st[cur] = s;
+  }
+}
+
 
 __global__ void k_inner_flags(const PNode* __restrict__ nodes, uint64_t m,
                               uint32_t* __restrict__ flags) {
@@ -353,18 +697,22 @@ __global__ void k_bvh2_single(const PNode* __restrict__ nodes,
 // wide nodes per launch: a wide node takes its binary node and expands the
 // interior child with the largest surface area until it has W children (or
 // only leaves); its interior children become the wide nodes of the next
-// level, allocated contiguously.  Node layout (2W float4, 32W bytes): the
+// level, allocated contiguously.  A level's length is a counter of its own
+// (n_in, n_out), so levels are enqueued without the host reading them.  Node
+// layout (2W float4, 32W bytes): the
 // children's lo.x, hi.x, lo.y, hi.y, lo.z, hi.z in groups of four, then the
 // references (>= 0 wide node, ~slot leaf, kEmptyRef unused), then padding.
 constexpr int kWideEmpty = (int)0x80000000;
 
 template <int W>
 __global__ void k_collapse(const PNode* __restrict__ nodes,
-                           const uint2* __restrict__ fin, uint32_t n_in,
-                           uint2* __restrict__ fout,
+                           const uint2* __restrict__ fin,
+                           const uint32_t* __restrict__ n_in_,
+                           uint2* __restrict__ fout, uint32_t* n_out,
                            uint32_t* __restrict__ counters,
                            float4* __restrict__ wide) {
   constexpr int G = W / 4;
+  const uint32_t n_in = *n_in_;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_in;
        i += gridDim.x * blockDim.x) {
     const uint2 e = fin[i];  // (binary node, wide slot)
@@ -393,8 +741,8 @@ __global__ void k_collapse(const PNode* __restrict__ nodes,
       ni += __float_as_int(nodes[ch[c]].b.w) == 0 ? 1 : 0;
     uint32_t base = 0, fo = 0;
     if (ni) {
-      base = atomicAdd(&counters[1], (uint32_t)ni);
-      fo = atomicAdd(&counters[0], (uint32_t)ni);
+      base = atomicAdd(&counters[0], (uint32_t)ni);
+      fo = atomicAdd(n_out, (uint32_t)ni);
     }
     float pl[6][W];
     int rf[W];
@@ -433,79 +781,17 @@ __global__ void k_collapse(const PNode* __restrict__ nodes,
   }
 }
 
-// SAH-optimal collapse into 4-wide nodes (the dynamic program of Ylitie,
-// Karras, Laine, "Efficient incoherent ray traversal on GPUs through
-// compressed wide BVHs", HPG 2017, with one triangle per leaf): cost[n].i
-// (i = 1..4 slots) is the least sum of wide-node surface areas with which
-// the subtree of binary node n fills at most i children of a wide node --
-// one slot holding n itself (a leaf, or a wide node of its own: its area
-// plus its children's best use of 4 slots), or its two children sharing
-// the slots.  Leaves cost 0 in every slot count (a leaf's triangle test is
-// the same whatever the tree).  choice[n] packs the decisions: byte 0 the
-// left child's share of a wide node's 4 slots, byte i-1 (i = 2..4) for i
-// slots 0 (n itself) or (left share << 4 | slots used).  One launch per
-// block of nodes the PLOC loop finalised, in the order they were
-// finalised: children always come before their parents.
-#ifndef AJG_SAH_COLLAPSE
-#define AJG_SAH_COLLAPSE 1
-#endif
-__global__ void k_sah_dp(const PNode* __restrict__ nodes, uint32_t lo,
-                         uint32_t hi, float4* __restrict__ cost,
-                         uint32_t* __restrict__ choice) {
-  for (uint32_t n = lo + blockIdx.x * blockDim.x + threadIdx.x; n < hi;
-       n += gridDim.x * blockDim.x) {
-    const PNode x = nodes[n];
-    if (__float_as_int(x.b.w) != 0) {  // leaf
-      cost[n] = make_float4(0.f, 0.f, 0.f, 0.f);
-      choice[n] = 0u;
-      continue;
-    }
-    const uint32_t f = (uint32_t)__float_as_int(x.a.w);
-    const float4 L = cost[f], R = cost[f + 1];
-    const float l[5] = {0.f, L.x, L.y, L.z, L.w};
-    const float r[5] = {0.f, R.x, R.y, R.z, R.w};
-    float dist[5];
-    uint32_t dk[5];
-#pragma unroll
-    for (int j = 2; j <= 4; ++j) {
-      dist[j] = __int_as_float(0x7f800000);
-      dk[j] = 1;
-#pragma unroll
-      for (int k = 1; k < j; ++k) {
-        const float v = l[k] + r[j - k];
-        if (v < dist[j]) {
-          dist[j] = v;
-          dk[j] = (uint32_t)k;
-        }
-      }
-    }
-    float c[5];
-    uint32_t kind[5] = {0u, 0u, 0u, 0u, 0u};
-    c[1] = area(xyz(x.a), xyz(x.b)) + dist[4];
-#pragma unroll
-    for (int i = 2; i <= 4; ++i) {
-      if (dist[i] < c[i - 1]) {
-        c[i] = dist[i];
-        kind[i] = (dk[i] << 4) | (uint32_t)i;
-      } else {
-        c[i] = c[i - 1];
-        kind[i] = kind[i - 1];
-      }
-    }
-    cost[n] = make_float4(c[1], c[2], c[3], c[4]);
-    choice[n] = dk[4] | (kind[2] << 8) | (kind[3] << 16) | (kind[4] << 24);
-  }
-}
-
 // k_collapse with the children of each wide node taken from the dynamic
 // program above instead of by expanding the largest-area child.
 __global__ void k_collapse_sah(const PNode* __restrict__ nodes,
                                const uint32_t* __restrict__ choice,
-                               const uint2* __restrict__ fin, uint32_t n_in,
-                               uint2* __restrict__ fout,
+                               const uint2* __restrict__ fin,
+                               const uint32_t* __restrict__ n_in_,
+                               uint2* __restrict__ fout, uint32_t* n_out,
                                uint32_t* __restrict__ counters,
                                float4* __restrict__ wide) {
   constexpr int W = 4;
+  const uint32_t n_in = *n_in_;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_in;
        i += gridDim.x * blockDim.x) {
     const uint2 e = fin[i];  // (binary node, wide slot)
@@ -545,8 +831,8 @@ __global__ void k_collapse_sah(const PNode* __restrict__ nodes,
       ni += __float_as_int(nodes[ch[c]].b.w) == 0 ? 1 : 0;
     uint32_t base = 0, fo = 0;
     if (ni) {
-      base = atomicAdd(&counters[1], (uint32_t)ni);
-      fo = atomicAdd(&counters[0], (uint32_t)ni);
+      base = atomicAdd(&counters[0], (uint32_t)ni);
+      fo = atomicAdd(n_out, (uint32_t)ni);
     }
     float pl[6][W];
     int rf[W];
@@ -586,12 +872,14 @@ __global__ void k_collapse_sah(const PNode* __restrict__ nodes,
 template <int W>
 __global__ void k_collapse_c(const PNode* __restrict__ nodes,
                              const float4* __restrict__ tris_old,
-                             const uint2* __restrict__ fin, uint32_t n_in,
-                             uint2* __restrict__ fout,
+                             const uint2* __restrict__ fin,
+                             const uint32_t* __restrict__ n_in_,
+                             uint2* __restrict__ fout, uint32_t* n_out,
                              uint32_t* __restrict__ counters,
                              float4* __restrict__ wide,
                              float4* __restrict__ tris_new) {
   constexpr int NF = CwLayout<W>::kFloat4;
+  const uint32_t n_in = *n_in_;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_in;
        i += gridDim.x * blockDim.x) {
     const uint2 e = fin[i];
@@ -675,10 +963,10 @@ __global__ void k_collapse_c(const PNode* __restrict__ nodes,
     const int ni = __popc(imask), nl = __popc(vmask & ~imask);
     uint32_t base = 0, fo = 0, tb = 0;
     if (ni) {
-      base = atomicAdd(&counters[1], (uint32_t)ni);
-      fo = atomicAdd(&counters[0], (uint32_t)ni);
+      base = atomicAdd(&counters[0], (uint32_t)ni);
+      fo = atomicAdd(n_out, (uint32_t)ni);
     }
-    if (nl) tb = atomicAdd(&counters[2], (uint32_t)nl);
+    if (nl) tb = atomicAdd(&counters[1], (uint32_t)nl);
     int ji = 0, jl = 0;
     for (int c = 0; c < nc; ++c) {
       const PNode x = nodes[ch[c]];
@@ -744,34 +1032,47 @@ __global__ void k_shade_data(const float* __restrict__ tris,
   }
 }
 
-__global__ void k_lum(const float* __restrict__ mats, uint32_t m,
-                      float4* __restrict__ out) {
-  for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
-    const float* r = mats + 16 * i;
-    // spectrum.h:80-82, evaluated in double as the reference does
-    float lum = (float)(0.2126 * (double)r[1] + 0.7152 * (double)r[2] +
-                        0.0722 * (double)r[3]);
-    out[i] = make_float4(lum, 0.f, 0.f, 0.f);
+// The build's temporaries: the context's kept scratch, or past kScratchKeep
+// an allocation of its own.
+struct BuildMem {
+  Scratch scratch;
+  void* own = nullptr;
+  char* p = nullptr;
+  bool take(ajg_ctx* ctx, uint64_t bytes, cudaStream_t st) {
+    if (bytes <= kScratchKeep) {
+      if (scratch.take(ctx, bytes, st) != cudaSuccess) return false;
+      p = scratch.p;
+      return true;
+    }
+    if (!device_malloc(ctx, &own, bytes)) return false;
+    p = static_cast<char*>(own);
+    return true;
   }
-}
+  ~BuildMem() {
+    if (own) cudaFree(own);
+  }
+};
 
-struct Arena {
+// The arrays only shading reads, copied in on the trace stream while the
+// tree is built (1,310,722 triangles: 58 of 105 MB, 330 us); done before the
+// build returns, whichever way it does.
+struct ShadingCopy {
   ajg_ctx* ctx;
-  std::vector<void*> ptrs;
-  explicit Arena(ajg_ctx* c) : ctx(c) {}
-  cudaError_t err = cudaSuccess;
-  template <class T>
-  T* get(uint64_t count) {
-    void* p = nullptr;
-    if (err != cudaSuccess) return nullptr;
-    if (!device_malloc(ctx, &p, count * sizeof(T) > 0 ? count * sizeof(T) : 16))
-      err = cudaErrorMemoryAllocation;
-    if (err != cudaSuccess) return nullptr;
-    ptrs.push_back(p);
-    return static_cast<T*>(p);
+  bool started = false;
+  void start(int32_t* d_mat, const int32_t* mat, int32_t* d_flags,
+             const int32_t* flags, float* d_corner, const float* corner,
+             uint64_t n) {
+    started = true;
+    cudaStream_t ts = ctx->trace_stream;
+    cudaMemcpyAsync(d_mat, mat, n * sizeof(int32_t), cudaMemcpyHostToDevice, ts);
+    cudaMemcpyAsync(d_flags, flags, n * sizeof(int32_t), cudaMemcpyHostToDevice, ts);
+    if (d_corner)
+      cudaMemcpyAsync(d_corner, corner, n * 9 * sizeof(float),
+                      cudaMemcpyHostToDevice, ts);
+    cudaEventRecord(ctx->ev_queue, ts);
   }
-  ~Arena() {
-    for (void* p : ptrs) cudaFree(p);
+  ~ShadingCopy() {
+    if (started) cudaStreamSynchronize(ctx->trace_stream);
   }
 };
 
@@ -820,14 +1121,6 @@ int build_scene(ajg_ctx* ctx, ajg_scene* s, const float* h_tris,
       break;
     }
 
-  // persistent scene buffers
-  auto keep = [&](size_t bytes) -> void* {
-    void* p = nullptr;
-    if (!device_malloc(ctx, &p, bytes > 0 ? bytes : 16)) return nullptr;
-    s->allocations.push_back(p);
-    s->info.device_bytes += bytes;
-    return p;
-  };
   const uint64_t inner = n > 1 ? n - 1 : 1;
   // default: the 4-wide tree (the fastest measured on GB300 for the
   // workloads here; 8-wide nodes cost occupancy)
@@ -841,55 +1134,102 @@ int build_scene(ajg_ctx* ctx, ajg_scene* s, const float* h_tris,
   // the binary layout: the tree itself (width 2), or beside a plain 4-wide
   // tree for the closest-hit traversal (closest_width)
   const bool hybrid = closest_width(width) != width;
-  float4* bvh =
-      width == 2 ? (float4*)keep(inner * 4 * sizeof(float4)) : nullptr;
-  float4* bvh_bin = hybrid ? (float4*)keep(inner * 4 * sizeof(float4)) : nullptr;
-  float4* slot_tris = (float4*)keep(n * 3 * sizeof(float4));
-  float4* shade = (float4*)keep(n * sizeof(float4));
-  float* corner = any_normals ? (float*)keep(n * 9 * sizeof(float)) : nullptr;
-  float4* ploc_nodes = (float4*)keep(m * sizeof(PNode));
-  int32_t* perm_keep = (int32_t*)keep(n * sizeof(int32_t));
-  if ((width == 2 && !bvh) || (hybrid && !bvh_bin) || !slot_tris || !shade ||
-      (any_normals && !corner) ||
-      !ploc_nodes || !perm_keep)
-    return set_err(ctx, AJG_ERR_OOM, "device allocation failed (scene)");
+  const bool wide = width != 2;
+  const bool sah = AJG_SAH_COLLAPSE && wn == 4 && !compressed;
+  const uint64_t node_f4 =
+      compressed ? (wn == 8 ? CwLayout<8>::kFloat4 : CwLayout<4>::kFloat4)
+                 : 2 * (uint64_t)wn;
 
-  Arena tmp(ctx);
-  float* d_tris = tmp.get<float>(n * 9);
-  int32_t* d_mat = tmp.get<int32_t>(n);
-  int32_t* d_flags = tmp.get<int32_t>(n);
-  uint32_t* ka = tmp.get<uint32_t>(n);
-  uint32_t* kb = tmp.get<uint32_t>(n);
-  int32_t* va = tmp.get<int32_t>(n);
-  int32_t* vb = tmp.get<int32_t>(n);
-  const uint32_t nbt = (uint32_t)((n + kRadixTile - 1) / kRadixTile);
+  // persistent scene buffers: one allocation (the wide tree, whose size the
+  // collapse finds, is the other)
+  float4 *bvh = nullptr, *bvh_bin = nullptr, *slot_tris, *shade, *ploc_nodes;
+  float* corner = nullptr;
+  int32_t* perm_keep;
+  uint64_t kept = 0;  // bytes in use
+  auto layout = [&](char* cur) {
+    kept = 0;
+    auto get = [&](auto* type, uint64_t count) {
+      using T = std::remove_pointer_t<decltype(type)>;
+      kept += count * sizeof(T);
+      return carve<T>(cur, count);
+    };
+    if (!wide) bvh = get((float4*)nullptr, inner * 4);
+    if (hybrid) bvh_bin = get((float4*)nullptr, inner * 4);
+    slot_tris = get((float4*)nullptr, n * 3);
+    shade = get((float4*)nullptr, n);
+    if (any_normals) corner = get((float*)nullptr, n * 9);
+    ploc_nodes = get((float4*)nullptr, 2 * m);
+    perm_keep = get((int32_t*)nullptr, n);
+    return cur;
+  };
+  void* block = nullptr;
+  if (!device_malloc(ctx, &block, (uint64_t)(uintptr_t)layout(nullptr)))
+    return set_err(ctx, AJG_ERR_OOM, "device allocation failed (scene)");
+  s->allocations.push_back(block);
+  layout(static_cast<char*>(block));
+  s->info.device_bytes += kept;
+
+  float* d_tris;
+  int32_t *d_mat, *d_flags, *va, *vb, *owner = nullptr;
+  uint32_t *ka, *kb, *hist, *scratch, *pos_of = nullptr, *acc, *nbr, *mate, *tile_sum,
+      *flags = nullptr, *mi = nullptr, *choice = nullptr, *wc = nullptr;
+  PNode *na, *nbuf;
+  PlocState* state;
+  float4 *cost = nullptr, *wtmp = nullptr, *tri_tmp = nullptr;
+  uint2 *fa = nullptr, *fb = nullptr;
+  const bool small_sort = n <= kSmallSort;
+  const uint64_t radix_tile =
+      (uint64_t)kRadixWarps * (small_sort ? kKeysPerWarpSmall : kKeysPerWarp);
+  const uint32_t nbt = (uint32_t)((n + radix_tile - 1) / radix_tile);
   const uint64_t hist_n = (uint64_t)kBuckets * nbt;
-  uint32_t* hist = tmp.get<uint32_t>(hist_n);
-  uint32_t* scratch =
-      tmp.get<uint32_t>(scan_scratch_words(hist_n > m ? hist_n : m));
-  int32_t* owner = opts.radix_compat ? tmp.get<int32_t>(n) : nullptr;
-  uint32_t* pos_of = opts.radix_compat ? tmp.get<uint32_t>(n) : nullptr;
-  uint32_t* acc = tmp.get<uint32_t>(2);
-  PNode* na = tmp.get<PNode>(m);
-  PNode* nbuf = tmp.get<PNode>(m);
-  uint32_t* nbr = tmp.get<uint32_t>(m);
-  uint32_t* mi = tmp.get<uint32_t>(m);
-  uint32_t* flags = tmp.get<uint32_t>(m);
-  if (tmp.err != cudaSuccess)
+  auto temporaries = [&](char* cur) {
+    d_tris = carve<float>(cur, n * 9);
+    d_mat = carve<int32_t>(cur, n);
+    d_flags = carve<int32_t>(cur, n);
+    ka = carve<uint32_t>(cur, n);
+    kb = carve<uint32_t>(cur, n);
+    va = carve<int32_t>(cur, n);
+    vb = carve<int32_t>(cur, n);
+    hist = carve<uint32_t>(cur, hist_n);
+    scratch = carve<uint32_t>(cur, scan_scratch_words(hist_n > m ? hist_n : m));
+    if (opts.radix_compat) {
+      owner = carve<int32_t>(cur, n);
+      pos_of = carve<uint32_t>(cur, n);
+    }
+    acc = carve<uint32_t>(cur, 2);  // the sort's, then the clustering's ticket
+    na = carve<PNode>(cur, n);
+    nbuf = carve<PNode>(cur, n);
+    nbr = carve<uint32_t>(cur, n);
+    mate = carve<uint32_t>(cur, n);
+    tile_sum = carve<uint32_t>(cur, (n + kPairTile - 1) / kPairTile);
+    state = carve<PlocState>(cur, 2);
+    if (!wide || hybrid) {
+      flags = carve<uint32_t>(cur, m);
+      mi = carve<uint32_t>(cur, m);
+    }
+    if (sah) {
+      cost = carve<float4>(cur, m);
+      choice = carve<uint32_t>(cur, m);
+    }
+    if (wide) {
+      wtmp = carve<float4>(cur, inner * node_f4);
+      if (compressed) tri_tmp = carve<float4>(cur, 3 * n);
+      fa = carve<uint2>(cur, inner);
+      fb = carve<uint2>(cur, inner);
+      wc = carve<uint32_t>(cur, 2 + kLevels + 1);
+    }
+    return cur;
+  };
+  BuildMem tmp;
+  if (!tmp.take(ctx, (uint64_t)(uintptr_t)temporaries(nullptr), st))
     return set_err(ctx, AJG_ERR_OOM, "device allocation failed (PLOC build)");
+  temporaries(tmp.p);
 
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   cudaMemcpyAsync(d_tris, h_tris, n * 9 * sizeof(float),
                   cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(d_mat, h_mat, n * sizeof(int32_t), cudaMemcpyHostToDevice,
-                  st);
-  cudaMemcpyAsync(d_flags, h_flags, n * sizeof(int32_t),
-                  cudaMemcpyHostToDevice, st);
-  if (corner)
-    cudaMemcpyAsync(corner, h_corner, n * 9 * sizeof(float),
-                    cudaMemcpyHostToDevice, st);
   cudaMemsetAsync(ctx->d_error, 0, sizeof(uint32_t), st);
   cudaEventRecord(e0, st);
 
@@ -916,13 +1256,18 @@ int build_scene(ajg_ctx* ctx, ajg_scene* s, const float* h_tris,
   int32_t* vin = va;
   int32_t* vout = vb;
   for (int bit = 0; bit < 30; bit += 10) {
-    k_radix_hist<<<nbt, kRadixThreads, 0, st>>>(kin, n, bit, hist, nbt);
+    if (small_sort)
+      k_radix_hist<kKeysPerWarpSmall><<<nbt, kRadixThreads, 0, st>>>(kin, n, bit, hist, nbt);
+    else
+      k_radix_hist<kKeysPerWarp><<<nbt, kRadixThreads, 0, st>>>(kin, n, bit, hist, nbt);
     device_scan(hist, hist, hist_n, true, scratch, st);
     if (opts.radix_compat) {
       k_compat_base<<<1, 1, 0, st>>>(hist, nbt, acc);
       cudaMemsetAsync(owner, 0xff, n * sizeof(int32_t), st);
     }
-    k_radix_scatter<<<nbt, kRadixThreads, 0, st>>>(
+    auto* scatter = small_sort ? k_radix_scatter<kKeysPerWarpSmall>
+                               : k_radix_scatter<kKeysPerWarp>;
+    scatter<<<nbt, kRadixThreads, 0, st>>>(
         kin, vin, kout, vout, n, bit, hist, nbt, opts.radix_compat ? 1 : 0,
         acc, owner, pos_of, ctx->d_error);
     if (opts.radix_compat)
@@ -933,62 +1278,57 @@ int build_scene(ajg_ctx* ctx, ajg_scene* s, const float* h_tris,
   }
   const int32_t* perm = vin;  // sorted values after three passes
 
-  // leaves, then cluster until one node remains
-  uint64_t begin = m - n, end = m, pre_end = m;
-  k_leaf_init<<<gb, 256, 0, st>>>(d_tris, perm, na, begin, n);
-  PNode* in = na;
-  PNode* out = nbuf;
-  uint32_t iters = 0;
+  // leaves, then cluster until one node remains: a batch of iterations is
+  // enqueued, then the one-block tail, and the state read once.  An iteration
+  // leaves about four of five clusters (1,310,722 triangles: 62 iterations in
+  // all), so the first batch rarely needs a second; iterations past the end
+  // cost three empty launches.
+  PNode* nodes = reinterpret_cast<PNode*>(ploc_nodes);
+  const SahTable table{cost, choice};
+  k_leaf_init<<<gb, 256, 0, st>>>(d_tris, perm, na, n);
+  k_ploc_start<<<1, 1, 0, st>>>(state, (uint32_t)n, acc);
   const size_t smem = (size_t)(kClusterThreads + 2 * r) * 6 * sizeof(float);
   if (smem > 48 * 1024)
     cudaFuncSetAttribute(k_neighbors,
                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)smem);
-  uint32_t merged_h = 0;
-  // the blocks of nodes each iteration finalises, in order (children
-  // before their parents), for the SAH collapse
-  std::vector<std::pair<uint64_t, uint64_t>> fin_blocks;
-  while (end - begin > 1) {
-    if (++iters > 100000)
-      return set_err(ctx, AJG_ERR_DEVICE, "PLOC did not converge");
-    const uint32_t cnt = (uint32_t)(end - begin);
-    const unsigned blocks = (cnt + kClusterThreads - 1) / kClusterThreads;
-    k_neighbors<<<blocks, kClusterThreads, smem, st>>>(
-        in, (uint32_t)begin, (uint32_t)end, r, nbr);
-    k_merge_flags<<<grid_for(cnt, 256), 256, 0, st>>>(nbr, (uint32_t)begin,
-                                                     (uint32_t)end, flags);
-    device_scan(flags, mi, cnt, false, scratch, st);
-    cudaMemcpyAsync(&merged_h, mi + cnt - 1, sizeof(uint32_t),
-                    cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess)
+  cudaFuncSetAttribute(k_cluster_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)sizeof(TailMem));
+  const int g_nb = grid_for(n, kClusterThreads, kSMs * 8);
+  const int g_pair = grid_for(n, kPairTile, kSMs * 8);
+  ShadingCopy shading{ctx};
+  PlocState h{};
+  int batch = n > kTail ? (int)std::ceil(std::log((double)n / kTail) / std::log(1.25)) + 1
+                        : 0;
+  uint64_t it = 0;
+  for (;;) {
+    for (int k = 0; k < batch; ++k, ++it) {
+      const int cur = (int)(it & 1);
+      k_neighbors<<<g_nb, kClusterThreads, smem, st>>>(state + cur, na, nbuf, r, nbr);
+      k_pairs<<<g_pair, kClusterThreads, 0, st>>>(state, cur, nbr, mate, tile_sum, acc);
+      k_cluster<<<g_pair, kClusterThreads, 0, st>>>(state, cur, na, nbuf, mate,
+                                                    tile_sum, nodes, table);
+    }
+    k_cluster_tail<<<1, kTailThreads, sizeof(TailMem), st>>>(
+        state, (int)(it & 1), na, nbuf, r, nodes, table);
+    if (!shading.started)  // beside the clustering
+      shading.start(d_mat, h_mat, d_flags, h_flags, corner, h_corner, n);
+    cudaError_t e = cudaMemcpyAsync(&h, state + (it & 1), sizeof(h),
+                                    cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess)
       return set_err(ctx, AJG_ERR_CUDA,
-                     std::string("PLOC build: ") +
-                         cudaGetErrorString(cudaGetLastError()));
-    if (merged_h == 0)
+                     std::string("PLOC build: ") + cudaGetErrorString(e));
+    if (h.stuck)
       return set_err(ctx, AJG_ERR_DEVICE, "PLOC iteration merged no pair");
-    const uint64_t merged = merged_h;
-    const uint64_t unmerged = cnt - merged;
-    const uint64_t children = merged * 2;
-    const uint64_t children_begin = end - children;
-    const uint64_t unmerged_begin = end - (children + unmerged);
-    fin_blocks.emplace_back(children_begin, end);
-    k_cluster_scatter<<<grid_for(cnt, 256), 256, 0, st>>>(
-        in, out, nbr, mi, (uint32_t)begin, (uint32_t)end,
-        (uint32_t)unmerged_begin, (uint32_t)children_begin);
-    if (pre_end > end)
-      cudaMemcpyAsync(out + end, in + end, (pre_end - end) * sizeof(PNode),
-                      cudaMemcpyDeviceToDevice, st);
-    std::swap(in, out);
-    pre_end = end;
-    begin = unmerged_begin;
-    end = children_begin;
+    if (h.cnt == 1) break;
+    if (h.iters > 100000)
+      return set_err(ctx, AJG_ERR_DEVICE, "PLOC did not converge");
+    batch = 8;
   }
-  const PNode* nodes = in;
-  fin_blocks.emplace_back(begin, end);  // the root
+  const uint32_t iters = h.iters;
 
   // traversal layout
-  cudaMemcpyAsync(ploc_nodes, nodes, m * sizeof(PNode),
-                  cudaMemcpyDeviceToDevice, st);
   cudaMemcpyAsync(perm_keep, perm, n * sizeof(int32_t),
                   cudaMemcpyDeviceToDevice, st);
   uint32_t num_nodes = (uint32_t)inner;
@@ -1009,74 +1349,65 @@ int build_scene(ajg_ctx* ctx, ajg_scene* s, const float* h_tris,
       k_bvh2_single<<<1, 1, 0, st>>>(nodes, bvh_bin);
     }
     // wide layout: collapse level by level into a worst-case buffer, then
-    // keep the nodes made
-    const uint64_t node_f4 =
-        compressed ? (wn == 8 ? CwLayout<8>::kFloat4 : CwLayout<4>::kFloat4)
-                   : 2 * (uint64_t)wn;
-    // the triangles move into node order for compressed nodes
+    // keep the nodes made; the triangles move into node order for compressed
+    // nodes.  wc: wide nodes, triangles moved, then the levels' lengths.
     k_slot_tris<<<gb, 256, 0, st>>>(d_tris, perm, n, slot_tris);
-    float4* wtmp = tmp.get<float4>(inner * node_f4);
-    float4* tri_tmp = compressed ? tmp.get<float4>(3 * n) : nullptr;
-    uint2* fa = tmp.get<uint2>(inner);
-    uint2* fb = tmp.get<uint2>(inner);
-    uint32_t* wc = tmp.get<uint32_t>(3);
-    if (tmp.err != cudaSuccess)
-      return set_err(ctx, AJG_ERR_OOM, "device allocation failed (wide BVH)");
-    const bool sah = AJG_SAH_COLLAPSE && wn == 4 && !compressed;
-    uint32_t* choice = nullptr;
-    if (sah) {
-      float4* cost = tmp.get<float4>(m);
-      choice = tmp.get<uint32_t>(m);
-      if (tmp.err != cudaSuccess)
-        return set_err(ctx, AJG_ERR_OOM, "device allocation failed (SAH collapse)");
-      for (const auto& b : fin_blocks) {
-        const uint32_t cnt = (uint32_t)(b.second - b.first);
-        k_sah_dp<<<grid_for(cnt, 256), 256, 0, st>>>(
-            nodes, (uint32_t)b.first, (uint32_t)b.second, cost, choice);
-      }
-    }
-    const uint32_t init[3] = {0u, 1u, 0u};
-    cudaMemcpyAsync(wc, init, sizeof(init), cudaMemcpyHostToDevice, st);
+    uint32_t init[3] = {1u, 0u, 1u};
     const uint2 root = make_uint2(0u, 0u);
     cudaMemcpyAsync(fa, &root, sizeof(root), cudaMemcpyHostToDevice, st);
-    uint32_t n_in = 1, levels = 0;
-    while (n_in) {
-      cudaMemsetAsync(wc, 0, sizeof(uint32_t), st);
-      const int g = grid_for(n_in, 128);
-      if (compressed && wn == 4)
-        k_collapse_c<4><<<g, 128, 0, st>>>(nodes, slot_tris, fa, n_in, fb, wc,
-                                           wtmp, tri_tmp);
-      else if (compressed)
-        k_collapse_c<8><<<g, 128, 0, st>>>(nodes, slot_tris, fa, n_in, fb, wc,
-                                           wtmp, tri_tmp);
-      else if (sah)
-        k_collapse_sah<<<g, 128, 0, st>>>(nodes, choice, fa, n_in, fb, wc,
-                                          wtmp);
-      else if (wn == 4)
-        k_collapse<4><<<g, 128, 0, st>>>(nodes, fa, n_in, fb, wc, wtmp);
-      else
-        k_collapse<8><<<g, 128, 0, st>>>(nodes, fa, n_in, fb, wc, wtmp);
-      uint32_t h[2] = {0, 0};
-      if (cudaMemcpyAsync(h, wc, sizeof(h), cudaMemcpyDeviceToHost, st) !=
+    const int g = grid_for(inner, 128, kSMs * 16);
+    int levels = std::min(kLevels, 6 + (int)(0.6 * std::log2((double)n)));
+    uint64_t done = 0;
+    for (;;) {
+      cudaMemsetAsync(wc + 3, 0, kLevels * sizeof(uint32_t), st);
+      cudaMemcpyAsync(wc, init, sizeof(init), cudaMemcpyHostToDevice, st);
+      for (int l = 0; l < levels; ++l) {
+        const uint32_t* ni = wc + 2 + l;
+        uint32_t* no = wc + 3 + l;
+        if (compressed && wn == 4)
+          k_collapse_c<4><<<g, 128, 0, st>>>(nodes, slot_tris, fa, ni, fb, no, wc,
+                                             wtmp, tri_tmp);
+        else if (compressed)
+          k_collapse_c<8><<<g, 128, 0, st>>>(nodes, slot_tris, fa, ni, fb, no, wc,
+                                             wtmp, tri_tmp);
+        else if (sah)
+          k_collapse_sah<<<g, 128, 0, st>>>(nodes, choice, fa, ni, fb, no, wc, wtmp);
+        else if (wn == 4)
+          k_collapse<4><<<g, 128, 0, st>>>(nodes, fa, ni, fb, no, wc, wtmp);
+        else
+          k_collapse<8><<<g, 128, 0, st>>>(nodes, fa, ni, fb, no, wc, wtmp);
+        std::swap(fa, fb);
+      }
+      uint32_t hw[2 + kLevels + 1];
+      if (cudaMemcpyAsync(hw, wc, sizeof(hw), cudaMemcpyDeviceToHost, st) !=
               cudaSuccess ||
           cudaStreamSynchronize(st) != cudaSuccess)
         return set_err(ctx, AJG_ERR_CUDA, "wide BVH collapse failed");
-      n_in = h[0];
-      num_nodes = h[1];
-      std::swap(fa, fb);
-      if (++levels > inner + 1)
+      num_nodes = hw[0];
+      if (hw[2 + levels] == 0) break;
+      done += levels;
+      if (done > inner + 1)
         return set_err(ctx, AJG_ERR_DEVICE, "wide BVH collapse did not end");
+      init[0] = hw[0];
+      init[1] = hw[1];
+      init[2] = hw[2 + levels];
+      levels = kLevels;
     }
-    bvh = (float4*)keep((uint64_t)num_nodes * node_f4 * sizeof(float4));
-    if (!bvh)
+    // (not device_malloc: the temporaries are in the kept scratch)
+    const uint64_t bytes = (uint64_t)num_nodes * node_f4 * sizeof(float4);
+    if (cudaMalloc((void**)&bvh, bytes) != cudaSuccess) {
+      cudaGetLastError();
       return set_err(ctx, AJG_ERR_OOM, "device allocation failed (wide BVH)");
-    cudaMemcpyAsync(bvh, wtmp, (uint64_t)num_nodes * node_f4 * sizeof(float4),
-                    cudaMemcpyDeviceToDevice, st);
+    }
+    s->allocations.push_back(bvh);
+    s->info.device_bytes += bytes;
+    cudaMemcpyAsync(bvh, wtmp, bytes, cudaMemcpyDeviceToDevice, st);
     if (compressed)
       cudaMemcpyAsync(slot_tris, tri_tmp, 3 * n * sizeof(float4),
                       cudaMemcpyDeviceToDevice, st);
   }
   if (width == 2) k_slot_tris<<<gb, 256, 0, st>>>(d_tris, perm, n, slot_tris);
+  cudaStreamWaitEvent(st, ctx->ev_queue, 0);
   k_shade_data<<<gb, 256, 0, st>>>(d_tris, d_mat, d_flags, n, shade);
   cudaEventRecord(e1, st);
   cudaError_t ce = cudaStreamSynchronize(st);
