@@ -1052,14 +1052,14 @@ int check_render(ajg_ctx* ctx, const DeviceScene& s, const ajg_camera& cam,
   return AJG_OK;
 }
 
-// Whether a pixel's samples fall within a few triangles of each other, so
-// that bounce 0's directional-light shadow rays pay as packets (a packet
-// walks the union of its rays' traversals, which near their origins grows
-// with the triangles they span): the pixel's footprint at the world box's
-// centre -- the angle between the rays through the film centre and the
-// pixel beside it, times the camera's distance to that centre -- against
-// kPacketSpread median triangle edges.
-static bool packets_pay(const ajg_scene* sc, const ajg_camera& cam) {
+// Bounce 0's directional-light shadow rays as packets (trace_packet_any): a
+// packet walks the union of its rays' traversals, which near their origins
+// grows with the triangles they span.  The measure is a pixel's footprint at
+// the world box's centre -- the angle between the rays through the film
+// centre and the pixel beside it, times the camera's distance to that centre
+// -- in median triangle edges (kPacketSpread of them: packet_spread), times
+// the pixels a packet of 32 spans when a wave holds S samples of each.
+static float packet_ratio(const ajg_scene* sc, const ajg_camera& cam) {
   auto apply = [](const float* m, const float v[4], float o[4]) {
     for (int r = 0; r < 4; ++r) {
       o[r] = 0.f;
@@ -1089,7 +1089,19 @@ static bool packets_pay(const ajg_scene* sc, const ajg_camera& cam) {
     const double e = (double)m[12 + k] / (m[15] != 0.f ? m[15] : 1.f) - c;
     dist2 += e * e;
   }
-  return angle * std::sqrt(dist2) <= (double)sc->d.packet_spread;
+  return (float)(angle * std::sqrt(dist2) / (double)sc->d.packet_spread);
+}
+// Packets pay up to one edge in waves of 4 Mi paths, half of one at 2 Mi (a
+// packet's walk is longer than a ray's, and a short launch waits for it), not
+// at all below.  Per-lane time over packet time of whole one-bounce renders
+// of displaced spheres, by span in edges: 2 Mi paths 0.24 1.015, 0.49 0.999,
+// 0.98 0.97; 4 Mi 0.49 1.03, 0.98 0.99 to 1.01, 1.96 0.91 to 0.95; 16 Mi and
+// more 0.98 1.03 to 1.05, 1.96 0.99, 3.9 0.90; 1 Mi 0.49 0.99, 3.9 0.79;
+// 262,144 paths 15.7 0.67, 31 0.61.
+bool packets_pay(const JobParams& j, uint64_t S, uint64_t paths) {
+  return paths >= (1u << 21) &&
+         j.packet_ratio * (float)((31 + S) / S) <=
+             std::min(1.f, (float)paths / (float)(1u << 22));
 }
 
 JobParams make_job_params(const ajg_scene* sc, const ajg_camera& cam,
@@ -1119,7 +1131,7 @@ JobParams make_job_params(const ajg_scene* sc, const ajg_camera& cam,
   j.x0 = j.y0 = 0;
   j.win_w = cam.width;
   j.win_h = cam.height;
-  j.packets = packets_pay(sc, cam) ? 1 : 0;
+  j.packet_ratio = packet_ratio(sc, cam);
   return j;
 }
 
@@ -1208,7 +1220,7 @@ static void run_waves(ajg_scene* sc, const ajg_camera& cam,
   // emitters use the top of the storage) over the plain 4-wide tree.
   uint32_t coh0 = 0;
   if (ctx->packet_shadow > 0 && !s.tri_emit && s.width == 4 && a.j.use_mis &&
-      (a.j.packets || ctx->packet_shadow >= 2)) {
+      (packets_pay(a.j, S, S * chunk) || ctx->packet_shadow >= 2)) {
     for (int l = 0; l < (int)s.num_lights && l < 31; ++l)
       if (ctx->packet_shadow == 2 ||
           (int)sc->host_lights[12 * l] == AJG_LIGHT_DIRECTIONAL)

@@ -54,13 +54,12 @@ struct DeviceScene {
   // AJG_HYBRID_CLOSEST=0)
   const float4* bvh_closest = nullptr;
   uint32_t num_inner_closest = 0;
-  // kPacketSpread times the scene's median triangle edge: a render traces
-  // bounce 0's directional-light shadow rays as packets when a pixel's
-  // footprint at the scene is within it
+  // kPacketSpread times the scene's median triangle edge: how far the rays of
+  // a packet may spread (packets_pay)
   float packet_spread = 0.f;
 };
 #ifndef AJG_PACKET_SPREAD
-#define AJG_PACKET_SPREAD 4.0f
+#define AJG_PACKET_SPREAD 1.0f
 #endif
 constexpr float kPacketSpread = AJG_PACKET_SPREAD;
 
@@ -116,7 +115,8 @@ struct JobParams {
   uint32_t film_w, film_h;
   uint32_t x0, y0, win_w, win_h;
   int32_t packets;  // bounce 0's directional-light shadow rays as packets
-  int32_t pad;
+                    // (multi-job waves: set per wave)
+  float packet_ratio;  // see packets_pay
 };
 
 // SPPM's visible point (TracerVP's result, sppm.cpp:77-92): the hit, its
@@ -532,6 +532,9 @@ void enqueue_resolve(const float4* fsum, const float4* fcomp,
                      bool fold_x, bool fold_y, float4* out, cudaStream_t st);
 int check_render(ajg_ctx* ctx, const DeviceScene& s, const ajg_camera& cam,
                  const ajg_render_params& prm);
+// Whether bounce 0's directional-light shadow rays go as packets in a wave
+// of `paths` paths that holds S samples of each pixel of the job.
+bool packets_pay(const JobParams& j, uint64_t S, uint64_t paths);
 JobParams make_job_params(const ajg_scene* sc, const ajg_camera& cam,
                           const ajg_render_params& prm);
 // The wave arena of a render of `npix` pixels (before any scratch is taken).

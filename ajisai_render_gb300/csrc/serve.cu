@@ -155,7 +155,7 @@ struct Server {
   std::vector<char*> h_tables;  // pinned, one per in-flight slot + 1
   size_t table_bytes = 0;
   uint64_t wave_no = 0;
-  std::map<std::tuple<int, int, int, bool>, cudaGraphExec_t> graphs;
+  std::map<std::tuple<int, int, int, bool, bool>, cudaGraphExec_t> graphs;
   std::deque<InFlight> inflight;
   std::vector<uint32_t*> err_words;  // pinned, recycled
   uint32_t* d_err = nullptr;
@@ -170,7 +170,8 @@ struct Server {
   void retire_oldest();
   void end_job_locked(Job* j, uint32_t state, int err);
   int ensure_arena(int nt, uint64_t target_paths);
-  cudaGraphExec_t graph_for(int bounces, int tri_test, int width, bool emit);
+  cudaGraphExec_t graph_for(int bounces, int tri_test, int width, bool emit,
+                            bool packets);
 };
 
 namespace {
@@ -220,8 +221,8 @@ int Server::ensure_arena(int nt, uint64_t target) {
 }
 
 cudaGraphExec_t Server::graph_for(int bounces, int tri_test, int width,
-                                  bool emit) {
-  const auto key = std::make_tuple(bounces, tri_test, width, emit);
+                                  bool emit, bool packets) {
+  const auto key = std::make_tuple(bounces, tri_test, width, emit, packets);
   auto it = graphs.find(key);
   if (it != graphs.end()) return it->second;
   prepare_mj_kernels();
@@ -232,7 +233,7 @@ cudaGraphExec_t Server::graph_for(int bounces, int tri_test, int width,
     return nullptr;
   enqueue_mj_wave(t, w, P, NT, bounces, tri_test, width, emit, d_ctr, d_err,
                   st, ctx->overlap ? ts : nullptr, ev_queue, ev_hits,
-                  ctx->packet_camera, ctx->packet_shadow > 0);
+                  ctx->packet_camera, packets);
   if (cudaStreamEndCapture(st, &g) != cudaSuccess || !g) return nullptr;
   if (cudaGraphInstantiate(&ex, g, 0) != cudaSuccess) ex = nullptr;
   cudaGraphDestroy(g);
@@ -519,6 +520,11 @@ bool Server::plan_and_launch() {
     path_off += p.n_pix * p.S;
     pix_off += p.n_pix;
   }
+  bool packets = false;  // a job of the wave takes them
+  for (size_t i = 0; i < plan.size() && ctx->packet_shadow > 0; ++i) {
+    hj[i].j.packets = packets_pay(hj[i].j, plan[i].S, path_off) ? 1 : 0;
+    packets |= hj[i].j.packets != 0;
+  }
   hdr->n_chunks = (uint32_t)plan.size();
   hdr->n_paths = path_off;
   hdr->n_pix = pix_off;
@@ -533,14 +539,14 @@ bool Server::plan_and_launch() {
   // the closest-hit MIS BSDF pass runs when a scene of the wave has emitters
   bool emit = false;
   for (const Plan& p : plan) emit |= p.job->scene->d.tri_emit != nullptr;
-  cudaGraphExec_t g = graph_for(bounces, tri_test, width, emit);
+  cudaGraphExec_t g = graph_for(bounces, tri_test, width, emit, packets);
   if (g) {
     cudaGraphLaunch(g, st);
   } else {  // capture unavailable: the same launches on the stream
     cudaGetLastError();
     enqueue_mj_wave(t, w, P, NT, bounces, tri_test, width, emit, d_ctr, d_err,
                     st, ctx->overlap ? ts : nullptr, ev_queue, ev_hits,
-                    ctx->packet_camera, ctx->packet_shadow > 0);
+                    ctx->packet_camera, packets);
   }
   // results this wave completes
   for (const Plan& p : plan) {
@@ -588,7 +594,7 @@ bool Server::plan_and_launch() {
     ++stats.waves;
     stats.paths += path_off;
     stats.kernel_launches +=
-        mj_wave_kernels(bounces, emit, width, ctx->packet_shadow > 0) +
+        mj_wave_kernels(bounces, emit, width, packets) +
         f.reports.size();
   }
   inflight.push_back(std::move(f));
