@@ -158,23 +158,22 @@ __global__ void k_bsdf_query(const ajg_material* __restrict__ mats,
     const float* m = reinterpret_cast<const float*>(mats + i);
     const float lum = (float)(0.2126 * (double)m[1] + 0.7152 * (double)m[2] +
                               0.0722 * (double)m[3]);
-    Bsdf f;
-    f.type = (int)mats[i].type;
-    f.ng = ld3(ng + 3 * i);
-    f.ns = ld3(ns + 3 * i);
-    f.m = m;
-    f.lum = lum;
+    const int type = (int)mats[i].type;
+    const F3 n_g = ld3(ng + 3 * i), n_s = ld3(ns + 3 * i), w_o = ld3(wo + 3 * i);
     float* o = out + 8 * i;
     if (op[i] == 0) {
-      const F3 v = f.eval(ld3(wi + 3 * i), ld3(wo + 3 * i));
+      F3 v;
+      float pdf;
+      bsdf_eval_pdf(type, m, lum, n_g, n_s, w_o, ld3(wi + 3 * i), v, pdf);
       o[0] = v.x;
       o[1] = v.y;
       o[2] = v.z;
-      o[3] = f.pdf(ld3(wi + 3 * i), ld3(wo + 3 * i));
+      o[3] = pdf;
       o[4] = o[5] = o[6] = 0.f;
       o[7] = 1.f;
     } else {
-      const BsdfSample s = f.sample(ld3(wo + 3 * i), ld3(sam + 3 * i));
+      const BsdfSample s =
+          bsdf_sample(type, m, lum, n_g, n_s, w_o, ld3(sam + 3 * i));
       o[0] = s.f.x;
       o[1] = s.f.y;
       o[2] = s.f.z;

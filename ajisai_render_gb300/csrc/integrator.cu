@@ -461,10 +461,8 @@ __global__ void __launch_bounds__(kShadeThreads, shade_min_blocks<MAT>())
       }
       T = xyz(w.thr[p]);
       hi = complete_hit(s, ro, rd, h.t, h.u, h.v, h.prim);
-      f.m = s.materials + 16 * hi.mat;
-      f.ng = hi.ng;
-      f.ns = hi.ns;
-      f.lum = __ldg(&s.mat_lum[hi.mat].x);
+      f.prepare(s.materials + 16 * hi.mat, __ldg(&s.mat_lum[hi.mat].x), hi.ng,
+                hi.ns, hi.wr);
       w.thr_shade[p] = make_float4(T.x, T.y, T.z, 0.f);
       // an emitter seen by a camera ray, or by any ray without MIS
       // (pt.cpp:185-190, 282-286; AreaLight::Radiance, area_light.cpp:30-34)
@@ -495,18 +493,54 @@ __global__ void __launch_bounds__(kShadeThreads, shade_min_blocks<MAT>())
       any_mis = __any_sync(kFull, mis);
     }
 
-    if (any_mis) {
-      for (int l = 0; l < nl_loop; ++l) {
-        const bool on = MJ ? (mis && l < nl) : hit;
-        const float* L = s.lights + 12 * (MJ ? (l < nl ? l : 0) : l);
-        bool emit = false;
-        F3 fo = mk3(0, 0, 0), so = mk3(0, 0, 0), sd = mk3(0, 0, 1);
-        float tmax = 0.f;
-        int draws = 2;
+    // SPPM's camera pass ends a path at its first diffuse surface or its
+    // last bounce with a visible point (sppm.cpp:77-92)
+    bool vp_here = false;
+    if constexpr (!MJ) {
+      if (a.vp && hit) {
+        bool diffuse;
+        if (MAT == AJG_MAT_DIFFUSE)
+          diffuse = true;
+        else if (MAT == AJG_MAT_DISNEY)
+          diffuse = f.m[5] < 1.f;  // DisneyBSDF: metallic < 1
+        else
+          diffuse = (int)f.m[0] == AJG_MAT_PLASTIC;
+        vp_here = diffuse || b == J.max_b - 1;
+        if (vp_here && isfinite(T.x) && isfinite(T.y) && isfinite(T.z)) {
+          VisPointD v;
+          v.pos = make_float4(hi.pos.x, hi.pos.y, hi.pos.z,
+                              __uint_as_float(hi.mat));
+          v.wr = make_float4(hi.wr.x, hi.wr.y, hi.wr.z, 0.f);
+          v.thr = make_float4(T.x, T.y, T.z, 0.f);
+          v.ng = make_float4(hi.ng.x, hi.ng.y, hi.ng.z, 0.f);
+          v.ns = make_float4(hi.ns.x, hi.ns.y, hi.ns.z, 0.f);
+          a.vp[a.pix0 + p / a.S] = v;
+        }
+      }
+    }
+
+    // The hit's directions, a round each: a sample per light, the MIS BSDF
+    // sample, the continuation.  A round draws a direction, evaluates the BSDF
+    // there and appends its ray.  Lanes without MIS only continue.
+    DisneyB::Stretched stretched;
+    if constexpr (BsdfT<MAT>::kDisney)
+      if (hit) stretched = f.b.stretched();
+    enum Kind { kLight, kMisBsdf, kContinue };
+    auto round = [&](Kind kind, int t_) __attribute__((always_inline)) {
+      const bool is_light = kind == kLight, is_mis = kind == kMisBsdf;
+      bool on, lit = false;  // lit: `wl` is a direction to evaluate
+      F3 wl = mk3(0, 0, 1), lrad = mk3(0, 0, 0);
+      float lpdf = 0.f, len = 0.f;
+      int type = -1, draws = 3;
+      const float* L = s.lights;
+      BsdfSample bs = invalid_sample();
+      if (is_light) {
+        on = MJ ? (mis && t_ < nl) : hit;
+        L = s.lights + 12 * (MJ ? (t_ < nl ? t_ : 0) : t_);
+        draws = 2;
         if (on) {
-          F3 lpos, lrad;
-          float lpdf;
-          const int type = (int)L[0];
+          F3 lpos;
+          type = (int)L[0];
           bool ok = true;
           if (type == kLightArea) {
             // AreaLight::Sample (area_light.cpp:36-57): three draws
@@ -556,149 +590,157 @@ __global__ void __launch_bounds__(kShadeThreads, shade_min_blocks<MAT>())
             }
           }
           if (ok && !(black3(lrad) || lpdf <= 0.f)) {
-            const float len = len3(lpos - hi.pos) - kRayEps;
+            len = len3(lpos - hi.pos) - kRayEps;
             if (!(len < kRayEps)) {
-              const F3 wl = normalize3(lpos - hi.pos);
-              F3 bf;
-              float bp;
-              f.eval_pdf(wl, hi.wr, bf, bp);
-              if (!black3(bf)) {
-                // MISSampleAreaLight takes the shading normal as it is, the
-                // others normalise it (helper.h:64, 91, 120)
-                const F3 nn = type == kLightArea ? hi.ns : normalize3(hi.ns);
-                F3 fv;
-                if (type != AJG_LIGHT_ENV)
-                  fv = mk3(1.f, 1.f, 1.f) * lrad * bf * fabsf(dot3(wl, nn));
-                else
-                  fv = lrad * bf * fabsf(dot3(wl, nn));
-                fo = fv / lpdf * power_heuristic(lpdf, bp);
-                make_ray(hi.pos, wl, so, sd);
-                tmax = 0.99f * len;
-                emit = true;
-              }
+              wl = normalize3(lpos - hi.pos);
+              lit = true;
             }
           }
-          const uint32_t slot = p * NT + l;
-          w.term_f[slot] = make_float4(fo.x, fo.y, fo.z, 0.f);
-          w.term_vis[slot] = 0;
         }
-        // to the packet queue: this term's rays (a single job), or a lane's
-        // directional-light rays when its job's footprint allows packets
-        // (multi-job lanes differ in their l-th light and their job)
-        const bool top =
-            MJ ? (coh != 0 && on && J.packets &&
-                  (int)L[0] == AJG_LIGHT_DIRECTIONAL)
-               : (l < 31 && ((coh >> l) & 1u));
-        emit_shadow<MJ>(w, so, sd, tmax, p * NT + l, sid, emit, shadow_cap,
-                        err, top, MJ && coh != 0);
-        if (on) dim += draws;
+      } else {
+        on = is_mis ? (MJ ? mis : hit) : hit && !vp_here && b + 1 < J.max_b;
+        if (on) {
+          const F3 sam = mk3(key_float(key, dim), key_float(key, dim + 1),
+                             key_float(key, dim + 2));
+          if constexpr (BsdfT<MAT>::kDisney) {
+            const F3 lwi = f.b.sample_dir(sam, stretched);
+            if (!(lwi.z <= 0.0f)) {
+              wl = f.b.frame().to_world(lwi);
+              lit = true;
+            }
+          } else {
+            bs = f.sample(sam);
+          }
+        }
       }
-      {
+      F3 bf = mk3(0, 0, 0);
+      float bp = 0.f;
+      if (lit) f.eval_pdf(wl, bf, bp, !is_light);
+      if constexpr (BsdfT<MAT>::kDisney) {
+        if (!is_light && lit) {
+          bs.dir = wl;
+          bs.f = bf;
+          bs.pdf = bp;
+        }
+      }
+
+      if (kind == kContinue) {
+        // the continuation sample (pt.cpp:215-223)
+        bool alive = false;
+        F3 nro = mk3(0, 0, 0), nrd = mk3(0, 0, 1);
+        if (on) {
+          if (!(black3(bs.f) || bs.pdf < 0.f)) {
+            T = T * (bs.f * fabsf(dot3(hi.ng, bs.dir)) / bs.pdf);
+            make_ray(eps_offset(hi, bs.dir), bs.dir, nro, nrd);
+            alive = true;
+            if (b + 1 > J.min_b) {
+              if (key_float(key, dim_base(J, b + 1)) > J.cont)
+                alive = false;
+              else
+                T = T / J.cont;
+            }
+          }
+          w.thr[p] = make_float4(T.x, T.y, T.z, 0.f);
+        }
+        const uint32_t kn = shade_append(&w.counts[nxt], alive);
+        if (alive) {
+          w.qpath[nxt][kn] = p;
+          w.ro[nxt][kn] = make_float4(nro.x, nro.y, nro.z, __uint_as_float(sid));
+          w.rd[nxt][kn] = make_float4(nrd.x, nrd.y, nrd.z, 0.f);
+        }
+        return;
+      }
+
+      // a shadow ray (or an emitter scene's closest-hit ray) of the term
+      bool emit = false, closest = false;
+      F3 fo = mk3(0, 0, 0), so = mk3(0, 0, 0), sd = mk3(0, 0, 1);
+      float tmax = __int_as_float(0x7f800000);
+      float w_o = __int_as_float(0x7f800000), cosv = 0.f;
+      if (is_light) {
+        if (lit && !black3(bf)) {
+          // MISSampleAreaLight takes the shading normal as it is, the
+          // others normalise it (helper.h:64, 91, 120)
+          const F3 nn = type == kLightArea ? hi.ns : normalize3(hi.ns);
+          F3 fv;
+          if (type != AJG_LIGHT_ENV)
+            fv = mk3(1.f, 1.f, 1.f) * lrad * bf * fabsf(dot3(wl, nn));
+          else
+            fv = lrad * bf * fabsf(dot3(wl, nn));
+          fo = fv / lpdf * power_heuristic(lpdf, bp);
+          make_ray(hi.pos, wl, so, sd);
+          tmax = 0.99f * len;
+          emit = true;
+        }
+      } else if (on && !(black3(bs.f) || bs.pdf == 0.f)) {
         // MISSampleBsdf (helper.h:209-265).  Without emitters only the
         // environment can answer, and an any-hit escape test decides; with
         // emitters the closest hit decides, so the ray goes to the closest
         // queue with the BSDF value and |cos| parked in its term and the pdf
         // in the ray (k_bsdf_emit completes the term).
-        const bool on = MJ ? mis : hit;
-        bool emit = false, closest = false;
-        F3 fo = mk3(0, 0, 0), so = mk3(0, 0, 0), sd = mk3(0, 0, 1);
-        float w_o = __int_as_float(0x7f800000);
-        float cosv = 0.f;
-        if (on) {
-          const F3 sam = mk3(key_float(key, dim), key_float(key, dim + 1),
-                             key_float(key, dim + 2));
-          BsdfSample bs = f.sample(hi.wr, sam);
-          if (!(black3(bs.f) || bs.pdf == 0.f)) {
-            if (s.tri_emit) {
-              bs.dir = normalize3(bs.dir);
-              make_ray(eps_offset(hi, bs.dir), bs.dir, so, sd);
-              fo = bs.f;
-              cosv = fabsf(dot3(hi.ns, sd));
-              w_o = bs.delta ? -bs.pdf : bs.pdf;  // a delta sample: negated
-              closest = true;
-            } else if (s.env >= 0) {
-              bs.dir = normalize3(bs.dir);
-              make_ray(eps_offset(hi, bs.dir), bs.dir, so, sd);
-              const F3 rad = mk3(J.env_rgb.x, J.env_rgb.y, J.env_rgb.z);
-              if (!black3(rad)) {
-                const F3 fv = rad * bs.f * fabsf(dot3(hi.ns, sd));
-                // a delta sample is not weighted (helper.h:236-241)
-                if (bs.delta) {
-                  fo = mk3(0, 0, 0) + fv / bs.pdf;
-                } else {
-                  const float lp = env_pdf(J.env_mass != 0, sd);
-                  fo = mk3(0, 0, 0) +
-                       fv / bs.pdf * power_heuristic(bs.pdf, lp);
-                }
-                emit = true;
-              }
+        if (s.tri_emit) {
+          bs.dir = normalize3(bs.dir);
+          make_ray(eps_offset(hi, bs.dir), bs.dir, so, sd);
+          fo = bs.f;
+          cosv = fabsf(dot3(hi.ns, sd));
+          w_o = bs.delta ? -bs.pdf : bs.pdf;  // a delta sample: negated
+          closest = true;
+        } else if (s.env >= 0) {
+          bs.dir = normalize3(bs.dir);
+          make_ray(eps_offset(hi, bs.dir), bs.dir, so, sd);
+          const F3 rad = mk3(J.env_rgb.x, J.env_rgb.y, J.env_rgb.z);
+          if (!black3(rad)) {
+            const F3 fv = rad * bs.f * fabsf(dot3(hi.ns, sd));
+            // a delta sample is not weighted (helper.h:236-241)
+            if (bs.delta) {
+              fo = mk3(0, 0, 0) + fv / bs.pdf;
+            } else {
+              const float lp = env_pdf(J.env_mass != 0, sd);
+              fo = mk3(0, 0, 0) +
+                   fv / bs.pdf * power_heuristic(bs.pdf, lp);
             }
+            emit = true;
           }
-          const uint32_t slot = p * NT + (NT - 1);
-          w.term_f[slot] = make_float4(fo.x, fo.y, fo.z, cosv);
-          w.term_vis[slot] = 0;
-          dim += 3;
-        }
-        emit_shadow<MJ>(w, so, sd, __int_as_float(0x7f800000),
-                        p * NT + (NT - 1), sid, emit, shadow_cap, err,
-                        !MJ && ((coh >> 31) & 1u));
-        // (a single job's scene without emitters never fills this queue:
-        // skip its block-wide append; the condition is uniform)
-        if (MJ || s.tri_emit)
-          emit_closest<MJ>(w, so, sd, w_o, p * NT + (NT - 1), sid, closest,
-                           shadow_cap, err);
-      }
-    }
-
-    // SPPM's camera pass ends a path at its first diffuse surface or its
-    // last bounce with a visible point (sppm.cpp:77-92)
-    bool vp_here = false;
-    if constexpr (!MJ) {
-      if (a.vp && hit) {
-        bool diffuse;
-        if (MAT == AJG_MAT_DIFFUSE)
-          diffuse = true;
-        else if (MAT == AJG_MAT_DISNEY)
-          diffuse = f.m[5] < 1.f;  // DisneyBSDF: metallic < 1
-        else
-          diffuse = (int)f.m[0] == AJG_MAT_PLASTIC;
-        vp_here = diffuse || b == J.max_b - 1;
-        if (vp_here && isfinite(T.x) && isfinite(T.y) && isfinite(T.z)) {
-          VisPointD v;
-          v.pos = make_float4(hi.pos.x, hi.pos.y, hi.pos.z,
-                              __uint_as_float(hi.mat));
-          v.wr = make_float4(hi.wr.x, hi.wr.y, hi.wr.z, 0.f);
-          v.thr = make_float4(T.x, T.y, T.z, 0.f);
-          v.ng = make_float4(hi.ng.x, hi.ng.y, hi.ng.z, 0.f);
-          v.ns = make_float4(hi.ns.x, hi.ns.y, hi.ns.z, 0.f);
-          a.vp[a.pix0 + p / a.S] = v;
         }
       }
-    }
-    bool alive = false;
-    F3 nro = mk3(0, 0, 0), nrd = mk3(0, 0, 1);
-    if (hit && !vp_here && b + 1 < J.max_b) {
-      const F3 sam = mk3(key_float(key, dim), key_float(key, dim + 1),
-                         key_float(key, dim + 2));
-      const BsdfSample bs = f.sample(hi.wr, sam);
-      if (!(black3(bs.f) || bs.pdf < 0.f)) {
-        T = T * (bs.f * fabsf(dot3(hi.ng, bs.dir)) / bs.pdf);
-        make_ray(eps_offset(hi, bs.dir), bs.dir, nro, nrd);
-        alive = true;
-        if (b + 1 > J.min_b) {
-          if (key_float(key, dim_base(J, b + 1)) > J.cont)
-            alive = false;
-          else
-            T = T / J.cont;
-        }
+      const uint32_t slot = p * NT + (is_mis ? NT - 1 : (uint32_t)t_);
+      if (on) {
+        w.term_f[slot] = make_float4(fo.x, fo.y, fo.z, cosv);
+        w.term_vis[slot] = 0;
+        dim += draws;
       }
-      w.thr[p] = make_float4(T.x, T.y, T.z, 0.f);
-    }
-    const uint32_t kn = shade_append(&w.counts[nxt], alive);
-    if (alive) {
-      w.qpath[nxt][kn] = p;
-      w.ro[nxt][kn] = make_float4(nro.x, nro.y, nro.z, __uint_as_float(sid));
-      w.rd[nxt][kn] = make_float4(nrd.x, nrd.y, nrd.z, 0.f);
+      // to the packet queue: this term's rays (a single job), or a lane's
+      // directional-light rays when its job's footprint allows packets
+      // (multi-job lanes differ in their t-th light and their job)
+      bool top;
+      if (is_mis)
+        top = !MJ && ((coh >> 31) & 1u);
+      else
+        top = MJ ? (coh != 0 && on && J.packets &&
+                    (int)L[0] == AJG_LIGHT_DIRECTIONAL)
+                 : (t_ < 31 && ((coh >> t_) & 1u));
+      emit_shadow<MJ>(w, so, sd, tmax, slot, sid, emit, shadow_cap, err, top,
+                      MJ && coh != 0 && is_light);
+      // (a single job's scene without emitters never fills this queue: skip
+      // its block-wide append; the condition is uniform)
+      if (is_mis && (MJ || s.tri_emit))
+        emit_closest<MJ>(w, so, sd, w_o, slot, sid, closest, shadow_cap, err);
+    };
+    if constexpr (BsdfT<MAT>::kDisney) {
+      // one loop: the BSDF's sample and evaluation are at one site each, so
+      // they are inlined with the hit's terms in registers and the kernel
+      // fits the instruction cache.  (Three sites with out-of-line calls:
+      // 9.7 ms of shading a 1024x1024x32 render of the 1.3 M-triangle
+      // sphere, its terms prepared in local memory 10.7, this loop 7.6.)
+      for (int t = any_mis ? 0 : nl_loop + 1; t < nl_loop + 2; ++t)
+        round(t < nl_loop ? kLight : (t == nl_loop ? kMisBsdf : kContinue), t);
+    } else {
+      // the kinds apart: each is short and needs fewer registers (256x256x64
+      // Cornell box: 1.67 ms, one loop 1.82)
+      if (any_mis) {
+        for (int t = 0; t < nl_loop; ++t) round(kLight, t);
+        round(kMisBsdf, nl_loop);
+      }
+      round(kContinue, nl_loop + 1);
     }
   }
 }

@@ -6,6 +6,7 @@
 // within a few ulp of the reference rather than bit-equal.
 #pragma once
 #include <cfloat>
+#include <type_traits>
 
 #include "common.cuh"
 #include "scene.cuh"
@@ -33,9 +34,13 @@ __device__ __forceinline__ float clampf(float v, float lo, float hi) {
 // CoordinateSystem (core/coordinate_system.h:37-52)
 struct Frame {
   F3 dx, dy, dz;
-  __device__ __forceinline__ explicit Frame(F3 n) : dz(n) {
+  // the division of the construction, for callers that keep it
+  static __device__ __forceinline__ float scale(F3 n) {
+    return -1.f / (copysignf(1.f, n.z) + n.z);
+  }
+  __device__ __forceinline__ explicit Frame(F3 n) : Frame(n, scale(n)) {}
+  __device__ __forceinline__ Frame(F3 n, float a) : dz(n) {
     const float sign = copysignf(1.f, n.z);
-    const float a = -1.f / (sign + n.z);
     const float b = n.x * n.y * a;
     dx = mk3(1.f + sign * n.x * n.x * a, sign * b, -sign * n.x);
     dy = mk3(b, sign + n.y * n.y * a, -n.y);
@@ -110,67 +115,46 @@ __device__ __forceinline__ BsdfSample invalid_sample() {
   return s;
 }
 
-struct MatParams {
-  int type;
-  F3 base;
-  float subsurface, metallic, specular, specular_tint, roughness, sheen,
-      sheen_tint, clearcoat, clearcoat_gloss, lum;
-};
-__device__ __forceinline__ MatParams load_material(const float* m,
-                                                   float lum) {
-  MatParams p;
-  p.type = (int)m[0];
-  p.base = mk3(m[1], m[2], m[3]);
-  p.subsurface = m[4];
-  p.metallic = m[5];
-  p.specular = m[6];
-  p.specular_tint = m[7];
-  p.roughness = m[8];
-  p.sheen = m[10];
-  p.sheen_tint = m[11];
-  p.clearcoat = m[12];
-  p.clearcoat_gloss = m[13];
-  p.lum = lum;
-  return p;
-}
-
 // ----------------------------------------------------------- Lambertian --
 // Diffuse::Shade -> AggregateBSDF{DiffuseComponent, weight 1}
 // (core/material/diffuse.cpp:35-48, core/bsdf/aggregate_bsdf.cpp:43-131,
 // core/bsdf/diffuse_component.cpp:28-64, core/bsdf/bsdf.cpp:30-63)
+// A hit's Lambertian lobe for one outgoing direction: what every evaluation
+// and sample of the hit shares (the frame, which side `wo` is on, the lobe's
+// value) is computed once, by the same operations.
 struct Lambert {
-  F3 ng, ns, albedo, coef;
-  __device__ __forceinline__ Lambert(F3 ng_, F3 ns_, F3 alb)
-      : ng(ng_), ns(ns_), albedo(alb), coef(alb / kPi) {}
-  __device__ __forceinline__ bool fringes(F3 w) const {
-    return (dot3(ng, w) > 0) != (dot3(ns, w) > 0);
+  F3 ng, ns, coef;
+  float fa;      // Frame(ns)'s division
+  bool fringe;   // wo is on different sides of the two normals
+  bool below;    // wo leaves it no lobe: under ng (a fringe), or under ns
+  bool above_g;  // wo is above ng
+  __device__ __forceinline__ void prepare(F3 ng_, F3 ns_, F3 albedo, F3 wo) {
+    ng = ng_;
+    ns = ns_;
+    coef = albedo / kPi;
+    const float cg = dot3(ng, wo);
+    above_g = cg > 0;
+    fringe = above_g != (dot3(ns, wo) > 0);
+    fa = Frame::scale(ns);
+    below = fringe ? cg <= 0.f : normalize3(frame().to_local(wo)).z <= 0.f;
   }
-  __device__ __forceinline__ BsdfSample sample(F3 wo, F3 sam) const {
-    if (fringes(wo)) {
-      if (dot3(ng, wo) <= 0.f) return invalid_sample();
-      float pdf;
-      const F3 lwi = cosine_hemisphere(sam.x, sam.y, &pdf);
-      if (pdf < FLT_EPSILON) return invalid_sample();
-      const F3 wi = normalize3(Frame(ng).to_world(lwi));
-      const float factor = correct_shading_normal(ng, ns, wi);
-      BsdfSample s;
-      s.dir = wi;
-      s.f = albedo / kPi * factor;
-      s.pdf = pdf;
-      return s;
-    }
-    const Frame sf(ns);
-    const F3 lwo = normalize3(sf.to_local(wo));
-    if (lwo.z <= 0.f) return invalid_sample();
+  __device__ __forceinline__ Frame frame() const { return Frame(ns, fa); }
+  __device__ __forceinline__ BsdfSample sample(F3 sam) const {
+    if (below) return invalid_sample();
     float pdf;
-    F3 lwi = cosine_hemisphere(sam.y, sam.z, &pdf);
+    F3 lwi = fringe ? cosine_hemisphere(sam.x, sam.y, &pdf)
+                    : cosine_hemisphere(sam.y, sam.z, &pdf);
     // pdf < 1e-3 compares in double in the reference
     // (diffuse_component.cpp:39); for a float pdf that is pdf < 1e-3f
     // exactly, as no float lies in [1e-3, 1e-3f)
-    if (pdf < 1e-3f) return invalid_sample();
-    lwi = normalize3(lwi);
-    pdf *= 1.f;
-    const F3 wi = sf.to_world(lwi);
+    if (pdf < (fringe ? FLT_EPSILON : 1e-3f)) return invalid_sample();
+    F3 wi;
+    if (fringe) {
+      wi = normalize3(Frame(ng).to_world(lwi));
+    } else {
+      lwi = normalize3(lwi);
+      wi = frame().to_world(lwi);
+    }
     const float factor = correct_shading_normal(ng, ns, wi);
     BsdfSample s;
     s.dir = wi;
@@ -178,31 +162,32 @@ struct Lambert {
     s.pdf = pdf;
     return s;
   }
-  __device__ F3 eval(F3 wi, F3 wo) const {
-    if (fringes(wo)) {
-      if ((dot3(ng, wi) <= 0.f) || (dot3(ng, wo) <= 0.f)) return mk3(0, 0, 0);
-      return albedo / kPi;
+  __device__ __forceinline__ float pdf(F3 wi) const {
+    if (fringe) {
+      if ((dot3(ng, wi) > 0.f) != above_g) return 0.f;
+      return normalize3(Frame(ng).to_local(wi)).z * kInvPi;
     }
-    const Frame sf(ns);
-    const F3 lwi = normalize3(sf.to_local(wi));
-    const F3 lwo = normalize3(sf.to_local(wo));
-    if (lwi.z <= 0.f || lwo.z <= 0.f) return mk3(0, 0, 0);
-    return mk3(0, 0, 0) + coef;
+    if (below) return 0.f;
+    const float z = normalize3(frame().to_local(wi)).z;
+    return z <= 0.f ? 0.f : z * kInvPi;
   }
-  __device__ float pdf(F3 wi, F3 wo) const {
-    if (fringes(wo)) {
-      if ((dot3(ng, wi) > 0.f) != (dot3(ng, wo) > 0.f)) return 0.f;
-      const F3 local = normalize3(Frame(ng).to_local(wi));
-      return local.z * kInvPi;
+  // f, and its pdf where f is not 0
+  __device__ __forceinline__ void eval_pdf(F3 wi, F3& f, float& pdf) const {
+    f = mk3(0, 0, 0);
+    pdf = 0.f;
+    if (below) return;
+    if (fringe) {
+      const float cg = dot3(ng, wi);
+      if (cg <= 0.f) return;
+      f = coef;
+      if ((cg > 0.f) == above_g)
+        pdf = normalize3(Frame(ng).to_local(wi)).z * kInvPi;
+      return;
     }
-    const Frame sf(ns);
-    const F3 lwi = normalize3(sf.to_local(wi));
-    const F3 lwo = normalize3(sf.to_local(wo));
-    if (lwi.z <= 0.f || lwo.z <= 0.f) return 0.f;
-    float wsum = 0.f, p = 0.f;
-    wsum += 1.f;
-    p += 1.f * (lwi.z * kInvPi);
-    return wsum > 0 ? p / wsum : 0;
+    const float z = normalize3(frame().to_local(wi)).z;
+    if (z <= 0.f) return;
+    f = mk3(0, 0, 0) + coef;
+    pdf = z * kInvPi;
   }
 };
 
@@ -278,50 +263,114 @@ __host__ __device__ __forceinline__ float vndf_fit_z(float u2f) {
 
 // --------------------------------------------------------------- Disney --
 // DisneyBSDF (core/material/disney.cpp:58-473)
+// A hit's Disney lobes for one outgoing direction.  What every evaluation
+// and sample of the hit shares -- wo in the frame, its masking terms and
+// clearcoat probabilities, and the visible normals' stretched direction -- is
+// computed once per hit, by the same operations as the reference's per-call
+// code, so every result is bit-equal to it.
 struct DisneyB {
-  const MatParams& m;
-  Frame sf;
-  __device__ __forceinline__ DisneyB(const MatParams& mat, F3 ns)
-      : m(mat), sf(ns) {}
+  const float* m;  // [16] record
+  F3 ns, wo, lwo;
+  float lum;
+  float fa;                      // Frame(ns)'s division
+  float pc_local, pc_world;      // clearcoat probability at lwo, at wo
+  float tt;                      // |tan theta| of lwo
+  float g_spec, g_coat, g_pdf;   // its masking at alpha_g, 0.25, alpha
+  float tt_w, g_w;               // |tan theta| of wo, its masking at the
+                                 // clearcoat's sampling alpha
+  struct Stretched {             // sample_vn's share of lwo and an alpha
+    float theta, sin_phi, cos_phi, tan_theta, a, g1;
+  };
 
+  // the material's derived parameters
+  __device__ __forceinline__ F3 base() const { return mk3(m[1], m[2], m[3]); }
+  __device__ __forceinline__ float rough() const { return clampf(m[8], 0.02f, 1.f); }
+  __device__ __forceinline__ float alpha() const { return rough() * rough(); }
+  __device__ __forceinline__ float alpha_g() const {
+    const float rg = (0.5f + 0.5f * rough());
+    return rg * rg;
+  }
+  __device__ __forceinline__ float nr() const { return std_lerp(0.f, 0.08f, m[6]); }
+  __device__ __forceinline__ float coat_alpha() const {
+    return std_lerp(0.005f, 0.10f, m[13]);
+  }
+  __device__ __forceinline__ Frame frame() const { return Frame(ns, fa); }
+
+  static __device__ __forceinline__ float masking(float tt, float alpha) {
+    const float root = alpha * tt;
+    return 2.0f / (1.0f + sqrtf(1.0f + root * root));
+  }
+  // smith_g with its value `g` for the visible side; vh = dot3(v, wh)
+  static __device__ __forceinline__ float smith(float tt, float vh, float vz,
+                                                float g) {
+    if (tt == 0.0f) return 1.0f;
+    if (vh * vz <= 0) return 0.0f;
+    return g;
+  }
+  __device__ __forceinline__ float coat_prob(float z) const {
+    const float cw = m[12] / (m[12] + lum);
+    const float fc = fresnel_coat(fabsf(z));
+    return (fc * cw) / (fc * cw + (1.f - fc) * (1.f - cw));
+  }
+  __device__ __forceinline__ void prepare(const float* __restrict__ m_, float lum_,
+                                          F3 ns_, F3 wo_) {
+    m = m_;
+    lum = lum_;
+    ns = ns_;
+    wo = wo_;
+    fa = Frame::scale(ns);
+    lwo = normalize3(frame().to_local(wo));
+    tt = fabsf(tan_theta(lwo));
+    g_spec = masking(tt, alpha_g());
+    g_pdf = masking(tt, alpha());
+    pc_local = pc_world = g_coat = tt_w = g_w = 0.f;
+    if (m[12] != 0.0f) {
+      g_coat = masking(tt, 0.25f);
+      // the clearcoat lobe's pdf reads the world-space wo
+      // (disney.cpp:208-220), its sampling the local one
+      pc_local = coat_prob(lwo.z);
+      pc_world = coat_prob(wo.z);
+      tt_w = fabsf(tan_theta(wo));
+      g_w = masking(tt_w, coat_alpha());
+    }
+  }
   __device__ static float tan_theta(F3 v) {
     const float temp = 1 - v.z * v.z;
     if (temp <= 0.0f) return 0.0f;
     return sqrtf(temp) / v.z;
   }
-  __device__ static float tan2(F3 v) {
-    const float tmp = 1.f - v.z * v.z;
-    if (tmp <= 0.f) return 0.f;
-    return tmp / (v.z * v.z);
-  }
   __device__ static F3 reflect(F3 vi, F3 n) {
     return vi + (2 * dot3(-vi, n) * n);
   }
-  __device__ static float ggx_d(F3 wh, float alpha) {
-    if (wh.z <= 0.f) return 0.f;
-    const float t2 = tan2(wh);
-    const float c2 = wh.z * wh.z;
+  // GGX's D of wh with c2 = wh.z^2 and t2 = tan^2 theta
+  __device__ static __forceinline__ float ggx_d(float z, float c2, float t2,
+                                                float alpha) {
+    if (z <= 0.f) return 0.f;
     const float root = alpha / (c2 * (alpha * alpha + t2));
     return kInvPi * (root * root);
   }
-  __device__ static float smith_g(F3 v, F3 wh, float alpha) {
-    const float tt = fabsf(tan_theta(v));
-    if (tt == 0.0f) return 1.0f;
-    if (dot3(v, wh) * v.z <= 0) return 0.0f;
-    const float root = alpha * tt;
-    return 2.0f / (1.0f + sqrtf(1.0f + root * root));
+  __device__ static __forceinline__ Stretched stretch(F3 v, float alpha) {
+    const F3 w = normalize3(mk3(alpha * v.x, alpha * v.y, v.z));
+    float phi = 0;
+    Stretched t;
+    t.theta = 0;
+    if (w.z < 0.99999f) {
+      t.theta = acosf(w.z);
+      phi = atan2f(w.y, w.x);
+    }
+    t.sin_phi = sinf(phi);
+    t.cos_phi = cosf(phi);
+    t.tan_theta = t.a = t.g1 = 0.f;
+    if (!(t.theta < 1e-4f)) {
+      t.tan_theta = tanf(t.theta);
+      t.a = 1 / t.tan_theta;
+      t.g1 = 2.0f / (1.0f + sqrtf(ref_max(1.0f + 1.0f / (t.a * t.a), 0.0f)));
+    }
+    return t;
   }
-  __device__ static float ggx_g(F3 wi, F3 wo, F3 wh, float alpha) {
-    return smith_g(wo, wh, alpha) * smith_g(wi, wh, alpha);
-  }
-  __device__ static float pdf_vn(F3 wi, F3 h, float alpha) {
-    const float D = ggx_d(h, alpha);
-    return smith_g(wi, h, alpha) * fabsf(dot3(wi, h)) * D /
-           (fabsf(wi.z) + 1e-4f);
-  }
-  __device__ static void vn_unit(float thetaI, float u1, float u2, float& sx,
-                                 float& sy) {
-    if (thetaI < 1e-4f) {
+  __device__ static __forceinline__ void vn_unit(const Stretched& t, float u1,
+                                                 float u2, float& sx, float& sy) {
+    if (t.theta < 1e-4f) {
       const float R = sqrtf(ref_max(u1 / ((1 - u1) + 1e-6f), 0.0f));
       const float SinPhi = sinf(2 * kPi * u2);
       const float CosPhi = cosf(2 * kPi * u2);
@@ -329,18 +378,15 @@ struct DisneyB {
       sy = R * SinPhi;
       return;
     }
-    const float TanThetaI = tanf(thetaI);
-    const float a = 1 / TanThetaI;
-    const float G1 = 2.0f / (1.0f + sqrtf(ref_max(1.0f + 1.0f / (a * a), 0.0f)));
-    float A = 2.0f * u1 / G1 - 1.0f;
+    float A = 2.0f * u1 / t.g1 - 1.0f;
     if (fabsf(A) == 1) A -= (A >= 0.0f ? 1.0f : -1.0f) * 1e-4f;
     const float Temp = 1.0f / (A * A - 1.0f);
-    const float B = TanThetaI;
+    const float B = t.tan_theta;
     const float D =
         sqrtf(ref_max(B * B * Temp * Temp - (A * A - B * B) * Temp, 0.0f));
     const float x1 = B * Temp - D;
     const float x2 = B * Temp + D;
-    sx = (A < 0.0f || x2 > 1.0f / TanThetaI) ? x1 : x2;
+    sx = (A < 0.0f || x2 > t.a) ? x1 : x2;
     float S;
     if (u2 > 0.5f) {
       S = 1.0f;
@@ -354,19 +400,12 @@ struct DisneyB {
     const float z = vndf_fit_z(u2);
     sy = S * z * sqrtf(1.0f + sx * sx);
   }
-  __device__ static __forceinline__ F3 sample_vn(F3 wi_in, float u1, float u2,
-                                                float Alpha) {
-    const F3 wi = normalize3(mk3(Alpha * wi_in.x, Alpha * wi_in.y, wi_in.z));
-    float Theta = 0, Phi = 0;
-    if (wi.z < 0.99999f) {
-      Theta = acosf(wi.z);
-      Phi = atan2f(wi.y, wi.x);
-    }
-    const float SinPhi = sinf(Phi), CosPhi = cosf(Phi);
+  __device__ static __forceinline__ F3 sample_vn(const Stretched& t, float u1,
+                                                 float u2, float Alpha) {
     float sx, sy;
-    vn_unit(Theta, u1, u2, sx, sy);
-    float rx = CosPhi * sx - SinPhi * sy;
-    float ry = SinPhi * sx + CosPhi * sy;
+    vn_unit(t, u1, u2, sx, sy);
+    float rx = t.cos_phi * sx - t.sin_phi * sy;
+    float ry = t.sin_phi * sx + t.cos_phi * sy;
     rx *= Alpha;
     ry *= Alpha;
     const float Norm = 1.f / sqrtf(rx * rx + ry * ry + 1.0f);
@@ -386,233 +425,159 @@ struct DisneyB {
     const float omc2 = omc * omc;
     const float fr = R0 + (1.f - R0) * omc2 * omc2 * omc;
     const float fc = fresnel_conductor(cosD, 0.4f, 1.6f);
-    return std_lerp(fr, fc, m.metallic);
+    return std_lerp(fr, fc, m[5]);
   }
   __device__ static float fresnel_coat(float cosD) {
     const float omc = 1.0f - cosD;
     const float omc2 = omc * omc;
     return 0.04f + (1.0f - 0.04f) * omc2 * omc2 * omc;
   }
-  __device__ float diffuse_term(F3 wi, F3 wo, float idh, float rough) const {
-    if (m.metallic == 1.f) return 0.f;
+  __device__ float diffuse_term(F3 wi, float idh) const {
+    if (m[5] == 1.f) return 0.f;
     const float l = 1.f - fabsf(wi.z), l2 = l * l;
-    const float v = 1.f - fabsf(wo.z), v2 = v * v;
-    const float FD90 = 0.5f + 2.f * idh * rough;
+    const float v = 1.f - fabsf(lwo.z), v2 = v * v;
+    const float FD90 = 0.5f + 2.f * idh * rough();
     return kInvPi * (1.f + (FD90 - 1.f) * l2 * l2 * l) *
            (1.f + (FD90 - 1.f) * v2 * v2 * v);
   }
-  __device__ float specular_term(F3 wi, F3 wo, F3 wh, float odh,
-                                 float rough) const {
-    if (wi.z * wo.z <= 0.f) return 0.f;
-    const float D = ggx_d(wh, rough * rough);
-    if (D == 0.f) return 0.f;
-    const float nr = std_lerp(0.f, 0.08f, m.specular);
-    const float F = fresnel_schlick(odh, nr);
-    const float rg = (0.5f + 0.5f * rough);
-    const float G = ggx_g(wi, wo, wh, rg * rg);
-    return F * D * G / (4.f * fabsf(wi.z) * fabsf(wo.z));
-  }
-  __device__ float subsurface_term(F3 wi, F3 wo, float idh,
-                                   float rough) const {
-    if (m.subsurface == 0.0f) return 0.0f;
+  __device__ float subsurface_term(F3 wi, float idh) const {
+    if (m[4] == 0.0f) return 0.0f;
     const float l = 1.0f - fabsf(wi.z), l2 = l * l;
-    const float v = 1.0f - fabsf(wo.z), v2 = v * v;
-    const float F = idh * idh * rough;
+    const float v = 1.0f - fabsf(lwo.z), v2 = v * v;
+    const float F = idh * idh * rough();
     const float S = (1.0f + (F - 1.0f) * l2 * l2 * l) *
                     (1.0f + (F - 1.0f) * v2 * v2 * v);
     return kInvPi * 1.25f *
-           (S * (1.0f / (fabsf(wo.z) + fabsf(wi.z)) - 0.5f) + 0.5f);
+           (S * (1.0f / (fabsf(lwo.z) + fabsf(wi.z)) - 0.5f) + 0.5f);
   }
-  __device__ float clearcoat_term(F3 wi, F3 wo, F3 wh, float idh,
-                                  float gloss) const {
-    if (m.clearcoat == 0.0f) return 0.0f;
-    const float rough = dlerp(0.005f, 0.1f, gloss);
-    const float D = ggx_d(wh, rough);
-    if (D == 0.0f) return 0.0f;
-    const float F = fresnel_coat(idh);
-    const float G = ggx_g(wo, wi, wh, 0.25f);
-    return m.clearcoat * D * F * G / (4.0f * fabsf(wi.z) * fabsf(wo.z));
-  }
-  __device__ __forceinline__ F3 eval(F3 wi, F3 wo) const {
-    const F3 lwi = normalize3(sf.to_local(wi));
-    const F3 lwo = normalize3(sf.to_local(wo));
-    if (fabsf(lwi.z) < FLT_EPSILON || fabsf(lwo.z) < FLT_EPSILON)
-      return mk3(0, 0, 0);
-    const float rough = clampf(m.roughness, 0.02f, 1.f);
-    const F3 untinted = mk3(m.lum, m.lum, m.lum);
-    F3 spec_alb = dlerp(dlerp(m.base, untinted, 1.0f - m.specular_tint),
-                        m.base, m.metallic);
-    const F3 sheen_alb = dlerp(untinted, m.base, m.sheen_tint);
+  // f of (wi, wo), and its pdf (where f is black only when `always`)
+  template <bool kPdf = true>
+  __device__ __forceinline__ void eval_pdf(F3 wi, F3& f, float& pdf,
+                                           bool always) const {
+    const float metallic = m[5], clearcoat = m[12];
+    const F3 lwi = normalize3(frame().to_local(wi));
     const F3 wh = normalize3(lwo + lwi);
     const float odh = dot3(lwo, wh);
     const float idh = dot3(lwi, wh);
-    const float omo = 1.f - odh;
-    spec_alb = dlerp(spec_alb, untinted, omo * omo * omo);
-    const float F = fresnel_schlick(odh, 0.0f);
-    const F3 sheen_term = F * m.sheen * sheen_alb;
-    const float dl = dlerp(diffuse_term(lwi, lwo, idh, rough),
-                           subsurface_term(lwi, lwo, idh, rough), m.subsurface);
-    const F3 t1 = (1.0f - m.metallic) * (m.base * dl + sheen_term);
-    const F3 t2 = spec_alb * specular_term(lwi, lwo, wh, odh, rough);
-    const float cc = clearcoat_term(lwi, lwo, wh, idh, m.clearcoat_gloss);
-    return t1 + t2 + mk3(cc, cc, cc);
-  }
-  __device__ __forceinline__ float pdf(F3 wi, F3 wo) const {
-    const F3 lwi = normalize3(sf.to_local(wi));
-    const F3 lwo = normalize3(sf.to_local(wo));
-    const F3 wh = normalize3(lwo + lwi);
-    if (maxc3(wh) <= 0.f) return 0.f;
-    const float rough = clampf(m.roughness, 0.02f, 1.f);
-    const float mpdf = pdf_vn(lwo, wh, rough * rough);
-    float p = 0.f;
-    const float dwhdwi = 1.f / (4.f * fabsf(dot3(lwi, wh)));
-    const float spec_pdf = mpdf * dwhdwi;
-    const float nr = std_lerp(0.f, 0.08f, m.specular);
-    const float odh = dot3(lwo, wh);
-    const float ps = fresnel_schlick(odh, nr);
-    p += spec_pdf * ps;
-    p += fabsf(lwi.z) * kInvPi * (1.f - ps);
-    if (m.clearcoat > 0.f) {
-      // the clearcoat lobe reads the world-space wo (disney.cpp:208-220)
-      const float cw = m.clearcoat / (m.clearcoat + m.lum);
-      const float fc = fresnel_coat(fabsf(wo.z));
-      const float pc = (fc * cw) / (fc * cw + (1 - fc) * (1 - cw));
-      const float cr = std_lerp(0.005f, 0.10f, m.clearcoat_gloss);
-      const float chp = pdf_vn(wo, wh, cr);
-      const float cp = chp * dwhdwi;
-      p *= 1.0f - pc;
-      p += cp * pc;
-    }
-    return p;
-  }
-  // eval() and pdf() of the same (wi, wo) with their common
-  // subexpressions computed once (the same operations, so bit-identical).
-  // pdf is left at 0 when f is black unless pdf_if_black.
-  __device__ __forceinline__ void eval_pdf(F3 wi, F3 wo, F3& f, float& pdf,
-                                           bool pdf_if_black) const {
-    const F3 lwi = normalize3(sf.to_local(wi));
-    const F3 lwo = normalize3(sf.to_local(wo));
-    const float rough = clampf(m.roughness, 0.02f, 1.f);
-    const F3 wh = normalize3(lwo + lwi);
+    const float c2 = wh.z * wh.z;
+    const float tmp = 1.f - wh.z * wh.z;
+    const float t2 = tmp <= 0.f ? 0.f : tmp / c2;
+    const float D = ggx_d(wh.z, c2, t2, alpha());
     f = mk3(0, 0, 0);
     if (!(fabsf(lwi.z) < FLT_EPSILON || fabsf(lwo.z) < FLT_EPSILON)) {
-      const F3 untinted = mk3(m.lum, m.lum, m.lum);
-      F3 spec_alb = dlerp(dlerp(m.base, untinted, 1.0f - m.specular_tint),
-                          m.base, m.metallic);
-      const F3 sheen_alb = dlerp(untinted, m.base, m.sheen_tint);
-      const float odh = dot3(lwo, wh);
-      const float idh = dot3(lwi, wh);
+      const F3 untinted = mk3(lum, lum, lum);
       const float omo = 1.f - odh;
+      F3 spec_alb = dlerp(dlerp(base(), untinted, 1.0f - m[7]), base(), metallic);
+      const F3 sheen_alb = dlerp(untinted, base(), m[11]);
       spec_alb = dlerp(spec_alb, untinted, omo * omo * omo);
       const float F = fresnel_schlick(odh, 0.0f);
-      const F3 sheen_term = F * m.sheen * sheen_alb;
+      const F3 sheen_term = F * m[10] * sheen_alb;
       const float dl =
-          dlerp(diffuse_term(lwi, lwo, idh, rough),
-                subsurface_term(lwi, lwo, idh, rough), m.subsurface);
-      const F3 t1 = (1.0f - m.metallic) * (m.base * dl + sheen_term);
-      const F3 t2 = spec_alb * specular_term(lwi, lwo, wh, odh, rough);
-      const float cc = clearcoat_term(lwi, lwo, wh, idh, m.clearcoat_gloss);
-      f = t1 + t2 + mk3(cc, cc, cc);
+          dlerp(diffuse_term(lwi, idh), subsurface_term(lwi, idh), m[4]);
+      const F3 t1 = (1.0f - metallic) * (base() * dl + sheen_term);
+      const float tti = fabsf(tan_theta(lwi));
+      float specular = 0.f;
+      if (!(lwi.z * lwo.z <= 0.f) && D != 0.f) {
+        const float Fs = fresnel_schlick(odh, nr());
+        const float G = smith(tt, odh, lwo.z, g_spec) *
+                        smith(tti, idh, lwi.z, masking(tti, alpha_g()));
+        specular = Fs * D * G / (4.f * fabsf(lwi.z) * fabsf(lwo.z));
+      }
+      const F3 ts = spec_alb * specular;
+      float cc = 0.f;
+      if (clearcoat != 0.0f) {
+        const float Dc = ggx_d(wh.z, c2, t2, dlerp(0.005f, 0.1f, m[13]));
+        if (Dc != 0.0f) {
+          const float Fc = fresnel_coat(idh);
+          const float G = smith(tti, idh, lwi.z, masking(tti, 0.25f)) *
+                          smith(tt, odh, lwo.z, g_coat);
+          cc = clearcoat * Dc * Fc * G / (4.0f * fabsf(lwi.z) * fabsf(lwo.z));
+        }
+      }
+      f = t1 + ts + mk3(cc, cc, cc);
     }
     pdf = 0.f;
-    if (!pdf_if_black && black3(f)) return;
+    if (!kPdf || (!always && black3(f))) return;
     if (maxc3(wh) <= 0.f) return;
-    const float mpdf = pdf_vn(lwo, wh, rough * rough);
+    const float mpdf = smith(tt, odh, lwo.z, g_pdf) * fabsf(odh) * D /
+                       (fabsf(lwo.z) + 1e-4f);
     float p = 0.f;
-    const float dwhdwi = 1.f / (4.f * fabsf(dot3(lwi, wh)));
+    const float dwhdwi = 1.f / (4.f * fabsf(idh));
     const float spec_pdf = mpdf * dwhdwi;
-    const float nr = std_lerp(0.f, 0.08f, m.specular);
-    const float odh = dot3(lwo, wh);
-    const float ps = fresnel_schlick(odh, nr);
+    const float ps = fresnel_schlick(odh, nr());
     p += spec_pdf * ps;
     p += fabsf(lwi.z) * kInvPi * (1.f - ps);
-    if (m.clearcoat > 0.f) {
-      const float cw = m.clearcoat / (m.clearcoat + m.lum);
-      const float fc = fresnel_coat(fabsf(wo.z));
-      const float pc = (fc * cw) / (fc * cw + (1 - fc) * (1 - cw));
-      const float cr = std_lerp(0.005f, 0.10f, m.clearcoat_gloss);
-      const float chp = pdf_vn(wo, wh, cr);
+    if (clearcoat > 0.f) {
+      const float wdh = dot3(wo, wh);
+      const float chp = smith(tt_w, wdh, wo.z, g_w) * fabsf(wdh) *
+                        ggx_d(wh.z, c2, t2, coat_alpha()) / (fabsf(wo.z) + 1e-4f);
       const float cp = chp * dwhdwi;
-      p *= 1.0f - pc;
-      p += cp * pc;
+      p *= 1.0f - pc_world;
+      p += cp * pc_world;
     }
     pdf = p;
   }
-  __device__ __forceinline__ BsdfSample sample(F3 wo, F3 sam) const {
-    const F3 lwo = normalize3(sf.to_local(wo));
-    F3 lwi, lwh;
+  __device__ __forceinline__ Stretched stretched() const {
+    return stretch(lwo, alpha());
+  }
+  // The sampled direction in the frame (z <= 0: no sample), from
+  // `t` = stretched().
+  __device__ __forceinline__ F3 sample_dir(F3 sam, const Stretched& t) const {
+    float r1 = sam.y;
+    Stretched w = t;
+    float al = alpha();
     bool coat = false;
-    float r0 = sam.x, r1 = sam.y;
-    const float r2 = sam.z;
-    if (m.clearcoat > 0.f) {
-      const float cw = m.clearcoat / (m.clearcoat + m.lum);
-      const float fc = fresnel_coat(fabsf(lwo.z));
-      const float pc = (fc * cw) / (fc * cw + (1.f - fc) * (1.f - cw));
-      if (sam.y < pc) {
-        coat = true;
-        r1 /= pc;
-        const float cr = std_lerp(0.005f, 0.1f, m.clearcoat_gloss);
-        lwh = sample_vn(lwo, r0, r1, cr);
-        lwi = reflect(-lwo, lwh);
+    if (m[12] > 0.f) {
+      coat = sam.y < pc_local;
+      if (coat) {
+        r1 /= pc_local;
+        al = coat_alpha();
+        w = stretch(lwo, al);
       } else {
-        r1 = (sam.y - pc) / (1.f - pc);
+        r1 = (sam.y - pc_local) / (1.f - pc_local);
       }
     }
-    if (!coat) {
-      const float rough = clampf(m.roughness, 0.02f, 1.0f);
-      lwh = sample_vn(lwo, r0, r1, rough * rough);
-      const float nr = std_lerp(0.0f, 0.08f, m.specular);
-      const float odh = dot3(lwo, lwh);
-      const float ps = fresnel_schlick(odh, nr);
-      if (r2 <= ps) {
-        lwi = reflect(-lwo, lwh);
-      } else {
-        lwi = cosine_hemisphere(r0, r1, nullptr);
-        if (lwo.z < 0.0f) lwi.z *= -1.0f;
-      }
+    const F3 lwh = sample_vn(w, sam.x, r1, al);
+    if (!coat && !(sam.z <= fresnel_schlick(dot3(lwo, lwh), nr()))) {
+      F3 lwi = cosine_hemisphere(sam.x, r1, nullptr);
+      if (lwo.z < 0.0f) lwi.z *= -1.0f;
+      return lwi;
     }
-    if (lwi.z <= 0.0f) return invalid_sample();
-    BsdfSample s;
-    s.dir = sf.to_world(lwi);
-    eval_pdf(s.dir, wo, s.f, s.pdf, true);
-    return s;
+    return reflect(-lwo, lwh);
   }
 };
 
-// One out-of-line copy of each BSDF routine: the path kernel calls them from
-// ten sites per hit, and inlining them all overflows the instruction cache.
-static __device__ __noinline__ F3 disney_eval(const float* __restrict__ m, float lum,
-                                       F3 ns, F3 wi, F3 wo) {
-  const MatParams p = load_material(m, lum);
-  return DisneyB(p, ns).eval(wi, wo);
-}
-static __device__ __noinline__ float disney_pdf(const float* __restrict__ m,
-                                         float lum, F3 ns, F3 wi, F3 wo) {
-  const MatParams p = load_material(m, lum);
-  return DisneyB(p, ns).pdf(wi, wo);
-}
+// Out of line for the kernels that switch on the material type, so that the
+// other types' lanes do not pay for its registers.
 static __device__ __noinline__ BsdfSample disney_sample(const float* __restrict__ m,
-                                                 float lum, F3 ns, F3 wo,
-                                                 F3 sam) {
-  const MatParams p = load_material(m, lum);
-  return DisneyB(p, ns).sample(wo, sam);
+                                                        float lum, F3 ns, F3 wo,
+                                                        F3 sam) {
+  DisneyB d;
+  d.prepare(m, lum, ns, wo);
+  const F3 lwi = d.sample_dir(sam, d.stretched());
+  if (lwi.z <= 0.0f) return invalid_sample();
+  BsdfSample s;
+  s.dir = d.frame().to_world(lwi);
+  d.eval_pdf(s.dir, s.f, s.pdf, true);
+  return s;
+}
+static __device__ __noinline__ void disney_prepare(DisneyB& d,
+                                                   const float* __restrict__ m,
+                                                   float lum, F3 ns, F3 wo) {
+  d.prepare(m, lum, ns, wo);
+}
+static __device__ __noinline__ F3 disney_eval(const DisneyB& d, F3 wi) {
+  F3 f;
+  float pdf;
+  d.eval_pdf<false>(wi, f, pdf, false);
+  return f;
 }
 static __device__ __noinline__ void disney_eval_pdf(const float* __restrict__ m,
-                                                    float lum, F3 ns, F3 wi,
-                                                    F3 wo, F3& f, float& pdf,
-                                                    bool pdf_if_black) {
-  const MatParams p = load_material(m, lum);
-  DisneyB(p, ns).eval_pdf(wi, wo, f, pdf, pdf_if_black);
-}
-static __device__ __noinline__ BsdfSample lambert_sample(F3 ng, F3 ns, F3 alb,
-                                                  F3 wo, F3 sam) {
-  return Lambert(ng, ns, alb).sample(wo, sam);
-}
-static __device__ __noinline__ F3 lambert_eval(F3 ng, F3 ns, F3 alb, F3 wi, F3 wo) {
-  return Lambert(ng, ns, alb).eval(wi, wo);
-}
-static __device__ __noinline__ float lambert_pdf(F3 ng, F3 ns, F3 alb, F3 wi, F3 wo) {
-  return Lambert(ng, ns, alb).pdf(wi, wo);
+                                                    float lum, F3 ns, F3 wo, F3 wi,
+                                                    F3& f, float& pdf) {
+  DisneyB d;
+  d.prepare(m, lum, ns, wo);
+  d.eval_pdf(wi, f, pdf, true);
 }
 
 // ------------------------------------- mirror, glass, metal, plastic, null --
@@ -1020,70 +985,112 @@ static __device__ __noinline__ void other_eval_pdf(int type, const float* m,
   }
 }
 
-// The BSDF at a hit: material record (in global memory) and the two normals.
+// One sample of a material's BSDF (record m, luminance of its base colour).
+__device__ __forceinline__ BsdfSample bsdf_sample(int type, const float* m,
+                                                  float lum, F3 ng, F3 ns, F3 wo,
+                                                  F3 sam) {
+  if (type == AJG_MAT_DIFFUSE) {
+    Lambert l;
+    l.prepare(ng, ns, mk3(m[1], m[2], m[3]), wo);
+    return l.sample(sam);
+  }
+  if (type == AJG_MAT_DISNEY) return disney_sample(m, lum, ns, wo, sam);
+  return other_sample(type, m, ng, ns, wo, sam);
+}
+
+// Its value, and its pdf.
+__device__ __forceinline__ void bsdf_eval_pdf(int type, const float* m, float lum,
+                                              F3 ng, F3 ns, F3 wo, F3 wi, F3& f,
+                                              float& pdf) {
+  if (type == AJG_MAT_DIFFUSE) {
+    Lambert l;
+    l.prepare(ng, ns, mk3(m[1], m[2], m[3]), wo);
+    l.eval_pdf(wi, f, pdf);
+    pdf = l.pdf(wi);
+  } else if (type == AJG_MAT_DISNEY) {
+    disney_eval_pdf(m, lum, ns, wo, wi, f, pdf);
+  } else {
+    other_eval_pdf(type, m, ng, ns, wi, wo, f, pdf);
+  }
+}
+
+// The BSDF's value at a point for one outgoing direction and many incoming
+// ones, with the type's terms prepared.
 struct Bsdf {
   int type;
-  F3 ng, ns;
-  const float* m;  // [16] record
-  float lum;
-  __device__ __forceinline__ F3 albedo() const {
-    return mk3(m[1], m[2], m[3]);
+  F3 ng, ns, wo;
+  const float* m;
+  union {
+    Lambert l;
+    DisneyB d;
+  };
+  __device__ __forceinline__ Bsdf() {}
+  __device__ __forceinline__ void prepare(const float* m_, float lum, F3 ng_,
+                                          F3 ns_, F3 wo_) {
+    type = (int)m_[0];
+    m = m_;
+    ng = ng_;
+    ns = ns_;
+    wo = wo_;
+    if (type == AJG_MAT_DIFFUSE)
+      l.prepare(ng, ns, mk3(m[1], m[2], m[3]), wo);
+    else if (type == AJG_MAT_DISNEY)
+      disney_prepare(d, m, lum, ns, wo);
   }
-  __device__ __forceinline__ BsdfSample sample(F3 wo, F3 s) const {
-    if (type == AJG_MAT_DIFFUSE) return lambert_sample(ng, ns, albedo(), wo, s);
-    if (type == AJG_MAT_DISNEY) return disney_sample(m, lum, ns, wo, s);
-    return other_sample(type, m, ng, ns, wo, s);
-  }
-  __device__ __forceinline__ F3 eval(F3 wi, F3 wo) const {
-    if (type == AJG_MAT_DIFFUSE) return lambert_eval(ng, ns, albedo(), wi, wo);
-    if (type == AJG_MAT_DISNEY) return disney_eval(m, lum, ns, wi, wo);
+  __device__ __forceinline__ F3 eval(F3 wi) const {
     F3 f;
-    float p;
-    other_eval_pdf(type, m, ng, ns, wi, wo, f, p);
+    float pdf;
+    if (type == AJG_MAT_DIFFUSE)
+      l.eval_pdf(wi, f, pdf);
+    else if (type == AJG_MAT_DISNEY)
+      f = disney_eval(d, wi);
+    else
+      other_eval_pdf(type, m, ng, ns, wi, wo, f, pdf);
     return f;
   }
-  __device__ __forceinline__ float pdf(F3 wi, F3 wo) const {
-    if (type == AJG_MAT_DIFFUSE) return lambert_pdf(ng, ns, albedo(), wi, wo);
-    if (type == AJG_MAT_DISNEY) return disney_pdf(m, lum, ns, wi, wo);
-    F3 f;
-    float p;
-    other_eval_pdf(type, m, ng, ns, wi, wo, f, p);
-    return p;
-  }
 };
 
-// The same with the material type fixed at compile time (the specialised
-// shading kernels): NEE needs f and, when f is not black, the pdf.
+// A hit's BSDF with the material type fixed at compile time (the specialised
+// shading kernels).  Each kernel has one site that samples and one that
+// evaluates, so everything is inlined and a hit's terms stay in registers.
 template <int MAT>
 struct BsdfT {
-  F3 ng, ns;
+  static constexpr bool kDisney = MAT == AJG_MAT_DISNEY;
+  F3 ng, ns, wo;
   const float* m;
-  float lum;
-  __device__ __forceinline__ F3 albedo() const {
-    return mk3(m[1], m[2], m[3]);
+  std::conditional_t<MAT == AJG_MAT_DIFFUSE, Lambert, DisneyB> b;
+  __device__ __forceinline__ BsdfT() {}
+  __device__ __forceinline__ void prepare(const float* m_, float lum, F3 ng_,
+                                          F3 ns_, F3 wo_) {
+    m = m_;
+    ng = ng_;
+    ns = ns_;
+    wo = wo_;
+    if constexpr (MAT == AJG_MAT_DIFFUSE)
+      b.prepare(ng, ns, mk3(m[1], m[2], m[3]), wo);
+    else if constexpr (kDisney)
+      b.prepare(m, lum, ns, wo);
   }
-  __device__ __forceinline__ BsdfSample sample(F3 wo, F3 s) const {
-    if (MAT == AJG_MAT_DIFFUSE) return Lambert(ng, ns, albedo()).sample(wo, s);
-    if (MAT == kMatOther) return other_sample((int)m[0], m, ng, ns, wo, s);
-    return disney_sample(m, lum, ns, wo, s);
+  // the types but Disney, whose sample is a direction (sample_dir) and its
+  // evaluation
+  __device__ __forceinline__ BsdfSample sample(F3 s) const {
+    if constexpr (MAT == AJG_MAT_DIFFUSE)
+      return b.sample(s);
+    else
+      return other_sample((int)m[0], m, ng, ns, wo, s);
   }
-  __device__ __forceinline__ void eval_pdf(F3 wi, F3 wo, F3& f,
-                                           float& pdf) const {
-    if (MAT == AJG_MAT_DIFFUSE) {
-      const Lambert l(ng, ns, albedo());
-      f = l.eval(wi, wo);
-      pdf = black3(f) ? 0.f : l.pdf(wi, wo);
-      return;
-    }
-    if (MAT == kMatOther) {
+  // f and its pdf; where f is black the pdf only when `always` (Disney)
+  __device__ __forceinline__ void eval_pdf(F3 wi, F3& f, float& pdf,
+                                           bool always) const {
+    if constexpr (MAT == AJG_MAT_DIFFUSE)
+      b.eval_pdf(wi, f, pdf);
+    else if constexpr (!kDisney)
       other_eval_pdf((int)m[0], m, ng, ns, wi, wo, f, pdf);
-      return;
-    }
-    disney_eval_pdf(m, lum, ns, wi, wo, f, pdf, false);
+    else
+      b.eval_pdf(wi, f, pdf, always);
   }
 };
 
-// ------------------------------------------------------------ hit record --
 struct HitInfo {
   F3 pos, ng, ns, wr;
   uint32_t mat;

@@ -452,18 +452,6 @@ __global__ void __launch_bounds__(128, trace_min_blocks<W>())
   flush_counters(ctr, nr, nn, nt);
 }
 
-// A BSDF from a material record and its two normals.
-__device__ __forceinline__ Bsdf bsdf_at(const DeviceScene& s, uint32_t mat,
-                                        F3 ng, F3 ns) {
-  Bsdf f;
-  f.m = s.materials + 16 * mat;
-  f.type = (int)f.m[0];
-  f.ng = ng;
-  f.ns = ns;
-  f.lum = __ldg(&s.mat_lum[mat].x);
-  return f;
-}
-
 // Records a photon's deposit at `pos` (VisiblePointSearcher::AddPhoton,
 // photon_mapping.h:101-120) for k_deposit, unless no visible point is filed
 // under its entry.
@@ -514,8 +502,12 @@ __global__ void k_deposit_sort(Deposits dp) {
 // on average against 585 us for all depths of an iteration (192x192 film of
 // the emitter box, radius 0.1, 100,000 photons: 118.6 -> 14.3 ms for 12
 // iterations; 512x512, radius 0.01, 2 M photons over 327,682 triangles:
-// 14.1 -> 10.8 ms for 4).
-__global__ void __launch_bounds__(kThreads)
+// 14.1 -> 10.8 ms for 4), 372 us with the points' BSDF terms prepared once.
+//
+// 8 blocks of 128 an SM (64 registers, 200 bytes of spills beside the BSDF's
+// prepared terms in local memory): 4.5 ms on the box above, 6 blocks 5.6,
+// 5 6.1, 4 without spills 7.0.  Only the Lambertian lobe prepared: 7.6.
+__global__ void __launch_bounds__(kThreads, 8)
     k_deposit(SppmArgs a, SppmPixels px, Grid g, Deposits dp) {
   __shared__ float4 s_rec[kThreads / 32][32 * 3];
   const int lane = threadIdx.x & 31;
@@ -557,7 +549,7 @@ __global__ void __launch_bounds__(kThreads)
     const bool on = item < i1;
     const float4 sp = on ? __ldg(&g.spheres[item]) : make_float4(0, 0, 0, 0);
     Bsdf f;
-    F3 vwr = mk3(0, 0, 0), sum = mk3(0, 0, 0);
+    F3 sum = mk3(0, 0, 0);
     uint32_t pix = 0, m_sum = 0;
     bool loaded = false;
     for (uint32_t t = t0; t < t1; ++t) {
@@ -580,8 +572,9 @@ __global__ void __launch_bounds__(kThreads)
       if (near && !loaded) {
         pix = g.items[item];
         const VisPointD v = px.vp[pix];
-        f = bsdf_at(a.s, __float_as_uint(v.pos.w), xyz(v.ng), xyz(v.ns));
-        vwr = xyz(v.wr);
+        const uint32_t mat = __float_as_uint(v.pos.w);
+        f.prepare(a.s.materials + 16 * mat, __ldg(&a.s.mat_lum[mat].x), xyz(v.ng),
+                  xyz(v.ns), xyz(v.wr));
         loaded = true;
       }
       while (__any_sync(kFull, near != 0)) {
@@ -591,7 +584,7 @@ __global__ void __launch_bounds__(kThreads)
           const float px_ = tile[3 * j].w;
           const float4 q = tile[3 * j + 1];
           const float wz = tile[3 * j + 2].x;
-          const F3 c = mk3(px_, q.x, q.y) * f.eval(mk3(q.z, q.w, wz), vwr);
+          const F3 c = mk3(px_, q.x, q.y) * f.eval(mk3(q.z, q.w, wz));
           if (isfinite(c.x) && isfinite(c.y) && isfinite(c.z)) {
             sum = sum + c;
             ++m_sum;
@@ -639,11 +632,12 @@ __global__ void __launch_bounds__(kThreads)
         pos = hi.pos;
         power = coef;
         wr = hi.wr;
-        const Bsdf f = bsdf_at(a.s, hi.mat, hi.ng, hi.ns);
+        const float* m = a.s.materials + 16 * hi.mat;
         const F3 sam = mk3(key_float(key, dim), key_float(key, dim + 1),
                            key_float(key, dim + 2));
         dim += 3;
-        const BsdfSample bs = f.sample(hi.wr, sam);
+        const BsdfSample bs = bsdf_sample(
+            (int)m[0], m, __ldg(&a.s.mat_lum[hi.mat].x), hi.ng, hi.ns, hi.wr, sam);
         if (!(black3(bs.f) || bs.pdf < 0.f)) {
           coef = coef * (bs.f / bs.pdf * fabsf(dot3(hi.ng, bs.dir)));
           make_ray(eps_offset(hi, bs.dir), bs.dir, no, nd);
