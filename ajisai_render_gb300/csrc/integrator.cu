@@ -217,50 +217,58 @@ __global__ void __launch_bounds__(kShadeThreads)
   }
 }
 
-// Files every queue slot under its hit's shading class (a miss, Lambertian,
-// Disney, or one of the other material types), so that shading runs in
-// class-specialised kernels; warps stay converged, so each list append is
-// one atomic per warp.
+// Files every queue slot under its hit's shading class (Lambertian, Disney, or
+// one of the other material types), so that shading runs in class-specialised
+// kernels, and ends the escaped paths: the environment counts only for camera
+// rays (pt.cpp:114-121), or on every bounce without MIS (pt.cpp:245-249).
+// (Beside the accumulation of the bounce before: no path of it is touched by
+// both, as with MIS only camera rays add here.)
 template <bool MJ>
 __global__ void __launch_bounds__(kClassifyThreads)
-    k_classify(DeviceScene s, MJTables t,
-                           const float4* __restrict__ ro,
-                           const uint32_t* __restrict__ count,
-                           const ajg_hit* __restrict__ hits,
-                           uint32_t* __restrict__ lists,
-                           uint32_t* __restrict__ list_counts,
-                           uint32_t list_cap) {
-  const uint32_t n = *count;
+    k_classify(WaveArgs a, MJTables t, WaveBufs w, int b, int cur,
+               uint32_t list_cap) {
+  const uint32_t n = w.counts[0];
   const uint32_t stride = gridDim.x * blockDim.x;
   // block-uniform iterations: block_append synchronises the block
   for (uint32_t bb = blockIdx.x * blockDim.x; bb < n; bb += stride) {
     const uint32_t k = bb + threadIdx.x;
     int cls = -1;
     if (k < n) {
-      const int prim = hits[k].prim;
-      cls = 0;
+      const int prim = w.hits[k].prim;
       if (prim >= 0) {
-        const float4* shade = s.shade;
-        const float* materials = s.materials;
+        const float4* shade = a.s.shade;
+        const float* materials = a.s.materials;
         if constexpr (MJ) {
-          const DeviceScene& sc = t.scenes[mj_scene(t, __float_as_uint(ro[k].w))];
+          const DeviceScene& sc =
+              t.scenes[mj_scene(t, __float_as_uint(w.ro[cur][k].w))];
           shade = sc.shade;
           materials = sc.materials;
         }
         const uint32_t mat =
             __float_as_uint(__ldg(&shade[prim].w)) & 0xffffffu;
         const int type = (int)__ldg(materials + 16 * mat);
-        cls = type == AJG_MAT_DIFFUSE ? 1 : (type == AJG_MAT_DISNEY ? 2 : 3);
+        cls = type == AJG_MAT_DIFFUSE ? 0 : (type == AJG_MAT_DISNEY ? 1 : 2);
+      } else if (MJ || ((b == 0 || !a.j.use_mis) && a.s.env >= 0)) {
+        const uint32_t p = w.qpath[cur][k];
+        const uint32_t jid = MJ ? mj_job(t, w.pjob[p]) : 0u;
+        const JobParams& J = Src<MJ>::job(a, t, jid);
+        if ((b == 0 || !J.use_mis) && Src<MJ>::scene(a, t, jid).env >= 0) {
+          float4 L = w.rad[p];
+          L.x += J.env_rgb.x;
+          L.y += J.env_rgb.y;
+          L.z += J.env_rgb.z;
+          w.rad[p] = L;
+        }
       }
     }
 #if AJG_BLOCK_APPEND
-    const uint32_t j = block_append<4, kClassifyThreads / 32>(list_counts, cls);
-    if (cls >= 0) lists[(uint64_t)cls * list_cap + j] = k;
+    const uint32_t j = block_append<3, kClassifyThreads / 32>(&w.counts[5], cls);
+    if (cls >= 0) w.lists[(uint64_t)(cls + 1) * list_cap + j] = k;
 #else
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const uint32_t j = warp_append(&list_counts[c], cls == c);
-      if (cls == c) lists[(uint64_t)c * list_cap + j] = k;
+    for (int c = 0; c < 3; ++c) {
+      const uint32_t j = warp_append(&w.counts[5 + c], cls == c);
+      if (cls == c) w.lists[(uint64_t)(c + 1) * list_cap + j] = k;
     }
 #endif
   }
@@ -381,33 +389,6 @@ __device__ __forceinline__ void emit_closest(const WaveBufs& w, F3 o, F3 d,
   w.sq_o[i] = make_float4(o.x, o.y, o.z, pdf);
   w.sq_d[i] = make_float4(d.x, d.y, d.z, __uint_as_float(slot));
   if constexpr (MJ) w.sq_scene[i] = (uint16_t)sid;
-}
-
-// Escaped paths: the environment counts only for camera rays
-// (pt.cpp:114-121), or on every bounce without MIS (pt.cpp:245-249).  The
-// single-job launch is skipped on the host when neither applies.
-template <bool MJ>
-__global__ void k_shade_miss(WaveArgs a, MJTables t, WaveBufs w, int b,
-                             int cur, const uint32_t* __restrict__ list,
-                             const uint32_t* __restrict__ count) {
-  const uint32_t n = *count;
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n;
-       j += gridDim.x * blockDim.x) {
-    const uint32_t p = w.qpath[cur][list[j]];
-    float4 env = a.j.env_rgb;
-    if constexpr (MJ) {
-      const uint32_t jid = mj_job(t, w.pjob[p]);
-      const JobParams& J = t.jobs[jid].j;
-      if (!(b == 0 || !J.use_mis) || Src<true>::scene(a, t, jid).env < 0)
-        continue;
-      env = J.env_rgb;
-    }
-    float4 L = w.rad[p];
-    L.x += env.x;
-    L.y += env.y;
-    L.z += env.z;
-    w.rad[p] = L;
-  }
 }
 
 // Shading of the hits on one material type: NEE to every light
@@ -642,7 +623,8 @@ __global__ void __launch_bounds__(kShadeThreads, shade_min_blocks<MAT>())
           }
           w.thr[p] = make_float4(T.x, T.y, T.z, 0.f);
         }
-        const uint32_t kn = shade_append(&w.counts[nxt], alive);
+        // the next bounce's queue
+        const uint32_t kn = shade_append(&w.counts[kCounterWords], alive);
         if (alive) {
           w.qpath[nxt][kn] = p;
           w.ro[nxt][kn] = make_float4(nro.x, nro.y, nro.z, __uint_as_float(sid));
@@ -750,7 +732,7 @@ __global__ void __launch_bounds__(kShadeThreads, shade_min_blocks<MAT>())
 template <bool MJ>
 __global__ void __launch_bounds__(kShadeThreads)
     k_accumulate(WaveArgs a, MJTables t, WaveBufs w, int cur, uint32_t NT) {
-  const uint32_t n = w.counts[cur];
+  const uint32_t n = w.counts[0];
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n;
        k += gridDim.x * blockDim.x) {
     if (w.hits[k].prim < 0) continue;
@@ -1018,7 +1000,7 @@ uint64_t wave_bytes(uint64_t P, int nt, bool mj) {
   add(slots * 16); add(slots * 16);  // shadow queue
   if (mj) add(slots * 2);      // sq_scene
   add(P * 4 * 4);              // shading-class lists
-  add(64);                     // counts
+  add(64);                     // (the counters' first 64 bytes)
   return b;
 }
 
@@ -1046,14 +1028,14 @@ WaveBufs carve_wave(char* base, uint64_t P, int nt, bool mj) {
   w.sq_d = carve<float4>(cur, P * nt);
   if (mj) w.sq_scene = carve<uint16_t>(cur, P * nt);
   w.lists = carve<uint32_t>(cur, P * 4);
-  w.counts = carve<uint32_t>(cur, 16);
+  w.counts = carve<uint32_t>(cur, 16);  // and behind: counter_bytes in all
   return w;
 }
 
 // The wave arena: one device allocation reused across renders of the
 // context, grown when a render needs more paths or light terms.
 static int ensure_arena(ajg_ctx* ctx, uint64_t P, int nt, char** base) {
-  const uint64_t need = wave_bytes(P, nt, false);
+  const uint64_t need = wave_bytes(P, nt, false) + counter_bytes(kMaxBounces);
   if (ctx->arena.empty() || ctx->arena[0].bytes < need) {
     for (auto& b : ctx->arena) cudaFree(b.ptr);
     ctx->arena.clear();
@@ -1085,7 +1067,7 @@ int check_render(ajg_ctx* ctx, const DeviceScene& s, const ajg_camera& cam,
                  const ajg_render_params& prm) {
   if (cam.width == 0 || cam.height == 0 || prm.spp == 0)
     return fail(ctx, AJG_ERR_INVALID, "empty film or zero spp");
-  if (prm.max_bounces < 0 || prm.max_bounces > 1024)
+  if (prm.max_bounces < 0 || prm.max_bounces > kMaxBounces)
     return fail(ctx, AJG_ERR_INVALID, "max_bounces must be in [0, 1024]");
   if (s.num_lights > kMaxLights)
     return fail(ctx, AJG_ERR_UNSUPPORTED, "at most 15 lights");
@@ -1217,42 +1199,60 @@ static void run_waves(ajg_scene* sc, const ajg_camera& cam,
   // bounce 0's camera rays (a pixel's samples side by side in the queue) as
   // masked packets over the binary layout (AJG_PACKET_CAMERA)
   const bool cam_packets = ctx->packet_camera && s_closest.width == 2;
-  auto extend = [&](int q, ajg_hit* hits, cudaStream_t es, bool cam) {
+  // The wave's buffers as bounce b's launches see them: its own counters, and
+  // with overlap the hits of its parity.
+  auto at_bounce = [&](int b, bool overlap) {
+    WaveBufs wb = w;
+    wb.counts = w.counts + kCounterWords * b;
+    if (overlap && (b & 1)) wb.hits = w.hits2;
+    return wb;
+  };
+  auto extend = [&](const WaveBufs& wb, int q, cudaStream_t es, bool cam) {
     if (cam)
       launch_wave_extend_packet(false, s_closest.tri_test, s_closest, t,
-                                w.ro[q], w.rd[q], &w.counts[q], &w.counts[8],
-                                hits, &ctx->d_counters[0], ctx->d_error, es);
+                                w.ro[q], w.rd[q], &wb.counts[0], &wb.counts[8],
+                                wb.hits, &ctx->d_counters[0], ctx->d_error, es);
     else
       launch_wave_extend(false, s_closest.tri_test, s_closest.width, s_closest,
-                         t, w.ro[q], w.rd[q], &w.counts[q], &w.counts[8], hits,
-                         &ctx->d_counters[0], ctx->d_error, es);
+                         t, w.ro[q], w.rd[q], &wb.counts[0], &wb.counts[8],
+                         wb.hits, &ctx->d_counters[0], ctx->d_error, es);
+  };
+  auto classify = [&](const WaveBufs& wb, int b, int q, cudaStream_t es) {
+    KernelTimer tm(ctx, es, -1);
+    k_classify<false><<<gs, kClassifyThreads, 0, es>>>(a, t, wb, b, q, (uint32_t)P);
   };
   // Bounce b+1's closest hits run on the trace stream beside bounce b's
   // shadow rays: the two persistent launches fill each other's drain.  The
   // hits alternate between two buffers by bounce parity (k_accumulate of
-  // bounce b still reads its own); everything else bounce b+1 touches is
-  // written after k_accumulate of bounce b on the render stream.
+  // bounce b still reads its own), and so do the queues; everything else
+  // bounce b+1 touches is written after k_accumulate of bounce b on the
+  // render stream.  Its classification follows the hits there, except in
+  // scenes with emitters, whose MIS BSDF hits borrow the lists.
   const bool overlap = ctx->overlap && !ctx->profiling && w.hits2 != nullptr;
+  const bool classify_ahead = overlap && !s.tri_emit;
   cudaStream_t ts = ctx->trace_stream;
-  auto extend_ahead = [&](int q, ajg_hit* hits, bool cam) {
+  auto extend_ahead = [&](int b, int q, bool cam) {
+    const WaveBufs wb = at_bounce(b, true);
     cudaEventRecord(ctx->ev_queue, st);
     cudaStreamWaitEvent(ts, ctx->ev_queue, 0);
-    cudaMemsetAsync(&w.counts[8], 0, sizeof(uint32_t), ts);
-    KernelTimer tm(ctx, ts, cam ? kcp : kc);
-    extend(q, hits, ts, cam);
+    {
+      KernelTimer tm(ctx, ts, cam ? kcp : kc);
+      extend(wb, q, ts, cam);
+    }
+    if (classify_ahead) classify(wb, b, q, ts);
     cudaEventRecord(ctx->ev_hits, ts);
   };
-  auto bsdf_closest = [&]() {
+  auto bsdf_closest = [&](const WaveBufs& wb) {
     launch_wave_bsdf_trace(false, s_closest.tri_test, s_closest.width, s_closest, t,
                            w.sq_o, w.sq_d,
-                           nullptr, &w.counts[9], &w.counts[10], shadow_cap,
+                           nullptr, &wb.counts[9], &wb.counts[10], shadow_cap,
                            (uint32_t)P, reinterpret_cast<float*>(w.lists),
                            reinterpret_cast<int32_t*>(w.lists + P),
                            &ctx->d_counters[0], ctx->d_error, st);
   };
-  auto shadow = [&]() {
+  auto shadow = [&](const WaveBufs& wb) {
     launch_wave_shadow(false, s.tri_test, s.width, s, t, w.sq_o, w.sq_d, nullptr,
-                       &w.counts[2], &w.counts[3], w.term_vis,
+                       &wb.counts[2], &wb.counts[3], w.term_vis,
                        &ctx->d_counters[1], ctx->d_error, st);
   };
   // Coherent shadow rays: at bounce 0 a shading block's rays of one light
@@ -1269,9 +1269,9 @@ static void run_waves(ajg_scene* sc, const ajg_camera& cam,
         coh0 |= 1u << l;
     if (ctx->packet_shadow >= 2) coh0 |= 1u << 31;  // 3: directional + BSDF
   }
-  auto shadow_packets = [&]() {
+  auto shadow_packets = [&](const WaveBufs& wb) {
     launch_wave_shadow_packet(false, s.tri_test, s, t, w.sq_o, w.sq_d, nullptr,
-                              &w.counts[11], &w.counts[12], shadow_cap,
+                              &wb.counts[11], &wb.counts[12], shadow_cap,
                               w.term_vis, &ctx->d_counters[1], ctx->d_error,
                               st);
   };
@@ -1287,79 +1287,61 @@ static void run_waves(ajg_scene* sc, const ajg_camera& cam,
       // slowest warp each round; small blocks of work keep the SMs evenly
       // busy to the end), never more than the wave's paths need
       const int gsh = grid_for(a.n_paths, kShadeThreads, kSMs * AJG_SHADE_GRID);
-      cudaMemsetAsync(w.counts, 0, 64, st);
+      cudaMemsetAsync(w.counts, 0, counter_bytes(a.j.max_b), st);
       KernelTimer{ctx, st, -1};
       k_raygen<false><<<grid_for(a.n_paths, kShadeThreads, gs), kShadeThreads,
                         0, st>>>(a, t, w);
       int q = 0;
-      if (overlap && a.j.max_b > 0) extend_ahead(0, w.hits, cam_packets);
+      if (overlap && a.j.max_b > 0) extend_ahead(0, 0, cam_packets);
       for (int b = 0; b < a.j.max_b; ++b) {
-        WaveBufs wb = w;
+        const WaveBufs wb = at_bounce(b, overlap);
         const uint32_t coh = b < ctx->packet_bounces ? coh0 : 0u;
         if (overlap) {
-          wb.hits = (b & 1) ? w.hits2 : w.hits;
           cudaStreamWaitEvent(st, ctx->ev_hits, 0);
-        }
-        // next queue, shadow queues, fetch counters and material lists
-        cudaMemsetAsync(&w.counts[q ^ 1], 0, sizeof(uint32_t), st);
-        if (overlap) {
-          cudaMemsetAsync(&w.counts[2], 0, 6 * sizeof(uint32_t), st);
-          cudaMemsetAsync(&w.counts[9], 0, 4 * sizeof(uint32_t), st);
         } else {
-          cudaMemsetAsync(&w.counts[2], 0, 11 * sizeof(uint32_t), st);
           const bool cam = b == 0 && cam_packets;
           KernelTimer tm(ctx, st, cam ? kcp : kc);
-          extend(q, w.hits, st, cam);
+          extend(wb, q, st, cam);
         }
-        {
-          KernelTimer tm(ctx, st, -1);
-          k_classify<false><<<gs, kClassifyThreads, 0, st>>>(s, t, w.ro[q], &w.counts[q],
-                                                wb.hits, w.lists, &w.counts[4],
-                                                (uint32_t)P);
-        }
-        if ((b == 0 || !a.j.use_mis) && s.env >= 0) {
-          KernelTimer tm(ctx, st, ks);
-          k_shade_miss<false><<<gs, kShadeThreads, 0, st>>>(
-              a, t, wb, b, q, w.lists, &w.counts[4]);
-        }
+        if (!classify_ahead) classify(wb, b, q, st);
         // one shading launch per material class the scene has
         if (s.mat_mask & (1u << AJG_MAT_DIFFUSE)) {
           KernelTimer tm(ctx, st, ks);
           k_shade<AJG_MAT_DIFFUSE, false><<<gsh, kShadeThreads, 0, st>>>(
-              a, t, wb, b, q, w.lists + P, &w.counts[5], (uint32_t)nt,
+              a, t, wb, b, q, w.lists + P, &wb.counts[5], (uint32_t)nt,
               shadow_cap, ctx->d_error, coh);
         }
         if (s.mat_mask & (1u << AJG_MAT_DISNEY)) {
           KernelTimer tm(ctx, st, ks);
           k_shade<AJG_MAT_DISNEY, false><<<gsh, kShadeThreads, 0, st>>>(
-              a, t, wb, b, q, w.lists + 2 * P, &w.counts[6], (uint32_t)nt,
+              a, t, wb, b, q, w.lists + 2 * P, &wb.counts[6], (uint32_t)nt,
               shadow_cap, ctx->d_error, coh);
         }
         if (s.mat_mask >> AJG_MAT_MIRROR) {
           KernelTimer tm(ctx, st, ks);
           k_shade<kMatOther, false><<<gsh, kShadeThreads, 0, st>>>(
-              a, t, wb, b, q, w.lists + 3 * P, &w.counts[7], (uint32_t)nt,
+              a, t, wb, b, q, w.lists + 3 * P, &wb.counts[7], (uint32_t)nt,
               shadow_cap, ctx->d_error, coh);
         }
         if (overlap && b + 1 < a.j.max_b)
-          extend_ahead(q ^ 1, (b & 1) ? w.hits : w.hits2, false);
+          extend_ahead(b + 1, q ^ 1, false);
         if (a.j.use_mis) {
           {
             KernelTimer tm(ctx, st, ka);
-            shadow();
+            shadow(wb);
           }
           if (coh) {
             KernelTimer tm(ctx, st, kap);
-            shadow_packets();
+            shadow_packets(wb);
           }
           if (s.tri_emit) {
             {
               KernelTimer tm(ctx, st, kc);
-              bsdf_closest();
+              bsdf_closest(wb);
             }
             KernelTimer{ctx, st, -1};
             k_bsdf_emit<false><<<gs, kShadeThreads, 0, st>>>(
-                a, t, w, (uint32_t)nt, shadow_cap, (uint32_t)P,
+                a, t, wb, (uint32_t)nt, shadow_cap, (uint32_t)P,
                 reinterpret_cast<const float*>(w.lists),
                 reinterpret_cast<const int32_t*>(w.lists + P));
           }
@@ -1409,73 +1391,74 @@ void enqueue_mj_wave(const MJTables& t, const WaveBufs& w, uint64_t P,
   // and its directional-light shadow rays, in waves without emitters over
   // plain 4-wide trees
   const bool shadow_ok = shadow_packets && !emit && width == 4;
-  auto extend = [&](int q, ajg_hit* hits, cudaStream_t es, bool cam) {
-    if (cam)
-      launch_wave_extend_packet(true, tri_test, s, t, w.ro[q], w.rd[q],
-                                &w.counts[q], &w.counts[8], hits, ctr, err, es);
-    else
-      launch_wave_extend(true, tri_test, closest_width(width), s, t, w.ro[q],
-                         w.rd[q], &w.counts[q], &w.counts[8], hits, ctr, err,
-                         es);
-  };
   // bounce b+1's closest hits on the trace stream beside bounce b's shadow
   // rays, as in the single-job waves (run_waves)
   const bool overlap = ts && ev_queue && ev_hits && w.hits2;
-  auto extend_ahead = [&](int q, ajg_hit* hits, bool cam) {
+  const bool classify_ahead = overlap && !emit;
+  auto at_bounce = [&](int b) {
+    WaveBufs wb = w;
+    wb.counts = w.counts + kCounterWords * b;
+    if (overlap && (b & 1)) wb.hits = w.hits2;
+    return wb;
+  };
+  auto extend = [&](const WaveBufs& wb, int q, cudaStream_t es, bool cam) {
+    if (cam)
+      launch_wave_extend_packet(true, tri_test, s, t, w.ro[q], w.rd[q],
+                                &wb.counts[0], &wb.counts[8], wb.hits, ctr, err,
+                                es);
+    else
+      launch_wave_extend(true, tri_test, closest_width(width), s, t, w.ro[q],
+                         w.rd[q], &wb.counts[0], &wb.counts[8], wb.hits, ctr, err,
+                         es);
+  };
+  auto classify = [&](const WaveBufs& wb, int b, int q, cudaStream_t es) {
+    k_classify<true><<<gs, kClassifyThreads, 0, es>>>(a, t, wb, b, q, (uint32_t)P);
+  };
+  auto extend_ahead = [&](int b, int q, bool cam) {
+    const WaveBufs wb = at_bounce(b);
     cudaEventRecord(ev_queue, st);
     cudaStreamWaitEvent(ts, ev_queue, 0);
-    cudaMemsetAsync(&w.counts[8], 0, sizeof(uint32_t), ts);
-    extend(q, hits, ts, cam);
+    extend(wb, q, ts, cam);
+    if (classify_ahead) classify(wb, b, q, ts);
     cudaEventRecord(ev_hits, ts);
   };
-  cudaMemsetAsync(w.counts, 0, 64, st);
+  cudaMemsetAsync(w.counts, 0, counter_bytes(bounces), st);
   k_raygen<true><<<gs, kShadeThreads, 0, st>>>(a, t, w);
   int q = 0;
-  if (overlap && bounces > 0) extend_ahead(0, w.hits, cam_ok);
+  if (overlap && bounces > 0) extend_ahead(0, 0, cam_ok);
   for (int b = 0; b < bounces; ++b) {
-    WaveBufs wb = w;
-    if (overlap) {
-      wb.hits = (b & 1) ? w.hits2 : w.hits;
-      cudaStreamWaitEvent(st, ev_hits, 0);
-    }
+    const WaveBufs wb = at_bounce(b);
     const uint32_t coh = b == 0 && shadow_ok ? 1u : 0u;
-    cudaMemsetAsync(&w.counts[q ^ 1], 0, sizeof(uint32_t), st);
-    if (overlap) {
-      cudaMemsetAsync(&w.counts[2], 0, 6 * sizeof(uint32_t), st);
-      cudaMemsetAsync(&w.counts[9], 0, 4 * sizeof(uint32_t), st);
-    } else {
-      cudaMemsetAsync(&w.counts[2], 0, 11 * sizeof(uint32_t), st);
-      extend(q, w.hits, st, b == 0 && cam_ok);
-    }
-    k_classify<true><<<gs, kClassifyThreads, 0, st>>>(s, t, w.ro[q], &w.counts[q], wb.hits,
-                                         w.lists, &w.counts[4], (uint32_t)P);
-    k_shade_miss<true><<<gs, kShadeThreads, 0, st>>>(a, t, wb, b, q, w.lists,
-                                                     &w.counts[4]);
+    if (overlap)
+      cudaStreamWaitEvent(st, ev_hits, 0);
+    else
+      extend(wb, q, st, b == 0 && cam_ok);
+    if (!classify_ahead) classify(wb, b, q, st);
     k_shade<AJG_MAT_DIFFUSE, true><<<gsh, kShadeThreads, 0, st>>>(
-        a, t, wb, b, q, w.lists + P, &w.counts[5], (uint32_t)NT, shadow_cap,
+        a, t, wb, b, q, w.lists + P, &wb.counts[5], (uint32_t)NT, shadow_cap,
         err, coh);
     k_shade<AJG_MAT_DISNEY, true><<<gsh, kShadeThreads, 0, st>>>(
-        a, t, wb, b, q, w.lists + 2 * P, &w.counts[6], (uint32_t)NT,
+        a, t, wb, b, q, w.lists + 2 * P, &wb.counts[6], (uint32_t)NT,
         shadow_cap, err, coh);
     k_shade<kMatOther, true><<<gsh, kShadeThreads, 0, st>>>(
-        a, t, wb, b, q, w.lists + 3 * P, &w.counts[7], (uint32_t)NT,
+        a, t, wb, b, q, w.lists + 3 * P, &wb.counts[7], (uint32_t)NT,
         shadow_cap, err, coh);
     if (overlap && b + 1 < bounces)
-      extend_ahead(q ^ 1, (b & 1) ? w.hits : w.hits2, false);
+      extend_ahead(b + 1, q ^ 1, false);
     launch_wave_shadow(true, tri_test, width, s, t, w.sq_o, w.sq_d, w.sq_scene,
-                       &w.counts[2], &w.counts[3], w.term_vis, ctr + 1, err, st);
+                       &wb.counts[2], &wb.counts[3], w.term_vis, ctr + 1, err, st);
     if (coh)
       launch_wave_shadow_packet(true, tri_test, s, t, w.sq_o, w.sq_d,
-                                w.sq_scene, &w.counts[11], &w.counts[12],
+                                w.sq_scene, &wb.counts[11], &wb.counts[12],
                                 shadow_cap, w.term_vis, ctr + 1, err, st);
     if (emit) {
       launch_wave_bsdf_trace(true, tri_test, closest_width(width), s, t, w.sq_o, w.sq_d,
-                             w.sq_scene, &w.counts[9], &w.counts[10], shadow_cap,
+                             w.sq_scene, &wb.counts[9], &wb.counts[10], shadow_cap,
                              (uint32_t)P, reinterpret_cast<float*>(w.lists),
                              reinterpret_cast<int32_t*>(w.lists + P), ctr, err,
                              st);
       k_bsdf_emit<true><<<gs, kShadeThreads, 0, st>>>(
-          a, t, w, (uint32_t)NT, shadow_cap, (uint32_t)P,
+          a, t, wb, (uint32_t)NT, shadow_cap, (uint32_t)P,
           reinterpret_cast<const float*>(w.lists),
           reinterpret_cast<const int32_t*>(w.lists + P));
     }

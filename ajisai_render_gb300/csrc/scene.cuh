@@ -178,13 +178,23 @@ struct WaveBufs {
   float4* sq_o;  // shadow queue: o.xyz, t_max
   float4* sq_d;  // d.xyz, slot bits
   uint16_t* sq_scene;  // multi-job waves: scene index per shadow ray
-  uint32_t* lists;   // [4][P]: queue slots of misses, Lambertian, Disney
-                     // and other hits
-  uint32_t* counts;  // [0],[1] path queues, [2] shadow queue, [3] shadow
-                     // fetch, [4..7] lists, [8] extend fetch, [9] closest
-                     // MIS BSDF queue, [10] its fetch, [11] coherent shadow
-                     // queue (single jobs without emitters), [12] its fetch
+  uint32_t* lists;   // [4][P]: queue slots of Lambertian (1), Disney (2) and
+                     // other (3) hits; the MIS BSDF hits of emitter scenes
+                     // borrow it
+  uint32_t* counts;  // kCounterWords words per bounce, zeroed once a wave (a
+                     // launch's copy points at its bounce's): [0] the path
+                     // queue, [2] shadow queue, [3] shadow fetch, [5..7]
+                     // lists, [8] extend fetch, [9] closest MIS BSDF queue,
+                     // [10] its fetch, [11] coherent shadow queue (waves
+                     // without emitters), [12] its fetch
 };
+constexpr int kCounterWords = 16;
+constexpr int kMaxBounces = 1024;
+// The counters of a wave (they follow its other state and are not part of
+// wave_bytes).
+constexpr uint64_t counter_bytes(int bounces) {
+  return (uint64_t)(bounces + 1) * kCounterWords * sizeof(uint32_t);
+}
 
 // Tables of a multi-job wave in device memory.
 struct MJTables {
@@ -443,6 +453,8 @@ int build_scene(ajg_ctx* ctx, ajg_scene* s, const float* h_tris,
                 const int32_t* h_flags, uint64_t n, const float* world,
                 const ajg_scene_opts& opts);
 // integrator.cu
+// Bytes of a wave's state without its counters; carve_wave lays it out and
+// puts the counters (counter_bytes) behind it.
 uint64_t wave_bytes(uint64_t P, int nt, bool mj);
 WaveBufs carve_wave(char* base, uint64_t P, int nt, bool mj);
 // Enqueues one multi-job wave on `st` (capturable: fixed arguments, queue
@@ -462,7 +474,7 @@ void enqueue_mj_wave(const MJTables& t, const WaveBufs& w, uint64_t P,
 // rays (waves without emitters over plain 4-wide trees).
 inline int mj_wave_kernels(int bounces, bool emit, int width = 0,
                            bool shadow_packets = false) {
-  return 2 + (emit ? 10 : 8) * bounces +
+  return 2 + (emit ? 9 : 7) * bounces +
          (shadow_packets && !emit && width == 4 && bounces > 0 ? 1 : 0);
 }
 // Looks up the persistent grids of the multi-job kernels (call before a

@@ -204,10 +204,10 @@ int Server::ensure_arena(int nt, uint64_t target) {
   P = target;
   NT = std::max(nt, NT > 0 ? NT : 3);
   arena_bytes = wave_bytes(P, NT, true);
-  bool ok = cudaMalloc(&arena, arena_bytes) == cudaSuccess;
+  bool ok = cudaMalloc(&arena, arena_bytes + counter_bytes(kMaxBounces)) == cudaSuccess;
   if (!ok && ctx->mu.try_lock()) {  // the calls' kept scratch gives way
     cudaGetLastError();
-    ok = scratch_drop(ctx) && cudaMalloc(&arena, arena_bytes) == cudaSuccess;
+    ok = scratch_drop(ctx) && cudaMalloc(&arena, arena_bytes + counter_bytes(kMaxBounces)) == cudaSuccess;
     ctx->mu.unlock();
   }
   if (!ok) {

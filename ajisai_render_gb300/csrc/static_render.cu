@@ -20,9 +20,11 @@
 
 namespace {
 
-// 32 MiB: 32 bytes per film pixel plus a wave of at least 1,024 paths.
+// 32 MiB: 32 bytes per film pixel plus a wave of at least 1,024 paths; and
+// behind it the wave's counters.
 constexpr uint64_t kStaticScratchBytes = 32ull << 20;
-static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
+static __device__ __align__(256) unsigned char
+    g_static_scratch[kStaticScratchBytes + ajg::counter_bytes(ajg::kMaxBounces)];
 
 constexpr int kMaxDevices = 64;
 std::mutex g_scratch_mu;
