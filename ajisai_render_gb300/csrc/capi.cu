@@ -2,6 +2,7 @@
 // queries, renders.  Every entry point validates its arguments, runs on the
 // context's stream under the context mutex, and turns CUDA or device-guard
 // failures into a status code plus a message for ajg_last_error().
+#include <algorithm>
 #include <cfloat>
 #include <cstdlib>
 #include <cmath>
@@ -824,39 +825,40 @@ static int trace_host(ajg_scene* s, const ajg_ray* rays, uint64_t n,
   ajg_ray* d_rays = carve<ajg_ray>(cur, n);
   char* d_out = cur;
   CK(cudaMemsetAsync(ctx->d_fetch, 0, kQueryParts * sizeof(uint32_t), st), "trace");
-  // A large batch runs in parts on two streams: a part's rays are copied in
-  // while the part before is traced, and a traversal's last rays run beside
-  // the next part's first (2,000,003 any-hit rays over 327,682 triangles:
-  // the copy takes 355 us, the traversal 594).
-  const int parts = n >= kSplitRays && !ctx->profiling ? kQueryParts : 1;
-  cudaStream_t ss[2] = {st, parts > 1 ? ctx->trace_stream : st};
+  // A large batch runs in parts: the rays of the next are copied in on the
+  // trace stream while one is traced (2,000,003 any-hit rays over 327,682
+  // triangles: the copy takes 355 us, the traversal 594; a part more costs
+  // about 40 us in gaps and drain, so small batches run whole).
+  const int parts =
+      ctx->profiling ? 1
+                     : (int)std::min<uint64_t>(
+                           kQueryParts, std::max<uint64_t>(1, n / kSplitRays));
+  cudaStream_t cs = parts > 1 ? ctx->trace_stream : st;
   if (parts > 1) {
     cudaEventRecord(ctx->ev_queue, st);
-    cudaStreamWaitEvent(ss[1], ctx->ev_queue, 0);
+    cudaStreamWaitEvent(cs, ctx->ev_queue, 0);
   }
   cudaError_t ce = cudaSuccess;
   for (int k = 0; k < parts && ce == cudaSuccess; ++k) {
     const uint64_t a = n * k / parts, m = n * (k + 1) / parts - a;
     ce = cudaMemcpyAsync(d_rays + a, rays + a, m * sizeof(ajg_ray),
-                         cudaMemcpyHostToDevice, ss[k & 1]);
-    KernelTimer tm(ctx, ss[k & 1], any ? kKindAny : kKindClosest);
+                         cudaMemcpyHostToDevice, cs);
+    if (parts > 1) {
+      cudaEventRecord(ctx->ev_queue, cs);
+      cudaStreamWaitEvent(st, ctx->ev_queue, 0);
+    }
+    KernelTimer tm(ctx, st, any ? kKindAny : kKindClosest);
     if (any)
       launch_trace_any(s->d, d_rays + a, m, (uint8_t*)d_out + a, ctx->d_fetch + k,
-                       &ctx->d_counters[1], ctx->d_error, ss[k & 1]);
+                       &ctx->d_counters[1], ctx->d_error, st);
     else
       launch_trace_closest(closest_view(s->d), d_rays + a, m, (ajg_hit*)d_out + a,
-                           ctx->d_fetch + k, &ctx->d_counters[0], ctx->d_error,
-                           ss[k & 1]);
+                           ctx->d_fetch + k, &ctx->d_counters[0], ctx->d_error, st);
   }
-  for (int k = 0; k < parts && ce == cudaSuccess; ++k) {
-    const uint64_t a = n * k / parts, m = n * (k + 1) / parts - a;
-    ce = cudaMemcpyAsync((char*)out + a * rec, d_out + a * rec, m * rec,
-                         cudaMemcpyDeviceToHost, ss[k & 1]);
-  }
-  if (parts > 1) {  // the host buffers are done with when `st` is
-    cudaEventRecord(ctx->ev_hits, ss[1]);
-    cudaStreamWaitEvent(st, ctx->ev_hits, 0);
-  }
+  if (ce == cudaSuccess)
+    ce = cudaMemcpyAsync(out, d_out, n * rec, cudaMemcpyDeviceToHost, st);
+  // (after an error too: the host arrays are done with on return)
+  if (parts > 1 && ce != cudaSuccess) cudaStreamSynchronize(cs);
   const int rc = finish(ctx, st, "trace");
   return ce != cudaSuccess ? cuda_fail(ctx, ce, "trace: copy") : rc;
 }

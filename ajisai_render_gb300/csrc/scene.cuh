@@ -298,9 +298,10 @@ struct PendingTiming {
   int64_t snap;  // the traversal counters' snapshot after it (-1: none)
 };
 constexpr int kLaunchLogCap = 65536;
-// A host ray query of at least kSplitRays rays runs in kQueryParts parts.
+// A host ray query of at least 2 x kSplitRays rays runs in up to kQueryParts
+// parts.
 constexpr int kQueryParts = 4;
-constexpr uint64_t kSplitRays = 1ull << 18;
+constexpr uint64_t kSplitRays = 3ull << 18;
 
 }  // namespace ajg
 
