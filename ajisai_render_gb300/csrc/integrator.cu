@@ -217,6 +217,18 @@ __global__ void __launch_bounds__(kShadeThreads)
   }
 }
 
+// A light term: term_f holds throughput x f, counted once its ray is found
+// unoccluded (kTermSeen, written by the traversal).  An occluded one adds
+// throughput x 0: nothing, except in the rare path whose throughput is not
+// finite (kTermUnseenBad; its throughput is then in thr_shade).
+constexpr uint8_t kTermUnseen = 0, kTermSeen = 1, kTermUnseenBad = 2;
+__device__ __forceinline__ uint8_t term_unseen(F3 T) {
+  return isfinite(T.x) && isfinite(T.y) && isfinite(T.z) ? kTermUnseen
+                                                         : kTermUnseenBad;
+}
+// In place of its path in a queue slot whose ray missed (set by k_classify).
+constexpr uint32_t kMissed = 0x80000000u;
+
 // Files every queue slot under its hit's shading class (Lambertian, Disney, or
 // one of the other material types), so that shading runs in class-specialised
 // kernels, and ends the escaped paths: the environment counts only for camera
@@ -248,17 +260,20 @@ __global__ void __launch_bounds__(kClassifyThreads)
             __float_as_uint(__ldg(&shade[prim].w)) & 0xffffffu;
         const int type = (int)__ldg(materials + 16 * mat);
         cls = type == AJG_MAT_DIFFUSE ? 0 : (type == AJG_MAT_DISNEY ? 1 : 2);
-      } else if (MJ || ((b == 0 || !a.j.use_mis) && a.s.env >= 0)) {
-        const uint32_t p = w.qpath[cur][k];
-        const uint32_t jid = MJ ? mj_job(t, w.pjob[p]) : 0u;
-        const JobParams& J = Src<MJ>::job(a, t, jid);
-        if ((b == 0 || !J.use_mis) && Src<MJ>::scene(a, t, jid).env >= 0) {
-          float4 L = w.rad[p];
-          L.x += J.env_rgb.x;
-          L.y += J.env_rgb.y;
-          L.z += J.env_rgb.z;
-          w.rad[p] = L;
+      } else {
+        if (MJ || ((b == 0 || !a.j.use_mis) && a.s.env >= 0)) {
+          const uint32_t p = w.qpath[cur][k];
+          const uint32_t jid = MJ ? mj_job(t, w.pjob[p]) : 0u;
+          const JobParams& J = Src<MJ>::job(a, t, jid);
+          if ((b == 0 || !J.use_mis) && Src<MJ>::scene(a, t, jid).env >= 0) {
+            float4 L = w.rad[p];
+            L.x += J.env_rgb.x;
+            L.y += J.env_rgb.y;
+            L.z += J.env_rgb.z;
+            w.rad[p] = L;
+          }
         }
+        w.qpath[cur][k] = kMissed;
       }
     }
 #if AJG_BLOCK_APPEND
@@ -333,8 +348,10 @@ __global__ void __launch_bounds__(kShadeThreads)
         }
       }
     }
+    const F3 T = xyz(w.thr_shade[p]);
+    fo = T * fo;
     w.term_f[slot] = make_float4(fo.x, fo.y, fo.z, 0.f);
-    w.term_vis[slot] = vis ? 1 : 0;
+    w.term_vis[slot] = vis ? kTermSeen : term_unseen(T);
   }
 }
 
@@ -444,7 +461,8 @@ __global__ void __launch_bounds__(kShadeThreads, shade_min_blocks<MAT>())
       hi = complete_hit(s, ro, rd, h.t, h.u, h.v, h.prim);
       f.prepare(s.materials + 16 * hi.mat, __ldg(&s.mat_lum[hi.mat].x), hi.ng,
                 hi.ns, hi.wr);
-      w.thr_shade[p] = make_float4(T.x, T.y, T.z, 0.f);
+      if (s.tri_emit || term_unseen(T) != kTermUnseen)
+        w.thr_shade[p] = make_float4(T.x, T.y, T.z, 0.f);
       // an emitter seen by a camera ray, or by any ray without MIS
       // (pt.cpp:185-190, 282-286; AreaLight::Radiance, area_light.cpp:30-34)
       if (emitter >= 0 && (b == 0 || !J.use_mis)) {
@@ -506,6 +524,11 @@ __global__ void __launch_bounds__(kShadeThreads, shade_min_blocks<MAT>())
     DisneyB::Stretched stretched;
     if constexpr (BsdfT<MAT>::kDisney)
       if (hit) stretched = f.b.stretched();
+    // The Lambertian kernels re-read the throughput (L1) where they need it:
+    // held over the rounds it would spill.
+    auto thr = [&]() __attribute__((always_inline)) {
+      return MAT == AJG_MAT_DIFFUSE ? xyz(w.thr[p]) : T;
+    };
     enum Kind { kLight, kMisBsdf, kContinue };
     auto round = [&](Kind kind, int t_) __attribute__((always_inline)) {
       const bool is_light = kind == kLight, is_mis = kind == kMisBsdf;
@@ -611,7 +634,7 @@ __global__ void __launch_bounds__(kShadeThreads, shade_min_blocks<MAT>())
         F3 nro = mk3(0, 0, 0), nrd = mk3(0, 0, 1);
         if (on) {
           if (!(black3(bs.f) || bs.pdf < 0.f)) {
-            T = T * (bs.f * fabsf(dot3(hi.ng, bs.dir)) / bs.pdf);
+            T = thr() * (bs.f * fabsf(dot3(hi.ng, bs.dir)) / bs.pdf);
             make_ray(eps_offset(hi, bs.dir), bs.dir, nro, nrd);
             alive = true;
             if (b + 1 > J.min_b) {
@@ -621,7 +644,7 @@ __global__ void __launch_bounds__(kShadeThreads, shade_min_blocks<MAT>())
                 T = T / J.cont;
             }
           }
-          w.thr[p] = make_float4(T.x, T.y, T.z, 0.f);
+          if (alive) w.thr[p] = make_float4(T.x, T.y, T.z, 0.f);
         }
         // the next bounce's queue
         const uint32_t kn = shade_append(&w.counts[kCounterWords], alive);
@@ -686,8 +709,11 @@ __global__ void __launch_bounds__(kShadeThreads, shade_min_blocks<MAT>())
       }
       const uint32_t slot = p * NT + (is_mis ? NT - 1 : (uint32_t)t_);
       if (on) {
+        // (a closest-hit term is completed, and multiplied, by k_bsdf_emit)
+        const F3 Th = thr();
+        if (!closest) fo = Th * fo;
         w.term_f[slot] = make_float4(fo.x, fo.y, fo.z, cosv);
-        w.term_vis[slot] = 0;
+        w.term_vis[slot] = term_unseen(Th);
         dim += draws;
       }
       // to the packet queue: this term's rays (a single job), or a lane's
@@ -735,8 +761,8 @@ __global__ void __launch_bounds__(kShadeThreads)
   const uint32_t n = w.counts[0];
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n;
        k += gridDim.x * blockDim.x) {
-    if (w.hits[k].prim < 0) continue;
     const uint32_t p = w.qpath[cur][k];
+    if (p == kMissed) continue;
     int nl = (int)a.s.num_lights;
     if constexpr (MJ) {
       const JobParams& J = t.jobs[mj_job(t, w.pjob[p])].j;
@@ -747,12 +773,14 @@ __global__ void __launch_bounds__(kShadeThreads)
         continue;
       }
     }
-    const F3 T = xyz(w.thr_shade[p]);
     F3 direct = mk3(0.f, 0.f, 0.f);
     for (int j = 0; j <= nl; ++j) {
       const uint32_t slot = p * NT + (j < nl ? (uint32_t)j : NT - 1);
-      const F3 fv = w.term_vis[slot] ? xyz(w.term_f[slot]) : mk3(0, 0, 0);
-      direct = direct + T * fv;
+      const uint8_t seen = w.term_vis[slot];
+      if (seen == kTermSeen)
+        direct = direct + xyz(w.term_f[slot]);
+      else if (seen == kTermUnseenBad)
+        direct = direct + xyz(w.thr_shade[p]) * mk3(0, 0, 0);
     }
     float4 L = w.rad[p];
     const F3 d1 = 1.f / 1 * direct;
@@ -994,7 +1022,6 @@ uint64_t wave_bytes(uint64_t P, int nt, bool mj) {
   add(P * 16); add(P * 16);    // ro
   add(P * 16); add(P * 16);    // rd
   add(P * sizeof(ajg_hit));
-  add(P * sizeof(ajg_hit));    // hits2
   add(slots * 16);             // term_f
   add(slots);                  // term_vis
   add(slots * 16); add(slots * 16);  // shadow queue
@@ -1021,7 +1048,6 @@ WaveBufs carve_wave(char* base, uint64_t P, int nt, bool mj) {
   w.rd[0] = carve<float4>(cur, P);
   w.rd[1] = carve<float4>(cur, P);
   w.hits = carve<ajg_hit>(cur, P);
-  w.hits2 = carve<ajg_hit>(cur, P);
   w.term_f = carve<float4>(cur, P * nt);
   w.term_vis = carve<uint8_t>(cur, P * nt);
   w.sq_o = carve<float4>(cur, P * nt);
@@ -1199,12 +1225,10 @@ static void run_waves(ajg_scene* sc, const ajg_camera& cam,
   // bounce 0's camera rays (a pixel's samples side by side in the queue) as
   // masked packets over the binary layout (AJG_PACKET_CAMERA)
   const bool cam_packets = ctx->packet_camera && s_closest.width == 2;
-  // The wave's buffers as bounce b's launches see them: its own counters, and
-  // with overlap the hits of its parity.
-  auto at_bounce = [&](int b, bool overlap) {
+  // the wave's buffers with bounce b's counters
+  auto at_bounce = [&](int b) {
     WaveBufs wb = w;
     wb.counts = w.counts + kCounterWords * b;
-    if (overlap && (b & 1)) wb.hits = w.hits2;
     return wb;
   };
   auto extend = [&](const WaveBufs& wb, int q, cudaStream_t es, bool cam) {
@@ -1223,16 +1247,15 @@ static void run_waves(ajg_scene* sc, const ajg_camera& cam,
   };
   // Bounce b+1's closest hits run on the trace stream beside bounce b's
   // shadow rays: the two persistent launches fill each other's drain.  The
-  // hits alternate between two buffers by bounce parity (k_accumulate of
-  // bounce b still reads its own), and so do the queues; everything else
-  // bounce b+1 touches is written after k_accumulate of bounce b on the
+  // queues alternate by bounce parity, the hits have been shaded; everything
+  // else bounce b+1 touches is written after k_accumulate of bounce b on the
   // render stream.  Its classification follows the hits there, except in
   // scenes with emitters, whose MIS BSDF hits borrow the lists.
-  const bool overlap = ctx->overlap && !ctx->profiling && w.hits2 != nullptr;
+  const bool overlap = ctx->overlap && !ctx->profiling;
   const bool classify_ahead = overlap && !s.tri_emit;
   cudaStream_t ts = ctx->trace_stream;
   auto extend_ahead = [&](int b, int q, bool cam) {
-    const WaveBufs wb = at_bounce(b, true);
+    const WaveBufs wb = at_bounce(b);
     cudaEventRecord(ctx->ev_queue, st);
     cudaStreamWaitEvent(ts, ctx->ev_queue, 0);
     {
@@ -1294,7 +1317,7 @@ static void run_waves(ajg_scene* sc, const ajg_camera& cam,
       int q = 0;
       if (overlap && a.j.max_b > 0) extend_ahead(0, 0, cam_packets);
       for (int b = 0; b < a.j.max_b; ++b) {
-        const WaveBufs wb = at_bounce(b, overlap);
+        const WaveBufs wb = at_bounce(b);
         const uint32_t coh = b < ctx->packet_bounces ? coh0 : 0u;
         if (overlap) {
           cudaStreamWaitEvent(st, ctx->ev_hits, 0);
@@ -1393,12 +1416,11 @@ void enqueue_mj_wave(const MJTables& t, const WaveBufs& w, uint64_t P,
   const bool shadow_ok = shadow_packets && !emit && width == 4;
   // bounce b+1's closest hits on the trace stream beside bounce b's shadow
   // rays, as in the single-job waves (run_waves)
-  const bool overlap = ts && ev_queue && ev_hits && w.hits2;
+  const bool overlap = ts && ev_queue && ev_hits;
   const bool classify_ahead = overlap && !emit;
   auto at_bounce = [&](int b) {
     WaveBufs wb = w;
     wb.counts = w.counts + kCounterWords * b;
-    if (overlap && (b & 1)) wb.hits = w.hits2;
     return wb;
   };
   auto extend = [&](const WaveBufs& wb, int q, cudaStream_t es, bool cam) {

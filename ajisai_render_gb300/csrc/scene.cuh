@@ -160,7 +160,8 @@ constexpr int kMaxWaveChunks = 1024;
 struct WaveBufs {
   // by path
   float4* thr;
-  float4* thr_shade;
+  float4* thr_shade;  // throughput at the shaded hit: emitter scenes, and
+                      // paths whose throughput is not finite
   float4* rad;
   uint32_t* pjob;  // multi-job waves: the path's job
   uint64_t* pkey;  // multi-job waves: the path's sampler key
@@ -170,9 +171,8 @@ struct WaveBufs {
   float4* ro[2];
   float4* rd[2];
   ajg_hit* hits;
-  ajg_hit* hits2;  // single-job waves: bounce parity 1's hits (overlap)
-  // light terms: slot = path * NT + term (lights first, the MIS BSDF term
-  // last at NT - 1)
+  // light terms, throughput included: slot = path * NT + term (lights first,
+  // the MIS BSDF term last at NT - 1)
   float4* term_f;
   uint8_t* term_vis;
   float4* sq_o;  // shadow queue: o.xyz, t_max
