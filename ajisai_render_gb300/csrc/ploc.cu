@@ -674,8 +674,8 @@ __global__ void k_bvh2(const PNode* __restrict__ nodes, uint64_t m,
     const uint32_t c0 = (uint32_t)__float_as_int(x.a.w);
     const PNode a = nodes[c0], b = nodes[c0 + 1];
     float4* o = bvh + 4 * (uint64_t)compact[k];
-    o[0] = make_float4(a.a.x, a.b.x, a.a.y, a.b.y);
-    o[1] = make_float4(b.a.x, b.b.x, b.a.y, b.b.y);
+    o[0] = make_float4(a.a.x, a.a.y, a.b.x, a.b.y);
+    o[1] = make_float4(b.a.x, b.a.y, b.b.x, b.b.y);
     o[2] = make_float4(a.a.z, a.b.z, b.a.z, b.b.z);
     o[3] = make_float4(__int_as_float(child_ref(nodes, compact, c0)),
                        __int_as_float(child_ref(nodes, compact, c0 + 1)), 0.f,
@@ -687,7 +687,7 @@ __global__ void k_bvh2(const PNode* __restrict__ nodes, uint64_t m,
 __global__ void k_bvh2_single(const PNode* __restrict__ nodes,
                               float4* __restrict__ bvh) {
   const PNode a = nodes[0];
-  bvh[0] = make_float4(a.a.x, a.b.x, a.a.y, a.b.y);
+  bvh[0] = make_float4(a.a.x, a.a.y, a.b.x, a.b.y);
   bvh[1] = bvh[0];
   bvh[2] = make_float4(a.a.z, a.b.z, a.a.z, a.b.z);
   bvh[3] = make_float4(__int_as_float(~0), __int_as_float(~0), 0.f, 0.f);
@@ -699,10 +699,24 @@ __global__ void k_bvh2_single(const PNode* __restrict__ nodes,
 // only leaves); its interior children become the wide nodes of the next
 // level, allocated contiguously.  A level's length is a counter of its own
 // (n_in, n_out), so levels are enqueued without the host reading them.  Node
-// layout (2W float4, 32W bytes): the
-// children's lo.x, hi.x, lo.y, hi.y, lo.z, hi.z in groups of four, then the
-// references (>= 0 wide node, ~slot leaf, kEmptyRef unused), then padding.
+// layout (2W float4, 32W bytes) for W = 8: the children's lo.x, hi.x, lo.y,
+// hi.y, lo.z, hi.z in groups of four, then the references (>= 0 wide node,
+// ~slot leaf, kWideEmpty unused), then padding; for W = 4: wide4_node.
 constexpr int kWideEmpty = (int)0x80000000;
+
+// A 4-wide node (8 float4) from its children's planes (lo.x, hi.x, lo.y, hi.y,
+// lo.z, hi.z) and references: per child (lo.x, lo.y, hi.x, hi.y), then the
+// children's (lo.z, hi.z), the references, padding.
+__device__ __forceinline__ void wide4_node(float4* o, const float pl[6][4],
+                                           const int rf[4]) {
+  for (int c = 0; c < 4; ++c)
+    o[c] = make_float4(pl[0][c], pl[2][c], pl[1][c], pl[3][c]);
+  o[4] = make_float4(pl[4][0], pl[5][0], pl[4][1], pl[5][1]);
+  o[5] = make_float4(pl[4][2], pl[5][2], pl[4][3], pl[5][3]);
+  o[6] = make_float4(__int_as_float(rf[0]), __int_as_float(rf[1]),
+                     __int_as_float(rf[2]), __int_as_float(rf[3]));
+  o[7] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
 
 template <int W>
 __global__ void k_collapse(const PNode* __restrict__ nodes,
@@ -769,14 +783,18 @@ __global__ void k_collapse(const PNode* __restrict__ nodes,
       }
     }
     float4* o = wide + (uint64_t)e.y * (2 * W);
-    for (int g = 0; g < G; ++g) {
-      for (int k = 0; k < 6; ++k)
-        o[k * G + g] = make_float4(pl[k][4 * g], pl[k][4 * g + 1],
-                                   pl[k][4 * g + 2], pl[k][4 * g + 3]);
-      o[6 * G + g] = make_float4(
-          __int_as_float(rf[4 * g]), __int_as_float(rf[4 * g + 1]),
-          __int_as_float(rf[4 * g + 2]), __int_as_float(rf[4 * g + 3]));
-      o[7 * G + g] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if constexpr (W == 4) {
+      wide4_node(o, pl, rf);
+    } else {
+      for (int g = 0; g < G; ++g) {
+        for (int k = 0; k < 6; ++k)
+          o[k * G + g] = make_float4(pl[k][4 * g], pl[k][4 * g + 1],
+                                     pl[k][4 * g + 2], pl[k][4 * g + 3]);
+        o[6 * G + g] = make_float4(
+            __int_as_float(rf[4 * g]), __int_as_float(rf[4 * g + 1]),
+            __int_as_float(rf[4 * g + 2]), __int_as_float(rf[4 * g + 3]));
+        o[7 * G + g] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
     }
   }
 }
@@ -859,11 +877,7 @@ __global__ void k_collapse_sah(const PNode* __restrict__ nodes,
       }
     }
     float4* o = wide + (uint64_t)e.y * (2 * W);
-    for (int k = 0; k < 6; ++k)
-      o[k] = make_float4(pl[k][0], pl[k][1], pl[k][2], pl[k][3]);
-    o[6] = make_float4(__int_as_float(rf[0]), __int_as_float(rf[1]),
-                       __int_as_float(rf[2]), __int_as_float(rf[3]));
-    o[7] = make_float4(0.f, 0.f, 0.f, 0.f);
+    wide4_node(o, pl, rf);
   }
 }
 

@@ -12,7 +12,7 @@ namespace ajg {
 
 // HBM layout of a built scene (all arrays are device pointers):
 //   bvh    width 2: [inner][4] float4, two child boxes per interior node:
-//          (c0.lo.x, c0.hi.x, c0.lo.y, c0.hi.y), (c1 ... same),
+//          (c0.lo.x, c0.lo.y, c0.hi.x, c0.hi.y), (c1 ... same),
 //          (c0.lo.z, c0.hi.z, c1.lo.z, c1.hi.z), (ref0, ref1, -, -) where a
 //          ref >= 0 is an interior node and ~slot a leaf;
 //          width W = 4, 8: [nodes][2W] float4 of the collapsed tree (see
