@@ -446,18 +446,20 @@ __device__ __forceinline__ void trace_persistent(
     t = stack_t[sp];
   };
 #endif
+  // lanes without a ray for good: only a refill adds to them
+  unsigned done = __ballot_sync(full, k == kDone);
   for (;;) {
     const unsigned idle = __ballot_sync(full, k == kIdle);
-    const unsigned done = __ballot_sync(full, k == kDone);
+    unsigned act = ~(idle | done);
     constexpr int kRefillQ = ANY ? AJG_REFILL_ANY : kRefill;
-    if (idle && (__popc(idle) >= kRefillQ || (idle | done) == full)) {
+    if (__popc(idle) >= kRefillQ || (idle | done) == full) {
       uint32_t base = own;
       own = kTaken;
       if (base == kTaken) {
         // rays past the warps' own, if any
         const uint32_t fixed = gridDim.x * blockDim.x;
         base = n;
-        if (n > fixed) {
+        if (idle && n > fixed) {
           const int leader = __ffs(idle) - 1;
           if (lane == leader) base = fixed + atomicAdd(next, (uint32_t)__popc(idle));
           base = __shfl_sync(full, base, leader);
@@ -479,13 +481,14 @@ __device__ __forceinline__ void trace_persistent(
           k = kDone;
         }
       }
+      done = __ballot_sync(full, k == kDone);
+      if (done == full) break;
+      act = ~done;
     }
-    if (__all_sync(full, k == kDone)) break;
     if constexpr (kDefer) {
-      const bool act = k >= 0 && k != kDone;
-      const unsigned pm = __ballot_sync(full, act && pend != 0);
-      const unsigned am = __ballot_sync(full, act);
-      if (pm && (__popc(pm) >= kLeafPass || pm == am)) {
+      // (lanes without a ray hold no leaves)
+      const unsigned pm = __ballot_sync(full, pend != 0);
+      if (pm && (__popc(pm) >= kLeafPass || pm == act)) {
         // the leaf pass
         if (pend) {
           const int c = __ffs(pend) - 1;
