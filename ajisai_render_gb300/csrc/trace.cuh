@@ -335,6 +335,16 @@ constexpr int trace_min_blocks() {
                           // tests pending leaves together once this many
                           // lanes hold some (0: each visit tests its leaves)
 #endif
+#ifndef AJG_VISITS_ANY
+#define AJG_VISITS_ANY 3  // any-hit queries: node visits between the loop's
+                          // votes (a lane leaves early with a leaf found or its
+                          // ray done).  Any-hit ms of the Cornell box, the 1.3 M
+                          // sphere and 16 batched jobs: 1 visit 1.77 / 24.9 /
+                          // 19.5, 2 1.81 / 24.5 / -, 3 1.70 / 24.5 / 18.9, 4
+                          // 1.80 / 25.0 / 19.1, 6 1.82 / 26.0 / 19.8.  Closest
+                          // hits, with their leaf tests in the visit: 1 visit
+                          // 20.2 ms, 2 20.6, 3 20.3, 4 20.7
+#endif
 #ifndef AJG_LEAF_DEFER_CLOSEST
 #define AJG_LEAF_DEFER_CLOSEST 0  // the same for closest-hit queries over
                                   // the binary layout
@@ -375,7 +385,8 @@ __device__ __forceinline__ void trace_persistent(
   WtSetup w;
   Hit hit;
   int node = 0, sp = 0;
-  uint32_t visits = 0;
+  uint32_t visit_end = 0;  // the visit count past which a ray is stopped
+  constexpr int kVisits = ANY ? AJG_VISITS_ANY : 1;
   // Deferred leaves: a node visit records its leaf children (mask `pend`,
   // slots pend_slot[child]) instead of testing them, and a lane holding
   // pending leaves visits no node (nor pops one) until the warp's next leaf
@@ -476,7 +487,7 @@ __device__ __forceinline__ void trace_persistent(
           hit.u = hit.v = 0.f;
           node = 0;
           sp = 0;
-          visits = 0;
+          visit_end = n_nodes + ts.max_visits;
         } else {
           k = kDone;
         }
@@ -522,296 +533,296 @@ __device__ __forceinline__ void trace_persistent(
         }
         continue;
       }
-      if (pend) continue;  // waits for the leaf pass
     }
-    if (k < 0 || k == kDone) continue;
-
-    // one node visit
-    bool finished = false;
-    ++n_nodes;
-    if (++visits > ts.max_visits) {
-      raise_device_error(err, kDevIterationBound);
-      finish((uint32_t)k, hit, hit.prim >= 0);
-      k = kIdle;
-      pend = 0;
-      continue;
-    }
-    const float4* __restrict__ bvh = ts.bvh;
-    const float4* __restrict__ tris = ts.tris;
-    const float lim = ANY ? r.tmax : fminf(hit.t, r.tmax);
-    bool descend = false;  // `node` holds the next node to visit
-    if constexpr (W == 2) {
-      uint64_t q[8];
-      ldg_pairs(bvh + 4 * (uint64_t)node, q);
-      ldg_pairs(bvh + 4 * (uint64_t)node + 2, q + 4);
-      float tn0, tn1;
-      bool h0 = slab_pairs(q[0], q[1], q[4], r, lim, tn0);
-      bool h1 = slab_pairs(q[2], q[3], q[5], r, lim, tn1);
-      int r0, r1;
-      unpack_refs(q[6], r0, r1);
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const bool hc = c == 0 ? h0 : h1;
-        const int rc = c == 0 ? r0 : r1;
-        if (kDefer && hc && rc < 0) {
-          pend |= 1u << c;
-          pend_slot[c] = ~rc;
-        } else if (hc && rc < 0 && !finished) {
-          ++n_tris;
-          finished = leaf_test<TEST, ANY>(tris, ~rc, r, w, hit);
-        }
-        if (hc && rc < 0) {
-          if (c == 0)
-            h0 = false;
-          else
-            h1 = false;
-        }
+    // node visits
+#pragma unroll 1
+    for (int u = 0; u < kVisits; ++u) {
+      if (k < 0 || k == kDone || (kDefer && pend)) break;
+      bool finished = false;
+      if (n_nodes++ == visit_end) {
+        raise_device_error(err, kDevIterationBound);
+        finish((uint32_t)k, hit, hit.prim >= 0);
+        k = kIdle;
+        pend = 0;
+        continue;
       }
-      if (!finished) {
-        if (h0 && h1) {
-          const bool first0 = tn0 <= tn1;
-          if (sp >= kStack) {
-            raise_device_error(err, kDevStackOverflow);
-            finished = true;
-          } else {
-            push(first0 ? r1 : r0, first0 ? tn1 : tn0);
-            node = first0 ? r0 : r1;
-            descend = true;
+      const float4* __restrict__ bvh = ts.bvh;
+      const float4* __restrict__ tris = ts.tris;
+      const float lim = ANY ? r.tmax : fminf(hit.t, r.tmax);
+      bool descend = false;  // `node` holds the next node to visit
+      if constexpr (W == 2) {
+        uint64_t q[8];
+        ldg_pairs(bvh + 4 * (uint64_t)node, q);
+        ldg_pairs(bvh + 4 * (uint64_t)node + 2, q + 4);
+        float tn0, tn1;
+        bool h0 = slab_pairs(q[0], q[1], q[4], r, lim, tn0);
+        bool h1 = slab_pairs(q[2], q[3], q[5], r, lim, tn1);
+        int r0, r1;
+        unpack_refs(q[6], r0, r1);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const bool hc = c == 0 ? h0 : h1;
+          const int rc = c == 0 ? r0 : r1;
+          if (kDefer && hc && rc < 0) {
+            pend |= 1u << c;
+            pend_slot[c] = ~rc;
+          } else if (hc && rc < 0 && !finished) {
+            ++n_tris;
+            finished = leaf_test<TEST, ANY>(tris, ~rc, r, w, hit);
           }
-        } else if (h0) {
-          node = r0;
-          descend = true;
-        } else if (h1) {
-          node = r1;
-          descend = true;
+          if (hc && rc < 0) {
+            if (c == 0)
+              h0 = false;
+            else
+              h1 = false;
+          }
         }
-      }
-    } else {
-      float tn[W];
-      int ref[W] = {};
-      unsigned inner = 0;  // interior children whose box passed
-#if AJG_LEAF_BATCH
-      // leaf children whose box passed (mask `leaves`, slot per child, both
-      // indexed by the child so that they stay in registers), tested after
-      // the box tests from one call site (all lanes with an i-th leaf test
-      // it together)
-      int leaf_slot[W];
-      unsigned leaves = 0;
-#endif
-      // files child c, whose box passed or not
-      auto child = [&](int c, bool h) {
-#if AJG_LEAF_BATCH
-        if (kDefer && h && ref[c] < 0) {
-          pend |= 1u << c;
-          pend_slot[c] = ~ref[c];
-        } else if (h && ref[c] < 0) {
-          leaf_slot[c] = ~ref[c];
-          leaves |= 1u << c;
-        }
-#else
-        if (h && ref[c] < 0 && !finished) {
-          ++n_tris;
-          finished = leaf_test<TEST, ANY>(tris, ~ref[c], r, w, hit);
-        }
-#endif
-        if (h && ref[c] >= 0) inner |= 1u << c;
-      };
-      if constexpr (!CMP && W == 4) {
-        const float4* nd = bvh + (uint64_t)node * 8;
-        uint64_t q[16];  // the node, the last two padding
-#pragma unroll
-        for (int i = 0; i < 4; ++i) ldg_pairs(nd + 2 * i, q + 4 * i);
-        unpack_refs(q[12], ref[0], ref[1]);
-        unpack_refs(q[13], ref[2], ref[3]);
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-          child(c, ref[c] != kEmptyRef && slab_pairs(q[2 * c], q[2 * c + 1],
-                                                     q[8 + c], r, lim, tn[c]));
-      } else if constexpr (!CMP) {
-        constexpr int G = W / 4;  // float4 groups per plane
-        const float4* nd = bvh + (uint64_t)node * (2 * W);
-        float4 q[8 * G];  // the node's 2W float4, the last G padding
-#pragma unroll
-        for (int i = 0; i < 7 * G; i += 2) ldg_node(nd + i, q[i], q[i + 1]);
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-          const float4 lx = q[0 * G + g], hx = q[1 * G + g];
-          const float4 ly = q[2 * G + g], hy = q[3 * G + g];
-          const float4 lz = q[4 * G + g], hz = q[5 * G + g];
-          const float4 rf = q[6 * G + g];
-          const float* plx = &lx.x;
-          const float* phx = &hx.x;
-          const float* ply = &ly.x;
-          const float* phy = &hy.x;
-          const float* plz = &lz.x;
-          const float* phz = &hz.x;
-          const float* prf = &rf.x;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int c = 4 * g + j;
-            ref[c] = __float_as_int(prf[j]);
-            child(c, ref[c] != kEmptyRef &&
-                         slab2(plx[j], phx[j], ply[j], phy[j], plz[j], phz[j], r,
-                               lim, tn[c]));
+        if (!finished) {
+          if (h0 && h1) {
+            const bool first0 = tn0 <= tn1;
+            if (sp >= kStack) {
+              raise_device_error(err, kDevStackOverflow);
+              finished = true;
+            } else {
+              push(first0 ? r1 : r0, first0 ? tn1 : tn0);
+              node = first0 ? r0 : r1;
+              descend = true;
+            }
+          } else if (h0) {
+            node = r0;
+            descend = true;
+          } else if (h1) {
+            node = r1;
+            descend = true;
           }
         }
       } else {
-        constexpr int NF = CwLayout<W>::kFloat4;
-        const float4* nd = bvh + (uint64_t)node * NF;
-        const float4 h0 = __ldg(nd), h1 = __ldg(nd + 1);
-        uint32_t qw[4 * (NF - 2)];
-#pragma unroll
-        for (int f = 0; f < NF - 2; ++f) {
-          const float4 v = __ldg(nd + 2 + f);
-          qw[4 * f] = __float_as_uint(v.x);
-          qw[4 * f + 1] = __float_as_uint(v.y);
-          qw[4 * f + 2] = __float_as_uint(v.z);
-          qw[4 * f + 3] = __float_as_uint(v.w);
-        }
-        const uint32_t hb = __float_as_uint(h0.w);
-        const float sx = cw_scale(hb & 0xffu);
-        const float sy = cw_scale((hb >> 8) & 0xffu);
-        const float sz = cw_scale((hb >> 16) & 0xffu);
-        const uint32_t imask = hb >> 24;
-        const uint32_t cbase = __float_as_uint(h1.x);
-        const uint32_t tbase = __float_as_uint(h1.y);
-        const uint32_t vmask = __float_as_uint(h1.z);
-        const uint32_t lmask = vmask & ~imask;
-#pragma unroll
-        for (int c = 0; c < W; ++c) {
-          tn[c] = 0.f;
-          ref[c] = 0;
-          if (!((vmask >> c) & 1u)) continue;
-          // plane k of child c: byte c of the plane's W bytes, decoded
-          // exactly as the build checked it
-          auto plane = [&](int k, float origin, float sc) {
-            const uint32_t word = qw[k * (W / 4) + (c >> 2)];
-            const uint32_t bits =
-                __byte_perm(word, 0x4B000000u, (uint32_t)(c & 3) | 0x7540u);
-            return cw_decode(origin, cw_qfloat(bits), sc);
-          };
-          float t0;
-          if (!slab2(plane(0, h0.x, sx), plane(1, h0.x, sx),
-                     plane(2, h0.y, sy), plane(3, h0.y, sy),
-                     plane(4, h0.z, sz), plane(5, h0.z, sz), r, lim, t0))
-            continue;
-          tn[c] = t0;
-          const uint32_t below = (1u << c) - 1u;
-          if ((imask >> c) & 1u) {
-            ref[c] = (int)(cbase + __popc(imask & below));
-            inner |= 1u << c;
-          } else {
+        float tn[W];
+        int ref[W] = {};
+        unsigned inner = 0;  // interior children whose box passed
 #if AJG_LEAF_BATCH
-            leaf_slot[c] = (int)(tbase + __popc(lmask & below));
+        // leaf children whose box passed (mask `leaves`, slot per child, both
+        // indexed by the child so that they stay in registers), tested after
+        // the box tests from one call site (all lanes with an i-th leaf test
+        // it together)
+        int leaf_slot[W];
+        unsigned leaves = 0;
+#endif
+        // files child c, whose box passed or not
+        auto child = [&](int c, bool h) {
+#if AJG_LEAF_BATCH
+          if (kDefer && h && ref[c] < 0) {
+            pend |= 1u << c;
+            pend_slot[c] = ~ref[c];
+          } else if (h && ref[c] < 0) {
+            leaf_slot[c] = ~ref[c];
             leaves |= 1u << c;
+          }
 #else
-            if (!finished) {
-              ++n_tris;
-              finished = leaf_test<TEST, ANY>(
-                  tris, (int)(tbase + __popc(lmask & below)), r, w, hit);
-            }
-#endif
+          if (h && ref[c] < 0 && !finished) {
+            ++n_tris;
+            finished = leaf_test<TEST, ANY>(tris, ~ref[c], r, w, hit);
           }
-        }
-      }
+#endif
+          if (h && ref[c] >= 0) inner |= 1u << c;
+        };
+        if constexpr (!CMP && W == 4) {
+          const float4* nd = bvh + (uint64_t)node * 8;
+          uint64_t q[16];  // the node, the last two padding
+#pragma unroll
+          for (int i = 0; i < 4; ++i) ldg_pairs(nd + 2 * i, q + 4 * i);
+          unpack_refs(q[12], ref[0], ref[1]);
+          unpack_refs(q[13], ref[2], ref[3]);
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            child(c, ref[c] != kEmptyRef && slab_pairs(q[2 * c], q[2 * c + 1],
+                                                       q[8 + c], r, lim, tn[c]));
+        } else if constexpr (!CMP) {
+          constexpr int G = W / 4;  // float4 groups per plane
+          const float4* nd = bvh + (uint64_t)node * (2 * W);
+          float4 q[8 * G];  // the node's 2W float4, the last G padding
+#pragma unroll
+          for (int i = 0; i < 7 * G; i += 2) ldg_node(nd + i, q[i], q[i + 1]);
+#pragma unroll
+          for (int g = 0; g < G; ++g) {
+            const float4 lx = q[0 * G + g], hx = q[1 * G + g];
+            const float4 ly = q[2 * G + g], hy = q[3 * G + g];
+            const float4 lz = q[4 * G + g], hz = q[5 * G + g];
+            const float4 rf = q[6 * G + g];
+            const float* plx = &lx.x;
+            const float* phx = &hx.x;
+            const float* ply = &ly.x;
+            const float* phy = &hy.x;
+            const float* plz = &lz.x;
+            const float* phz = &hz.x;
+            const float* prf = &rf.x;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const int c = 4 * g + j;
+              ref[c] = __float_as_int(prf[j]);
+              child(c, ref[c] != kEmptyRef &&
+                           slab2(plx[j], phx[j], ply[j], phy[j], plz[j], phz[j], r,
+                                 lim, tn[c]));
+            }
+          }
+        } else {
+          constexpr int NF = CwLayout<W>::kFloat4;
+          const float4* nd = bvh + (uint64_t)node * NF;
+          const float4 h0 = __ldg(nd), h1 = __ldg(nd + 1);
+          uint32_t qw[4 * (NF - 2)];
+#pragma unroll
+          for (int f = 0; f < NF - 2; ++f) {
+            const float4 v = __ldg(nd + 2 + f);
+            qw[4 * f] = __float_as_uint(v.x);
+            qw[4 * f + 1] = __float_as_uint(v.y);
+            qw[4 * f + 2] = __float_as_uint(v.z);
+            qw[4 * f + 3] = __float_as_uint(v.w);
+          }
+          const uint32_t hb = __float_as_uint(h0.w);
+          const float sx = cw_scale(hb & 0xffu);
+          const float sy = cw_scale((hb >> 8) & 0xffu);
+          const float sz = cw_scale((hb >> 16) & 0xffu);
+          const uint32_t imask = hb >> 24;
+          const uint32_t cbase = __float_as_uint(h1.x);
+          const uint32_t tbase = __float_as_uint(h1.y);
+          const uint32_t vmask = __float_as_uint(h1.z);
+          const uint32_t lmask = vmask & ~imask;
+#pragma unroll
+          for (int c = 0; c < W; ++c) {
+            tn[c] = 0.f;
+            ref[c] = 0;
+            if (!((vmask >> c) & 1u)) continue;
+            // plane k of child c: byte c of the plane's W bytes, decoded
+            // exactly as the build checked it
+            auto plane = [&](int k, float origin, float sc) {
+              const uint32_t word = qw[k * (W / 4) + (c >> 2)];
+              const uint32_t bits =
+                  __byte_perm(word, 0x4B000000u, (uint32_t)(c & 3) | 0x7540u);
+              return cw_decode(origin, cw_qfloat(bits), sc);
+            };
+            float t0;
+            if (!slab2(plane(0, h0.x, sx), plane(1, h0.x, sx),
+                       plane(2, h0.y, sy), plane(3, h0.y, sy),
+                       plane(4, h0.z, sz), plane(5, h0.z, sz), r, lim, t0))
+              continue;
+            tn[c] = t0;
+            const uint32_t below = (1u << c) - 1u;
+            if ((imask >> c) & 1u) {
+              ref[c] = (int)(cbase + __popc(imask & below));
+              inner |= 1u << c;
+            } else {
 #if AJG_LEAF_BATCH
-      while (leaves && !finished) {
-        const int c = __ffs(leaves) - 1;
-        leaves &= leaves - 1;
-        ++n_tris;
-        int slot = 0;
-#pragma unroll
-        for (int j = 0; j < W; ++j)
-          if (j == c) slot = leaf_slot[j];
-        finished = leaf_test<TEST, ANY>(tris, slot, r, w, hit);
-      }
+              leaf_slot[c] = (int)(tbase + __popc(lmask & below));
+              leaves |= 1u << c;
+#else
+              if (!finished) {
+                ++n_tris;
+                finished = leaf_test<TEST, ANY>(
+                    tris, (int)(tbase + __popc(lmask & below)), r, w, hit);
+              }
 #endif
-      if (!finished && inner && ANY) {
-        // occlusion: any order will do -- visit the first, push the rest
-        const int c0 = __ffs(inner) - 1;
-        inner &= inner - 1;
-        while (inner && !finished) {
-          const int c = __ffs(inner) - 1;
+            }
+          }
+        }
+#if AJG_LEAF_BATCH
+        while (leaves && !finished) {
+          const int c = __ffs(leaves) - 1;
+          leaves &= leaves - 1;
+          ++n_tris;
+          int slot = 0;
+#pragma unroll
+          for (int j = 0; j < W; ++j)
+            if (j == c) slot = leaf_slot[j];
+          finished = leaf_test<TEST, ANY>(tris, slot, r, w, hit);
+        }
+#endif
+        if (!finished && inner && ANY) {
+          // occlusion: any order will do -- visit the first, push the rest
+          const int c0 = __ffs(inner) - 1;
           inner &= inner - 1;
-          if (sp >= kStack) {
-            raise_device_error(err, kDevStackOverflow);
-            finished = true;
-            break;
-          }
-          int fr = 0;
-          float ft = 0.f;
-#pragma unroll
-          for (int cc = 0; cc < W; ++cc)
-            if (cc == c) {
-              fr = ref[cc];
-              ft = tn[cc];
+          while (inner && !finished) {
+            const int c = __ffs(inner) - 1;
+            inner &= inner - 1;
+            if (sp >= kStack) {
+              raise_device_error(err, kDevStackOverflow);
+              finished = true;
+              break;
             }
-          push(fr, ft);
-        }
-        if (!finished) {
-          int nr = 0;
+            int fr = 0;
+            float ft = 0.f;
 #pragma unroll
-          for (int cc = 0; cc < W; ++cc)
-            if (cc == c0) nr = ref[cc];
-          node = nr;
-          descend = true;
-        }
-      } else if (!finished && inner) {
-        // push all but the nearest, farthest first
-        while (__popc(inner) > 1) {
-          int far_c = -1;
-          float far_t = -__int_as_float(0x7f800000);
-#pragma unroll
-          for (int c = 0; c < W; ++c)
-            if (((inner >> c) & 1u) && (far_c < 0 || tn[c] > far_t)) {
-              far_c = c;
-              far_t = tn[c];
-            }
-          if (sp >= kStack) {
-            raise_device_error(err, kDevStackOverflow);
-            finished = true;
-            break;
+            for (int cc = 0; cc < W; ++cc)
+              if (cc == c) {
+                fr = ref[cc];
+                ft = tn[cc];
+              }
+            push(fr, ft);
           }
-          int fr = 0;
+          if (!finished) {
+            int nr = 0;
 #pragma unroll
-          for (int c = 0; c < W; ++c)
-            if (c == far_c) fr = ref[c];
-          push(fr, far_t);
-          inner &= ~(1u << far_c);
-        }
-        if (!finished) {
-          const int c = __ffs(inner) - 1;
-          int nr = 0;
+            for (int cc = 0; cc < W; ++cc)
+              if (cc == c0) nr = ref[cc];
+            node = nr;
+            descend = true;
+          }
+        } else if (!finished && inner) {
+          // push all but the nearest, farthest first
+          while (__popc(inner) > 1) {
+            int far_c = -1;
+            float far_t = -__int_as_float(0x7f800000);
 #pragma unroll
-          for (int cc = 0; cc < W; ++cc)
-            if (cc == c) nr = ref[cc];
-          node = nr;
-          descend = true;
+            for (int c = 0; c < W; ++c)
+              if (((inner >> c) & 1u) && (far_c < 0 || tn[c] > far_t)) {
+                far_c = c;
+                far_t = tn[c];
+              }
+            if (sp >= kStack) {
+              raise_device_error(err, kDevStackOverflow);
+              finished = true;
+              break;
+            }
+            int fr = 0;
+#pragma unroll
+            for (int c = 0; c < W; ++c)
+              if (c == far_c) fr = ref[c];
+            push(fr, far_t);
+            inner &= ~(1u << far_c);
+          }
+          if (!finished) {
+            const int c = __ffs(inner) - 1;
+            int nr = 0;
+#pragma unroll
+            for (int cc = 0; cc < W; ++cc)
+              if (cc == c) nr = ref[cc];
+            node = nr;
+            descend = true;
+          }
         }
       }
-    }
-    if (kDefer && !finished && !descend && pend) {
-      node = -1;  // pops after the leaf pass
-    } else if (!finished && !descend) {
-      // pop, skipping boxes a closer hit has since excluded
-      finished = true;
-      while (sp > 0) {
-        int nd;
-        float st;
-        pop(nd, st);
-        const float lim2 = ANY ? r.tmax : fminf(hit.t, r.tmax);
-        if (st <= lim2) {
-          node = nd;
-          finished = false;
-          break;
+      if (kDefer && !finished && !descend && pend) {
+        node = -1;  // pops after the leaf pass
+      } else if (!finished && !descend) {
+        // pop, skipping boxes a closer hit has since excluded
+        finished = true;
+        while (sp > 0) {
+          int nd;
+          float st;
+          pop(nd, st);
+          const float lim2 = ANY ? r.tmax : fminf(hit.t, r.tmax);
+          if (st <= lim2) {
+            node = nd;
+            finished = false;
+            break;
+          }
         }
       }
-    }
-    if (finished) {
-      ++n_rays;
-      finish((uint32_t)k, hit, hit.prim >= 0);
-      k = kIdle;
-      pend = 0;
+      if (finished) {
+        ++n_rays;
+        finish((uint32_t)k, hit, hit.prim >= 0);
+        k = kIdle;
+        pend = 0;
+      }
     }
   }
 }
