@@ -9,13 +9,14 @@
 //     (photon_mapping.h:69-148): 40960 hash entries, each visible point
 //     filed under the cells [lo, hi) of its radius box -- built as count,
 //     scan and fill over the entries instead of linked lists;
-//   the photon pass (TracerPhoton, sppm.cpp:103-143) as a wavefront: emit
+//   the photon pass (TracerPhoton, sppm.cpp:103-143) as a wavefront, of one
+//     iteration or several (photons do not depend on the visible points): emit
 //     from a light chosen by the scene's uniform selector, then per depth a
 //     closest-hit traversal and a shading kernel that records the photon's
 //     deposit and samples the BSDF; roulette draws as the reference draws
 //     them;
 //   the deposits (AddPhoton: EvalAll at each visible point of the photon's
-//     entry within its radius) of all depths at once: the records sorted by
+//     entry within its radius) of all depths of an iteration at once: the records sorted by
 //     hash entry and joined entry by entry with the grid's visible points
 //     (k_deposit);
 //   the radius reduction and UpdatePixel (sppm.cpp:145-169).
@@ -35,7 +36,8 @@ namespace {
 constexpr uint32_t kEntries = 40960;   // VisiblePointSearcher(..., 40960)
 constexpr int kMaxCellsPerAxis = 4;    // a radius box spans <= 3 cells
 constexpr int kThreads = 128;
-constexpr uint64_t kDepositRecords = 1ull << 25;  // of a chunk: 48 + 4 bytes each
+constexpr uint64_t kDepositRecords = 1ull << 25;  // of a wave: 48 + 4 bytes each
+constexpr uint64_t kWavePhotons = 1ull << 21;  // waves of several iterations
 constexpr unsigned kFull = 0xffffffffu;
 
 int fail(ajg_ctx* ctx, int code, const std::string& m) {
@@ -56,7 +58,8 @@ struct SppmArgs {
   float init_radius;
   uint64_t pseed;     // photon stream seed
   uint32_t npix;
-  uint32_t it;        // iteration
+  // a photon wave: photons [i0, i0 + m) of each iteration from it0 on
+  uint32_t it0, i0, m;
   int pmin, pmax;
   float cont;
   // DefaultScene's light selector (default_scene.cpp:48-53, 77-86)
@@ -141,13 +144,15 @@ __global__ void k_grid_count(SppmArgs a, SppmPixels px, Grid g,
   }
 }
 
-// A photon's deposit, three float4: position and power, incoming direction,
-// hash entry and rank among the entry's deposits.  `hist` counts an entry's
-// deposits, `offsets` and `units` are their exclusive scans (k_entry_scan),
-// `sorted` the records' indices entry by entry.
+// The deposits of one iteration's photons of a wave.  A record is three
+// float4: position and power, incoming direction, and -- filled in once the
+// iteration's grid stands (k_deposit_enter) -- hash entry and rank among the
+// entry's deposits.  `hist` counts an entry's deposits, `offsets` and `units`
+// are their exclusive scans (k_entry_scan), `sorted` the records' indices
+// entry by entry.
 struct Deposits {
-  float4* rec;                // [cap][3]
-  uint32_t* count;
+  float4* rec;                // [cap][3]; a wave's iterations one after the other
+  uint32_t* count;            // one per iteration of the wave
   uint32_t* hist;             // [kEntries]
   uint32_t* offsets;          // [kEntries + 1]
   unsigned long long* units;  // [kEntries + 1]
@@ -390,19 +395,24 @@ __device__ Emission sample_emit(const SppmArgs& a, const float* L,
   return e;
 }
 
+// Photon i of iteration k draws from path_key(photon_seed(seed), i, k).
+__device__ __forceinline__ uint64_t photon_key(const SppmArgs& a, uint32_t pid) {
+  return path_key(a.pseed, a.i0 + pid % a.m, a.it0 + pid / a.m);
+}
+
 // TracerPhoton's start (sppm.cpp:105-121) and depth 1's roulette.
 __global__ void __launch_bounds__(kThreads)
-    k_photon_emit(SppmArgs a, PhotonQ q, uint32_t i0, uint32_t n,
-                  uint32_t* err) {
+    k_photon_emit(SppmArgs a, PhotonQ q, uint32_t n, uint32_t* err) {
   const uint32_t lane = threadIdx.x & 31;
   for (uint32_t wb = blockIdx.x * blockDim.x + (threadIdx.x - lane); wb < n;
        wb += gridDim.x * blockDim.x) {
     const uint32_t t = wb + lane;
     bool live = false;
     F3 o = mk3(0, 0, 0), d = mk3(0, 0, 1), coef = mk3(0, 0, 0);
-    uint32_t pid = i0 + t, dim = 0;
+    const uint32_t pid = t;  // the photon's number in the wave
+    uint32_t dim = 0;
     if (t < n && a.nl > 0) {
-      const uint64_t key = path_key(a.pseed, pid, a.it);
+      const uint64_t key = photon_key(a, pid);
       const float u = key_float(key, dim++);
       // upper_bound with <=: the first j with u <= cdf[j]
       uint32_t j = 0;
@@ -452,32 +462,47 @@ __global__ void __launch_bounds__(128, trace_min_blocks<W>())
   flush_counters(ctr, nr, nn, nt);
 }
 
-// Records a photon's deposit at `pos` (VisiblePointSearcher::AddPhoton,
-// photon_mapping.h:101-120) for k_deposit, unless no visible point is filed
-// under its entry.
-__device__ __forceinline__ void record_deposit(const SppmArgs& a, const Grid& g,
-                                               const Deposits& dp, bool pred,
-                                               F3 pos, F3 phi, F3 wr,
+// Records a photon's deposit for k_deposit, among those of its iteration
+// (`seg` of the wave).  Every lane of the warp calls it.
+__device__ __forceinline__ void record_deposit(const Deposits& dp, uint32_t seg,
+                                               bool pred, F3 pos, F3 phi, F3 wr,
                                                uint32_t* err) {
-  uint32_t e = 0;
-  if (pred) {
-    const float side = 1.05f * *g.maxr;
-    int c[3];
-    to_grid(pos, a.lo, side, c);
-    e = to_entry(c[0], c[1], c[2]);
-    pred = g.offsets[e] < min(g.offsets[e + 1], g.cap);
-  }
-  const uint32_t k = warp_append(dp.count, pred);
+  const int lane = threadIdx.x & 31;
+  const unsigned peers = __match_any_sync(kFull, pred ? seg : 0xffffffffu);
+  const int leader = __ffs(peers) - 1;
+  uint32_t k = 0;
+  if (pred && lane == leader) k = atomicAdd(&dp.count[seg], (uint32_t)__popc(peers));
+  k = __shfl_sync(kFull, k, leader) + __popc(peers & ((1u << lane) - 1u));
   if (!pred) return;
   if (k >= dp.cap) {
     raise_device_error(err, kDevQueueOverflow);
     return;
   }
-  const uint32_t rank = atomicAdd(&dp.hist[e], 1u);
-  float4* r = dp.rec + 3 * (uint64_t)k;
+  float4* r = dp.rec + 3 * ((uint64_t)seg * dp.cap + k);
   r[0] = make_float4(pos.x, pos.y, pos.z, phi.x);
   r[1] = make_float4(phi.y, phi.z, wr.x, wr.y);
-  r[2] = make_float4(wr.z, __uint_as_float(e), __uint_as_float(rank), 0.f);
+  r[2] = make_float4(wr.z, 0.f, 0.f, 0.f);
+}
+
+// The entry a deposit falls into (VisiblePointSearcher::AddPhoton,
+// photon_mapping.h:101-120) and its rank there; entries without visible
+// points drop theirs (kEntries).
+__global__ void k_deposit_enter(SppmArgs a, Grid g, Deposits dp) {
+  const uint32_t n = min(*dp.count, dp.cap);
+  const float side = 1.05f * *g.maxr;
+  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n;
+       k += gridDim.x * blockDim.x) {
+    float4* r = dp.rec + 3 * (uint64_t)k;
+    int c[3];
+    to_grid(xyz(r[0]), a.lo, side, c);
+    uint32_t e = to_entry(c[0], c[1], c[2]), rank = 0;
+    if (g.offsets[e] < min(g.offsets[e + 1], g.cap))
+      rank = atomicAdd(&dp.hist[e], 1u);
+    else
+      e = kEntries;
+    reinterpret_cast<uint32_t*>(r + 2)[1] = e;
+    reinterpret_cast<uint32_t*>(r + 2)[2] = rank;
+  }
 }
 
 __global__ void k_deposit_sort(Deposits dp) {
@@ -485,7 +510,8 @@ __global__ void k_deposit_sort(Deposits dp) {
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n;
        k += gridDim.x * blockDim.x) {
     const float4 r = dp.rec[3 * (uint64_t)k + 2];
-    dp.sorted[dp.offsets[__float_as_uint(r.y)] + __float_as_uint(r.z)] = k;
+    const uint32_t e = __float_as_uint(r.y);
+    if (e < kEntries) dp.sorted[dp.offsets[e] + __float_as_uint(r.z)] = k;
   }
 }
 
@@ -606,7 +632,7 @@ __global__ void __launch_bounds__(kThreads, 8)
 // One depth of TracerPhoton (sppm.cpp:122-142) over the queue: the deposit
 // (from depth 2 on), the BSDF sample, and the next depth's roulette.
 __global__ void __launch_bounds__(kThreads)
-    k_photon_shade(SppmArgs a, Grid g, PhotonQ q, Deposits dp, int depth,
+    k_photon_shade(SppmArgs a, PhotonQ q, Deposits dp, int depth,
                    uint32_t* err) {
   const int cur = depth & 1;
   const uint32_t n = min(q.counts[2 * depth], q.cap);
@@ -625,7 +651,7 @@ __global__ void __launch_bounds__(kThreads)
       dim = __float_as_uint(d4.w);
       coef = xyz(q.coef[cur][k]);
       if (h.prim >= 0) {
-        const uint64_t key = path_key(a.pseed, pid, a.it);
+        const uint64_t key = photon_key(a, pid);
         const HitInfo hi =
             complete_hit(a.s, xyz(o4), xyz(d4), h.t, h.u, h.v, h.prim);
         hit = true;
@@ -651,7 +677,7 @@ __global__ void __launch_bounds__(kThreads)
         }
       }
     }
-    if (depth > 1) record_deposit(a, g, dp, hit, pos, power, wr, err);
+    if (depth > 1) record_deposit(dp, pid / a.m, hit, pos, power, wr, err);
     push_photon(q, depth + 1, no, nd, coef, pid, dim, live, err);
   }
 }
@@ -782,19 +808,33 @@ int sppm_render(ajg_scene* sc, const ajg_camera& cam, const ajg_sppm_params& p,
     a.lpdf = table[0];
   }
 
-  // the photon queue, in equal chunks of at most the context's wave size
-  // whose deposits (one per depth from 2 on) fit the record buffer
+  // A photon wave holds an iteration's photons, in equal chunks of at most the
+  // context's wave size whose deposits (one per depth from 2 on) fit the record
+  // buffer -- or, as photons do not depend on the iterations before, those of
+  // several iterations, so that a wave of small ones still fills the GPU (12
+  // iterations x 100,000 photons of the emitter box, radius 0.1: 240 launches
+  // of rays and shading, 4.7 ms, became 20, 1.5 ms; 10.9 -> 7.5 ms a render).
   const uint64_t dep_depths = p.photon_max_depth > 1 ? p.photon_max_depth - 1 : 0;
+  uint64_t most = ctx->wave_paths;
+  if (dep_depths) most = std::min<uint64_t>(most, kDepositRecords / dep_depths);
   uint64_t chunk = std::max<uint64_t>(
-      1, std::min<uint64_t>(p.photons_per_iteration, ctx->wave_paths));
-  if (dep_depths)
-    chunk = std::min<uint64_t>(chunk, kDepositRecords / dep_depths);
+      1, std::min<uint64_t>(p.photons_per_iteration, most));
   const uint64_t n_chunks = (p.photons_per_iteration + chunk - 1) / chunk;
   if (n_chunks) chunk = (p.photons_per_iteration + n_chunks - 1) / n_chunks;
-  const uint64_t dep_cap = chunk * dep_depths;
-  // zeroed per chunk: the depths' queue counters, the deposit count, the
-  // entries' deposit counts
-  const uint64_t n_counts = 2 * ((uint64_t)p.photon_max_depth + 2);
+  uint64_t group = 1;  // iterations of a wave
+  if (n_chunks == 1) {
+    group = std::min<uint64_t>(std::min<uint64_t>(most, kWavePhotons) / chunk,
+                               p.iterations);
+    group = std::max<uint64_t>(group, 1);
+    const uint64_t waves = (p.iterations + group - 1) / group;
+    group = (p.iterations + waves - 1) / waves;
+  }
+  const uint64_t wave = chunk * group;  // photons
+  const uint64_t dep_cap = chunk * dep_depths;  // deposits of an iteration
+  // zeroed per wave: the depths' queue counters and the iterations' deposit
+  // counts
+  const uint64_t n_depths = 2 * ((uint64_t)p.photon_max_depth + 2);
+  const uint64_t n_counts = n_depths + group;
   const uint32_t cap = (uint32_t)std::min<uint64_t>(8 * npix, 0xffffffffull);
 
   // the camera pass's wave arena first, then everything else
@@ -805,7 +845,7 @@ int sppm_render(ajg_scene* sc, const ajg_camera& cam, const ajg_sppm_params& p,
   float4* d_out = nullptr;
   float* d_rad = nullptr;
   float *radius, *N, *maxr;
-  uint32_t *M, *counts, *offsets, *cursor, *items, *bits, *qcounts, *doff, *dsorted;
+  uint32_t *M, *counts, *offsets, *cursor, *items, *bits, *qcounts, *dhist, *doff, *dsorted;
   unsigned long long* dunits;
   ajg_hit* qhits;
   EntryVal* totals;
@@ -825,12 +865,13 @@ int sppm_render(ajg_scene* sc, const ajg_camera& cam, const ajg_sppm_params& p,
     items = carve<uint32_t>(cur, cap);
     spheres = carve<float4>(cur, cap);
     bits = carve<uint32_t>(cur, 1);
-    qro = carve<float4>(cur, 2 * chunk);
-    qrd = carve<float4>(cur, 2 * chunk);
-    qcoef = carve<float4>(cur, 2 * chunk);
-    qhits = carve<ajg_hit>(cur, chunk);
-    qcounts = carve<uint32_t>(cur, n_counts + 1 + kEntries);
-    drec = carve<float4>(cur, 3 * dep_cap);
+    qro = carve<float4>(cur, 2 * wave);
+    qrd = carve<float4>(cur, 2 * wave);
+    qcoef = carve<float4>(cur, 2 * wave);
+    qhits = carve<ajg_hit>(cur, wave);
+    qcounts = carve<uint32_t>(cur, n_counts);
+    dhist = carve<uint32_t>(cur, kEntries);
+    drec = carve<float4>(cur, 3 * dep_cap * group);
     doff = carve<uint32_t>(cur, kEntries + 1);
     dunits = carve<unsigned long long>(cur, kEntries + 1);
     dsorted = carve<uint32_t>(cur, dep_cap);
@@ -860,58 +901,69 @@ int sppm_render(ajg_scene* sc, const ajg_camera& cam, const ajg_sppm_params& p,
   const Grid g{counts, offsets, cursor, items, spheres, cap, maxr};
   PhotonQ q{};
   q.ro[0] = qro;
-  q.ro[1] = qro + chunk;
+  q.ro[1] = qro + wave;
   q.rd[0] = qrd;
-  q.rd[1] = qrd + chunk;
+  q.rd[1] = qrd + wave;
   q.coef[0] = qcoef;
-  q.coef[1] = qcoef + chunk;
+  q.coef[1] = qcoef + wave;
   q.hits = qhits;
   q.counts = qcounts;
-  q.cap = (uint32_t)chunk;
+  q.cap = (uint32_t)wave;
   Deposits dp{};
   dp.rec = drec;
-  dp.count = qcounts + n_counts;
-  dp.hist = dp.count + 1;
+  dp.count = qcounts + n_depths;
+  dp.hist = dhist;
   dp.offsets = doff;
   dp.units = dunits;
   dp.sorted = dsorted;
   dp.cap = (uint32_t)dep_cap;
   const int gd = resident_grid((const void*)k_deposit, kThreads);
+  // Traces photons [i0, i0 + m) of `iters` iterations from it0 on.
+  auto trace = [&](uint32_t it0, uint32_t iters, uint64_t i0) {
+    a.it0 = it0;
+    a.i0 = (uint32_t)i0;
+    a.m = (uint32_t)std::min<uint64_t>(chunk, p.photons_per_iteration - i0);
+    const uint32_t n = a.m * iters;
+    cudaMemsetAsync(q.counts, 0, n_counts * sizeof(uint32_t), st);
+    k_photon_emit<<<grid_for(n, kThreads, gs), kThreads, 0, st>>>(a, q, n,
+                                                                  ctx->d_error);
+    for (int depth = 1; depth <= p.photon_max_depth; ++depth) {
+      const int cur = depth & 1;
+      // photon rays keep the wide tree: over the binary layout the
+      // photon pass measured 8% slower (long rays from the lights)
+      dispatch_trace(s.tri_test, s.width, [&](auto T, auto Wd) {
+        constexpr int TT = decltype(T)::value, WW = decltype(Wd)::value;
+        const int gr = resident_grid((const void*)k_photon_extend<TT, WW>, 128);
+        k_photon_extend<TT, WW><<<gr, 128, 0, st>>>(
+            s, q.ro[cur], q.rd[cur], &q.counts[2 * depth],
+            &q.counts[2 * depth + 1], q.hits, &ctx->d_counters[0], ctx->d_error);
+      });
+      k_photon_shade<<<grid_for(n, kThreads, gs), kThreads, 0, st>>>(
+          a, q, dp, depth, ctx->d_error);
+    }
+    ctx->paths_total += n;
+  };
   for (uint32_t it = 0; it < p.iterations; ++it) {
-    a.it = it;
     cudaMemsetAsync(counts, 0, kEntries * sizeof(uint32_t), st);
     k_grid_count<<<grid_for(npix, 256, gs), 256, 0, st>>>(a, px, g, ctx->d_error);
     k_entry_totals<false><<<kEntryBlocks, kEntryThreads, 0, st>>>(g, dp, totals);
     k_entry_scan<false><<<kEntryBlocks, kEntryThreads, 0, st>>>(g, dp, totals);
     k_grid_fill<<<grid_for(npix, 256, gs), 256, 0, st>>>(a, px, g, ctx->d_error);
+    const uint32_t j = it % (uint32_t)group;  // of its wave
     for (uint64_t i0 = 0; i0 < p.photons_per_iteration; i0 += chunk) {
-      const uint32_t n =
-          (uint32_t)std::min<uint64_t>(chunk, p.photons_per_iteration - i0);
-      cudaMemsetAsync(q.counts, 0, (n_counts + 1 + kEntries) * sizeof(uint32_t), st);
-      k_photon_emit<<<grid_for(n, kThreads, gs), kThreads, 0, st>>>(
-          a, q, (uint32_t)i0, n, ctx->d_error);
-      for (int depth = 1; depth <= p.photon_max_depth; ++depth) {
-        const int cur = depth & 1;
-        // photon rays keep the wide tree: over the binary layout the
-        // photon pass measured 8% slower (long rays from the lights)
-        dispatch_trace(s.tri_test, s.width, [&](auto T, auto Wd) {
-          constexpr int TT = decltype(T)::value, WW = decltype(Wd)::value;
-          const int gr = resident_grid((const void*)k_photon_extend<TT, WW>, 128);
-          k_photon_extend<TT, WW><<<gr, 128, 0, st>>>(
-              s, q.ro[cur], q.rd[cur], &q.counts[2 * depth],
-              &q.counts[2 * depth + 1], q.hits, &ctx->d_counters[0],
-              ctx->d_error);
-        });
-        k_photon_shade<<<grid_for(n, kThreads, gs), kThreads, 0, st>>>(
-            a, g, q, dp, depth, ctx->d_error);
-      }
-      if (dep_depths) {
-        k_entry_totals<true><<<kEntryBlocks, kEntryThreads, 0, st>>>(g, dp, totals);
-        k_entry_scan<true><<<kEntryBlocks, kEntryThreads, 0, st>>>(g, dp, totals);
-        k_deposit_sort<<<grid_for(dep_cap, 256, gs), 256, 0, st>>>(dp);
-        k_deposit<<<gd, kThreads, 0, st>>>(a, px, g, dp);
-      }
-      ctx->paths_total += n;
+      if (j == 0)
+        trace(it, std::min<uint32_t>((uint32_t)group, p.iterations - it), i0);
+      if (!dep_depths) continue;
+      Deposits own = dp;
+      own.rec += 3 * dep_cap * j;
+      own.count += j;
+      const int gr = grid_for(dep_cap, 256, gs);
+      cudaMemsetAsync(dp.hist, 0, kEntries * sizeof(uint32_t), st);
+      k_deposit_enter<<<gr, 256, 0, st>>>(a, g, own);
+      k_entry_totals<true><<<kEntryBlocks, kEntryThreads, 0, st>>>(g, own, totals);
+      k_entry_scan<true><<<kEntryBlocks, kEntryThreads, 0, st>>>(g, own, totals);
+      k_deposit_sort<<<gr, 256, 0, st>>>(own);
+      k_deposit<<<gd, kThreads, 0, st>>>(a, px, g, own);
     }
     cudaMemsetAsync(bits, 0, sizeof(uint32_t), st);
     k_max_radius<<<grid_for(npix, 256, gs), 256, 0, st>>>(a, px, bits);

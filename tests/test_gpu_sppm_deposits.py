@@ -50,3 +50,16 @@ def test_chunks_sum_to_the_same_estimate():
     _, a = radiance(args)
     _, b = radiance(args, wave_paths=1024)
     np.testing.assert_allclose(b, a, rtol=1e-4, atol=1e-6, equal_nan=True)
+
+
+def test_waves_of_iterations_sum_to_the_same_estimate():
+    """70 iterations of 31,000 photons (several waves of many iterations, the
+    last one short) and the same in a context whose waves hold one iteration
+    or a part of it."""
+    args = api.SPPMRendererArgs(forward_max_depth=4, init_radius=0.05, iteration_count=70,
+                                photons_per_iteration=31_000, photon_max_depth=5)
+    _, a = radiance(args)
+    _, b = radiance(args, wave_paths=40_960)
+    _, c = radiance(args, wave_paths=16_384)
+    np.testing.assert_allclose(b, a, rtol=1e-4, atol=1e-6, equal_nan=True)
+    np.testing.assert_allclose(c, a, rtol=1e-4, atol=1e-6, equal_nan=True)
