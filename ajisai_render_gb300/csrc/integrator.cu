@@ -61,8 +61,7 @@ __device__ __forceinline__ uint32_t shade_append(uint32_t* counter,
 #endif
 #ifndef AJG_MJ_SHADE_GRID
 #define AJG_MJ_SHADE_GRID 64  // multi-job shading grid: blocks per SM (8 for
-                              // the rare other materials, whose launch is
-                              // mostly empty).  16 batched jobs: Lambertian
+                              // the rarer other materials).  16 batched jobs: Lambertian
                               // 8.15 -> 7.84 ms, Disney 7.20 -> 6.80 against 8
 #endif
 #ifndef AJG_SHADE_MIN_BLOCKS_DIFFUSE
@@ -232,8 +231,8 @@ __device__ __forceinline__ uint8_t term_unseen(F3 T) {
 // In place of its path in a queue slot whose ray missed (set by k_classify).
 constexpr uint32_t kMissed = 0x80000000u;
 
-// Files every queue slot under its hit's shading class (Lambertian, Disney, or
-// one of the other material types), so that shading runs in class-specialised
+// Files every queue slot under its hit's shading class (delta types,
+// Lambertian, Disney, the others), so that shading runs in class-specialised
 // kernels, and ends the escaped paths: the environment counts only for camera
 // rays (pt.cpp:114-121), or on every bounce without MIS (pt.cpp:245-249).
 // (Beside the accumulation of the bounce before: no path of it is touched by
@@ -262,7 +261,9 @@ __global__ void __launch_bounds__(kClassifyThreads)
         const uint32_t mat =
             __float_as_uint(__ldg(&shade[prim].w)) & 0xffffffu;
         const int type = (int)__ldg(materials + 16 * mat);
-        cls = type == AJG_MAT_DIFFUSE ? 0 : (type == AJG_MAT_DISNEY ? 1 : 2);
+        cls = type == AJG_MAT_DIFFUSE  ? 1
+              : type == AJG_MAT_DISNEY ? 2
+                                       : ((kDeltaTypes >> type) & 1u ? 0 : 3);
       } else {
         if (MJ || ((b == 0 || !a.j.use_mis) && a.s.env >= 0)) {
           const uint32_t p = w.qpath[cur][k];
@@ -280,13 +281,13 @@ __global__ void __launch_bounds__(kClassifyThreads)
       }
     }
 #if AJG_BLOCK_APPEND
-    const uint32_t j = block_append<3, kClassifyThreads / 32>(&w.counts[5], cls);
-    if (cls >= 0) w.lists[(uint64_t)(cls + 1) * list_cap + j] = k;
+    const uint32_t j = block_append<4, kClassifyThreads / 32>(&w.counts[4], cls);
+    if (cls >= 0) w.lists[(uint64_t)cls * list_cap + j] = k;
 #else
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const uint32_t j = warp_append(&w.counts[5 + c], cls == c);
-      if (cls == c) w.lists[(uint64_t)(c + 1) * list_cap + j] = k;
+    for (int c = 0; c < 4; ++c) {
+      const uint32_t j = warp_append(&w.counts[4 + c], cls == c);
+      if (cls == c) w.lists[(uint64_t)c * list_cap + j] = k;
     }
 #endif
   }
@@ -535,6 +536,15 @@ __global__ void __launch_bounds__(kShadeThreads, shade_min_blocks<MAT>())
     enum Kind { kLight, kMisBsdf, kContinue };
     auto round = [&](Kind kind, int t_) __attribute__((always_inline)) {
       const bool is_light = kind == kLight, is_mis = kind == kMisBsdf;
+      if constexpr (MAT == kMatDelta) {
+        if (is_light) {  // f is 0: the light's draws are passed over
+          if (MJ ? (mis && t_ < nl) : hit) {
+            w.term_vis[p * NT + t_] = term_unseen(T);
+            dim += (int)s.lights[12 * t_] == kLightArea ? 3 : 2;
+          }
+          return;
+        }
+      }
       bool on, lit = false;  // lit: `wl` is a direction to evaluate
       F3 wl = mk3(0, 0, 1), lrad = mk3(0, 0, 0);
       float lpdf = 0.f, len = 0.f;
@@ -1343,11 +1353,17 @@ static void run_waves(ajg_scene* sc, const ajg_camera& cam,
               a, t, wb, b, q, w.lists + 2 * P, &wb.counts[6], (uint32_t)nt,
               shadow_cap, ctx->d_error, coh);
         }
-        if (s.mat_mask >> AJG_MAT_MIRROR) {
+        if (s.mat_mask & kOtherTypes) {
           KernelTimer tm(ctx, st, ks);
           k_shade<kMatOther, false><<<gsh, kShadeThreads, 0, st>>>(
               a, t, wb, b, q, w.lists + 3 * P, &wb.counts[7], (uint32_t)nt,
               shadow_cap, ctx->d_error, coh);
+        }
+        if (s.mat_mask & kDeltaTypes) {
+          KernelTimer tm(ctx, st, ks);
+          k_shade<kMatDelta, false><<<gsh, kShadeThreads, 0, st>>>(
+              a, t, wb, b, q, w.lists, &wb.counts[4], (uint32_t)nt, shadow_cap,
+              ctx->d_error, coh);
         }
         if (overlap && b + 1 < a.j.max_b)
           extend_ahead(b + 1, q ^ 1, false);
@@ -1402,7 +1418,7 @@ static void run_waves(ajg_scene* sc, const ajg_camera& cam,
 
 void enqueue_mj_wave(const MJTables& t, const WaveBufs& w, uint64_t P,
                      int NT, int bounces, int tri_test, int width, bool emit,
-                     TraceCounters* ctr, uint32_t* err, cudaStream_t st,
+                     uint32_t mat_mask, TraceCounters* ctr, uint32_t* err, cudaStream_t st,
                      cudaStream_t ts, cudaEvent_t ev_queue,
                      cudaEvent_t ev_hits, bool cam_packets,
                      bool shadow_packets) {
@@ -1466,9 +1482,14 @@ void enqueue_mj_wave(const MJTables& t, const WaveBufs& w, uint64_t P,
     k_shade<AJG_MAT_DISNEY, true><<<gsh, kShadeThreads, 0, st>>>(
         a, t, wb, b, q, w.lists + 2 * P, &wb.counts[6], (uint32_t)NT,
         shadow_cap, err, coh);
-    k_shade<kMatOther, true><<<gso, kShadeThreads, 0, st>>>(
-        a, t, wb, b, q, w.lists + 3 * P, &wb.counts[7], (uint32_t)NT,
-        shadow_cap, err, coh);
+    if (mat_mask & kOtherTypes)
+      k_shade<kMatOther, true><<<gso, kShadeThreads, 0, st>>>(
+          a, t, wb, b, q, w.lists + 3 * P, &wb.counts[7], (uint32_t)NT,
+          shadow_cap, err, coh);
+    if (mat_mask & kDeltaTypes)
+      k_shade<kMatDelta, true><<<gso, kShadeThreads, 0, st>>>(
+          a, t, wb, b, q, w.lists, &wb.counts[4], (uint32_t)NT, shadow_cap, err,
+          coh);
     if (overlap && b + 1 < bounces)
       extend_ahead(b + 1, q ^ 1, false);
     launch_wave_shadow(true, tri_test, width, s, t, w.sq_o, w.sq_d, w.sq_scene,

@@ -97,6 +97,13 @@ inline DeviceScene closest_view(const DeviceScene& s) {
 //   [10] first corner in emit_pts (uint bits)
 constexpr int kLightArea = 2;
 
+// Shading classes of the types >= AJG_MAT_MIRROR: metal and plastic, and the
+// delta types (mirror, glass, null), which no light sample can see.
+constexpr int kMatOther = 7, kMatDelta = 8;
+constexpr uint32_t kOtherTypes = (1u << AJG_MAT_METAL) | (1u << AJG_MAT_PLASTIC);
+constexpr uint32_t kDeltaTypes =
+    (1u << AJG_MAT_MIRROR) | (1u << AJG_MAT_GLASS) | (1u << AJG_MAT_NULL);
+
 // Per-job constants of the integrator, shared by the single-job and the
 // multi-job waves.  The film of a job covers the window (x0, y0, win_w,
 // win_h) of a film_w x film_h image; the sampler keys by the image pixel
@@ -178,12 +185,12 @@ struct WaveBufs {
   float4* sq_o;  // shadow queue: o.xyz, t_max
   float4* sq_d;  // d.xyz, slot bits
   uint16_t* sq_scene;  // multi-job waves: scene index per shadow ray
-  uint32_t* lists;   // [4][P]: queue slots of Lambertian (1), Disney (2) and
-                     // other (3) hits; the MIS BSDF hits of emitter scenes
-                     // borrow it
+  uint32_t* lists;   // [4][P]: queue slots of delta (0), Lambertian (1),
+                     // Disney (2) and other (3) hits; the MIS BSDF hits of
+                     // emitter scenes borrow it
   uint32_t* counts;  // kCounterWords words per bounce, zeroed once a wave (a
                      // launch's copy points at its bounce's): [0] the path
-                     // queue, [2] shadow queue, [3] shadow fetch, [5..7]
+                     // queue, [2] shadow queue, [3] shadow fetch, [4..7]
                      // lists, [8] extend fetch, [9] closest MIS BSDF queue,
                      // [10] its fetch, [11] coherent shadow queue (waves
                      // without emitters), [12] its fetch
@@ -461,21 +468,23 @@ WaveBufs carve_wave(char* base, uint64_t P, int nt, bool mj);
 // Enqueues one multi-job wave on `st` (capturable: fixed arguments, queue
 // lengths and table contents read on the device): raygen, `bounces` bounce
 // iterations, film update.  NT = light terms per path of the arena; `emit`:
-// a scene of the wave has emitters (the closest-hit MIS BSDF pass runs).
+// a scene of the wave has emitters (the closest-hit MIS BSDF pass runs);
+// `mat_mask`: bit t set where a scene has materials of type t (the classes of
+// the types from AJG_MAT_MIRROR on are shaded only where present).
 // With a trace stream and two events, bounce b+1's closest hits run there
 // beside bounce b's shadow rays (null: one stream).
 void enqueue_mj_wave(const MJTables& t, const WaveBufs& w, uint64_t P,
                      int NT, int bounces, int tri_test, int width, bool emit,
-                     TraceCounters* ctr, uint32_t* err, cudaStream_t st,
+                     uint32_t mat_mask, TraceCounters* ctr, uint32_t* err, cudaStream_t st,
                      cudaStream_t ts = nullptr, cudaEvent_t ev_queue = nullptr,
                      cudaEvent_t ev_hits = nullptr, bool cam_packets = false,
                      bool shadow_packets = false);
 // Kernels of a multi-job wave launched per wave (for launch counts):
 // `shadow_packets` adds bounce 0's packet traversal of its directional-light
 // rays (waves without emitters over plain 4-wide trees).
-inline int mj_wave_kernels(int bounces, bool emit, int width = 0,
-                           bool shadow_packets = false) {
-  return 2 + (emit ? 9 : 7) * bounces +
+inline int mj_wave_kernels(int bounces, bool emit, int width,
+                           bool shadow_packets, int other_classes) {
+  return 2 + ((emit ? 8 : 6) + other_classes) * bounces +
          (shadow_packets && !emit && width == 4 && bounces > 0 ? 1 : 0);
 }
 // Looks up the persistent grids of the multi-job kernels (call before a

@@ -155,7 +155,7 @@ struct Server {
   std::vector<char*> h_tables;  // pinned, one per in-flight slot + 1
   size_t table_bytes = 0;
   uint64_t wave_no = 0;
-  std::map<std::tuple<int, int, int, bool, bool>, cudaGraphExec_t> graphs;
+  std::map<std::tuple<int, int, int, bool, bool, uint32_t>, cudaGraphExec_t> graphs;
   std::deque<InFlight> inflight;
   std::vector<uint32_t*> err_words;  // pinned, recycled
   uint32_t* d_err = nullptr;
@@ -171,7 +171,7 @@ struct Server {
   void end_job_locked(Job* j, uint32_t state, int err);
   int ensure_arena(int nt, uint64_t target_paths);
   cudaGraphExec_t graph_for(int bounces, int tri_test, int width, bool emit,
-                            bool packets);
+                            bool packets, uint32_t mat_mask);
 };
 
 namespace {
@@ -221,8 +221,10 @@ int Server::ensure_arena(int nt, uint64_t target) {
 }
 
 cudaGraphExec_t Server::graph_for(int bounces, int tri_test, int width,
-                                  bool emit, bool packets) {
-  const auto key = std::make_tuple(bounces, tri_test, width, emit, packets);
+                                  bool emit, bool packets,
+                                  uint32_t mat_mask) {
+  const auto key =
+      std::make_tuple(bounces, tri_test, width, emit, packets, mat_mask);
   auto it = graphs.find(key);
   if (it != graphs.end()) return it->second;
   prepare_mj_kernels();
@@ -231,8 +233,8 @@ cudaGraphExec_t Server::graph_for(int bounces, int tri_test, int width,
   if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) !=
       cudaSuccess)
     return nullptr;
-  enqueue_mj_wave(t, w, P, NT, bounces, tri_test, width, emit, d_ctr, d_err,
-                  st, ctx->overlap ? ts : nullptr, ev_queue, ev_hits,
+  enqueue_mj_wave(t, w, P, NT, bounces, tri_test, width, emit, mat_mask, d_ctr,
+                  d_err, st, ctx->overlap ? ts : nullptr, ev_queue, ev_hits,
                   ctx->packet_camera, packets);
   if (cudaStreamEndCapture(st, &g) != cudaSuccess || !g) return nullptr;
   if (cudaGraphInstantiate(&ex, g, 0) != cudaSuccess) ex = nullptr;
@@ -538,14 +540,21 @@ bool Server::plan_and_launch() {
   cudaEventRecord(f.ev0, st);
   // the closest-hit MIS BSDF pass runs when a scene of the wave has emitters
   bool emit = false;
-  for (const Plan& p : plan) emit |= p.job->scene->d.tri_emit != nullptr;
-  cudaGraphExec_t g = graph_for(bounces, tri_test, width, emit, packets);
+  // and the rarer materials' shading classes when a scene has some
+  uint32_t types = 0;
+  for (const Plan& p : plan) {
+    emit |= p.job->scene->d.tri_emit != nullptr;
+    types |= p.job->scene->d.mat_mask;
+  }
+  const bool other = (types & kOtherTypes) != 0, delta = (types & kDeltaTypes) != 0;
+  const uint32_t mat_mask = (other ? kOtherTypes : 0u) | (delta ? kDeltaTypes : 0u);
+  cudaGraphExec_t g = graph_for(bounces, tri_test, width, emit, packets, mat_mask);
   if (g) {
     cudaGraphLaunch(g, st);
   } else {  // capture unavailable: the same launches on the stream
     cudaGetLastError();
-    enqueue_mj_wave(t, w, P, NT, bounces, tri_test, width, emit, d_ctr, d_err,
-                    st, ctx->overlap ? ts : nullptr, ev_queue, ev_hits,
+    enqueue_mj_wave(t, w, P, NT, bounces, tri_test, width, emit, mat_mask, d_ctr,
+                    d_err, st, ctx->overlap ? ts : nullptr, ev_queue, ev_hits,
                     ctx->packet_camera, packets);
   }
   // results this wave completes
@@ -594,7 +603,7 @@ bool Server::plan_and_launch() {
     ++stats.waves;
     stats.paths += path_off;
     stats.kernel_launches +=
-        mj_wave_kernels(bounces, emit, width, packets) +
+        mj_wave_kernels(bounces, emit, width, packets, (int)other + (int)delta) +
         f.reports.size();
   }
   inflight.push_back(std::move(f));

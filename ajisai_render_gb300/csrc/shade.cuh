@@ -587,7 +587,6 @@ static __device__ __noinline__ void disney_eval_pdf(const float* __restrict__ m,
 // the constructor's terms the host computes once (plastic_bsdf.cpp:32-45):
 // [14] the average transmittance exp(-2 thickness sigma_a), [15] the
 // diffuse Fresnel integral.
-constexpr int kMatOther = 7;  // shading class of the types >= AJG_MAT_MIRROR
 
 // Fresnel::dielectricReflectance (bsdf/helper.h:35-56)
 __device__ __forceinline__ float dielectric_reflectance(float eta,
@@ -954,23 +953,23 @@ struct PlasticB {
 
 // The types >= AJG_MAT_MIRROR (type passed separately: the record's first
 // word is a float in the scene tables and a uint32 in ajg_bsdf_query's).
+__device__ __forceinline__ BsdfSample delta_sample(int type, const float* m, F3 ng,
+                                                   F3 ns, F3 wo, F3 sam) {
+  if (type == AJG_MAT_MIRROR) return mirror_sample(m, ng, ns, wo);
+  if (type == AJG_MAT_GLASS) return glass_sample(m, ng, ns, wo, sam);
+  BsdfSample s;  // NullBsdf (null.cpp:31-52): straight through
+  s.dir = -wo;
+  s.f = mk3(1.f, 1.f, 1.f);
+  s.pdf = 1.f;
+  s.delta = true;
+  return s;
+}
 static __device__ __noinline__ BsdfSample other_sample(int type,
                                                        const float* m, F3 ng,
                                                        F3 ns, F3 wo, F3 sam) {
-  switch (type) {
-    case AJG_MAT_MIRROR: return mirror_sample(m, ng, ns, wo);
-    case AJG_MAT_GLASS: return glass_sample(m, ng, ns, wo, sam);
-    case AJG_MAT_METAL: return metal_sample(m, ng, ns, wo, sam);
-    case AJG_MAT_PLASTIC: return PlasticB(m, ng, ns).sample(wo, sam);
-    default: {  // NullBsdf (null.cpp:31-52): straight through
-      BsdfSample s;
-      s.dir = -wo;
-      s.f = mk3(1.f, 1.f, 1.f);
-      s.pdf = 1.f;
-      s.delta = true;
-      return s;
-    }
-  }
+  if (type == AJG_MAT_METAL) return metal_sample(m, ng, ns, wo, sam);
+  if (type == AJG_MAT_PLASTIC) return PlasticB(m, ng, ns).sample(wo, sam);
+  return delta_sample(type, m, ng, ns, wo, sam);
 }
 static __device__ __noinline__ void other_eval_pdf(int type, const float* m,
                                                    F3 ng, F3 ns, F3 wi, F3 wo,
@@ -1076,6 +1075,8 @@ struct BsdfT {
   __device__ __forceinline__ BsdfSample sample(F3 s) const {
     if constexpr (MAT == AJG_MAT_DIFFUSE)
       return b.sample(s);
+    else if constexpr (MAT == kMatDelta)
+      return delta_sample((int)m[0], m, ng, ns, wo, s);
     else
       return other_sample((int)m[0], m, ng, ns, wo, s);
   }
