@@ -15,7 +15,7 @@ candidates apart), capped at the real render, and compared by time per
 sample.  Block shapes and the shared-memory stack depth are compile-time
 constants of the kernels, chosen offline with tagged builds
 (AJG_BUILD_TAG / AJG_EXTRA_NVCC, e.g. -DAJG_SHADE_THREADS=128 or
--DAJG_SMEM_STACK=8) and loaded through AJG_LIB.
+-DAJG_SMEM_STACK=16) and loaded through AJG_LIB.
 
     from ajisai_render_gb300 import api, autotune
     best = autotune.tune(flat_scene, camera, api.PTRendererArgs(spp=256, ...))

@@ -1002,7 +1002,7 @@ bool device_malloc(ajg_ctx* ctx, void** p, uint64_t bytes) {
   return false;
 }
 
-int resident_grid(const void* fn, int threads) {
+int resident_grid(const void* fn, int threads, int carveout) {
   static std::mutex mu;
   static std::map<std::pair<const void*, int>, int> cache;
   int dev = 0;
@@ -1011,6 +1011,9 @@ int resident_grid(const void* fn, int threads) {
   auto key = std::make_pair(fn, dev);
   auto it = cache.find(key);
   if (it != cache.end()) return it->second;
+  if (carveout >= 0)
+    cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
+                         carveout);
   int sms = kSMs, per_sm = 1;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, 0) !=

@@ -531,8 +531,9 @@ void launch_wave_bsdf_trace(bool mj, int tri_test, int width,
                             float* t_hit, int32_t* prim_hit,
                             TraceCounters* ctr, uint32_t* err, cudaStream_t st);
 // Blocks of `fn` (launched with `threads` threads) resident on the device at
-// once: the grid of a persistent kernel.
-int resident_grid(const void* fn, int threads);
+// once: the grid of a persistent kernel.  The first call for a kernel sets its
+// shared-memory carveout (percent; -1: the driver's choice).
+int resident_grid(const void* fn, int threads, int carveout = -1);
 // SPPM's camera pass (TracerVP, sppm.cpp:35-101) through the path-tracing
 // wave: one path per pixel (sample 0), no roulette, depth `fmd`; fills
 // vp[npix] (kNoVisPoint where none) and the direct light direct[npix].

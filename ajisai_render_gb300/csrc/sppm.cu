@@ -933,7 +933,7 @@ int sppm_render(ajg_scene* sc, const ajg_camera& cam, const ajg_sppm_params& p,
       // photon pass measured 8% slower (long rays from the lights)
       dispatch_trace(s.tri_test, s.width, [&](auto T, auto Wd) {
         constexpr int TT = decltype(T)::value, WW = decltype(Wd)::value;
-        const int gr = resident_grid((const void*)k_photon_extend<TT, WW>, 128);
+        const int gr = trace_grid((const void*)k_photon_extend<TT, WW>, 128);
         k_photon_extend<TT, WW><<<gr, 128, 0, st>>>(
             s, q.ro[cur], q.rd[cur], &q.counts[2 * depth],
             &q.counts[2 * depth + 1], q.hits, &ctx->d_counters[0], ctx->d_error);

@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(kTraceThreads, trace_min_blocks<W>())
 // as give each warp one ray (the traversal spreads a batch evenly over the
 // warps launched).
 static int query_grid(const void* fn, uint64_t n) {
-  return grid_for(n, kTraceThreads / 32, resident_grid(fn, kTraceThreads));
+  return grid_for(n, kTraceThreads / 32, trace_grid(fn, kTraceThreads));
 }
 
 // `next` is a zeroed device word (the persistent lanes' ray counter).

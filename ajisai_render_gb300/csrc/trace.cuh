@@ -22,7 +22,7 @@
 // held until the warp's next leaf pass, in which every lane holding some
 // tests one (the lanes that found leaves in a visit are a few of the 32, and
 // the pass gathers their tests into fewer warp instructions).  Each lane's
-// stack keeps its top 16 entries
+// stack keeps its top 8 entries
 // in a shared-memory ring and the rest in local memory, and is guarded:
 // overflow sets the device error word and ends the ray.  Coherent rays -- a
 // pixel's shadow rays toward a directional light, and on request its camera
@@ -313,9 +313,25 @@ constexpr int trace_min_blocks() {
                                     : AJG_TRACE_MIN_BLOCKS;
 }
 #ifndef AJG_SMEM_STACK
-#define AJG_SMEM_STACK 16  // stack entries per lane in shared memory (a power
-                           // of two; 0: the whole stack in local memory)
+#define AJG_SMEM_STACK 8  // stack entries per lane in shared memory (a power
+                          // of two; 0: the whole stack in local memory)
 #endif
+// The share of an SM's 228 KB, in percent, every traversal kernel asks for as
+// shared memory: 82 KB, rounded up to the 100 KB configuration, the smallest
+// that holds 9 blocks' rings.  An SM changes its configuration only when it is
+// empty, so closest hits run beside any hits on one SM only if both ask for
+// the same; with 16 entries and each kernel's own size (164 and 100 KB) they
+// shared the chip by SMs.  16 entries and no request -> 8 entries and this
+// one: a 64x48x4 box 433 -> 424 us, 1024x1024x32 over 1.3 M triangles 63.3 ->
+// 62.5 ms, the material box 4.59 -> 4.49 ms, 16 batched jobs 50.7 -> 50.3 ms.
+// 64 KB holds too few blocks (+6% over the triangles), larger ones leave less
+// cache (132 KB +0.3%, 196 KB +2%); 4 entries spill too often (+1%); and the
+// shading kernels asking for it too lose their own cache (+1%, the material
+// box +6%).
+constexpr int kTraceCarveout = 36;
+inline int trace_grid(const void* fn, int threads) {
+  return resident_grid(fn, threads, kTraceCarveout);
+}
 #ifndef AJG_ANY_RING
 #define AJG_ANY_RING AJG_SMEM_STACK  // the same for any-hit queries
 #endif

@@ -190,11 +190,11 @@ void launch_wave_extend(bool mj, int tri_test, int width, const DeviceScene& s,
   dispatch_trace(tri_test, width, [&](auto T, auto Wd) {
     constexpr int TT = decltype(T)::value, WW = decltype(Wd)::value;
     if (mj) {
-      const int g = resident_grid((const void*)k_extend<TT, true, WW>, kTraceThreads);
+      const int g = trace_grid((const void*)k_extend<TT, true, WW>, kTraceThreads);
       k_extend<TT, true, WW><<<g, kTraceThreads, 0, st>>>(
           s, t, ro, rd, count, fetch_next, hits, ctr, err);
     } else {
-      const int g = resident_grid((const void*)k_extend<TT, false, WW>, kTraceThreads);
+      const int g = trace_grid((const void*)k_extend<TT, false, WW>, kTraceThreads);
       k_extend<TT, false, WW><<<g, kTraceThreads, 0, st>>>(
           s, t, ro, rd, count, fetch_next, hits, ctr, err);
     }
@@ -210,11 +210,11 @@ void launch_wave_shadow(bool mj, int tri_test, int width, const DeviceScene& s,
   dispatch_trace(tri_test, width, [&](auto T, auto Wd) {
     constexpr int TT = decltype(T)::value, WW = decltype(Wd)::value;
     if (mj) {
-      const int g = resident_grid((const void*)k_shadow<TT, true, WW>, kTraceThreads);
+      const int g = trace_grid((const void*)k_shadow<TT, true, WW>, kTraceThreads);
       k_shadow<TT, true, WW><<<g, kTraceThreads, 0, st>>>(
           s, t, sq_o, sq_d, sq_scene, count, fetch_next, vis, ctr, err);
     } else {
-      const int g = resident_grid((const void*)k_shadow<TT, false, WW>, kTraceThreads);
+      const int g = trace_grid((const void*)k_shadow<TT, false, WW>, kTraceThreads);
       k_shadow<TT, false, WW><<<g, kTraceThreads, 0, st>>>(
           s, t, sq_o, sq_d, sq_scene, count, fetch_next, vis, ctr, err);
     }
@@ -230,7 +230,7 @@ void launch_wave_extend_packet(bool mj, int tri_test, const DeviceScene& s,
   auto go = [&](auto T, auto M) {
     constexpr int TT = decltype(T)::value;
     constexpr bool MM = decltype(M)::value;
-    const int g = resident_grid((const void*)k_extend_packet<TT, MM>, kPacketThreads);
+    const int g = trace_grid((const void*)k_extend_packet<TT, MM>, kPacketThreads);
     k_extend_packet<TT, MM><<<g, kPacketThreads, 0, st>>>(
         s, t, ro, rd, count, fetch_next, hits, ctr, err);
   };
@@ -258,7 +258,7 @@ void launch_wave_shadow_packet(bool mj, int tri_test, const DeviceScene& s,
   auto go = [&](auto T, auto M) {
     constexpr int TT = decltype(T)::value;
     constexpr bool MM = decltype(M)::value;
-    const int g = resident_grid((const void*)k_shadow_packet<TT, MM>, kPacketThreads);
+    const int g = trace_grid((const void*)k_shadow_packet<TT, MM>, kPacketThreads);
     k_shadow_packet<TT, MM><<<g, kPacketThreads, 0, st>>>(
         s, t, sq_o, sq_d, sq_scene, count, fetch_next, cap, vis, ctr, err);
   };
@@ -288,13 +288,13 @@ void launch_wave_bsdf_trace(bool mj, int tri_test, int width,
     constexpr int TT = decltype(T)::value, WW = decltype(Wd)::value;
     if (mj) {
       const int g =
-          resident_grid((const void*)k_bsdf_trace<TT, true, WW>, kTraceThreads);
+          trace_grid((const void*)k_bsdf_trace<TT, true, WW>, kTraceThreads);
       k_bsdf_trace<TT, true, WW><<<g, kTraceThreads, 0, st>>>(
           s, t, sq_o, sq_d, sq_scene, count, fetch_next, cap, n_max, t_hit,
           prim_hit, ctr, err);
     } else {
       const int g =
-          resident_grid((const void*)k_bsdf_trace<TT, false, WW>, kTraceThreads);
+          trace_grid((const void*)k_bsdf_trace<TT, false, WW>, kTraceThreads);
       k_bsdf_trace<TT, false, WW><<<g, kTraceThreads, 0, st>>>(
           s, t, sq_o, sq_d, sq_scene, count, fetch_next, cap, n_max, t_hit,
           prim_hit, ctr, err);
@@ -307,17 +307,17 @@ void prepare_mj_kernels() {
     for (int wd : {2, 4, 8, 4 | (int)kBvhCompressed, 8 | (int)kBvhCompressed})
       dispatch_trace(tt, wd, [&](auto T, auto Wd) {
         constexpr int TT = decltype(T)::value, WW = decltype(Wd)::value;
-        resident_grid((const void*)k_extend<TT, true, WW>, kTraceThreads);
-        resident_grid((const void*)k_shadow<TT, true, WW>, kTraceThreads);
-        resident_grid((const void*)k_bsdf_trace<TT, true, WW>, kTraceThreads);
+        trace_grid((const void*)k_extend<TT, true, WW>, kTraceThreads);
+        trace_grid((const void*)k_shadow<TT, true, WW>, kTraceThreads);
+        trace_grid((const void*)k_bsdf_trace<TT, true, WW>, kTraceThreads);
       });
-  resident_grid((const void*)k_extend_packet<AJG_TRI_MOLLER_TRUMBORE, true>,
+  trace_grid((const void*)k_extend_packet<AJG_TRI_MOLLER_TRUMBORE, true>,
                 kPacketThreads);
-  resident_grid((const void*)k_extend_packet<AJG_TRI_WATERTIGHT, true>,
+  trace_grid((const void*)k_extend_packet<AJG_TRI_WATERTIGHT, true>,
                 kPacketThreads);
-  resident_grid((const void*)k_shadow_packet<AJG_TRI_MOLLER_TRUMBORE, true>,
+  trace_grid((const void*)k_shadow_packet<AJG_TRI_MOLLER_TRUMBORE, true>,
                 kPacketThreads);
-  resident_grid((const void*)k_shadow_packet<AJG_TRI_WATERTIGHT, true>,
+  trace_grid((const void*)k_shadow_packet<AJG_TRI_WATERTIGHT, true>,
                 kPacketThreads);
 }
 
