@@ -801,6 +801,15 @@ __global__ void k_collapse(const PNode* __restrict__ nodes,
 
 // k_collapse with the children of each wide node taken from the dynamic
 // program above instead of by expanding the largest-area child.
+//
+// The order of a node's children is the order any-hit rays take them in (the
+// first, then from the last to the second).  Sorted by area, the smallest
+// first, they find occluders sooner than in the program's left-to-right order:
+// any hits of a 256x256x64 box 1.71 -> 1.45 ms, of 1024x1024x32 paths over
+// 1.3 M triangles 25.3 -> 23.2 ms and their packets 7.7 -> 6.4, of 16 batched
+// jobs 18.6 -> 17.5; point pairs over 327,682 triangles unchanged.  The
+// largest first, or the most expensive subtree: 1.86 ms, 25.1, 7.2, 18.6; by
+// subtree cost per area the same as by area.
 __global__ void k_collapse_sah(const PNode* __restrict__ nodes,
                                const uint32_t* __restrict__ choice,
                                const uint2* __restrict__ fin,
@@ -844,9 +853,38 @@ __global__ void k_collapse_sah(const PNode* __restrict__ nodes,
         }
       }
     }
+    // interior children by surface area, the smallest first, then the leaves,
+    // then the unused slots
+    constexpr float kLeaf = 3.402823466e38f;
+    float key[W];
     int ni = 0;
-    for (int c = 0; c < nc; ++c)
-      ni += __float_as_int(nodes[ch[c]].b.w) == 0 ? 1 : 0;
+#pragma unroll
+    for (int c = 0; c < W; ++c) {
+      key[c] = __int_as_float(0x7f800000);
+      if (c < nc) {
+        const PNode x = nodes[ch[c]];
+        const bool leaf = __float_as_int(x.b.w) != 0;
+        key[c] = leaf ? kLeaf : fminf(area(xyz(x.a), xyz(x.b)), 1e38f);
+        ni += leaf ? 0 : 1;
+      } else {
+        ch[c] = 0;
+      }
+    }
+    auto order = [&](int p, int q) {
+      if (key[q] < key[p]) {
+        const float tk = key[p];
+        key[p] = key[q];
+        key[q] = tk;
+        const uint32_t tc = ch[p];
+        ch[p] = ch[q];
+        ch[q] = tc;
+      }
+    };
+    order(0, 1);
+    order(2, 3);
+    order(0, 2);
+    order(1, 3);
+    order(1, 2);
     uint32_t base = 0, fo = 0;
     if (ni) {
       base = atomicAdd(&counters[0], (uint32_t)ni);

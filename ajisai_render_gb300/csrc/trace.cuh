@@ -121,7 +121,7 @@ __device__ __forceinline__ bool mt_test(const RayQ& r, float4 A, float4 B,
 // sum and the scaled distance exactly: the sign test is symmetric, and t and
 // the barycentrics are the quotients, so the winding needs no axis swap.
 // (Six selects a vertex by the axes' numbers, and their comparisons: closest
-// hits of a 512x512x8 path trace over 4,814 triangles 8.51 ms, so 7.67.)
+// hits of 853x479x16 paths over 9,002 triangles: 8.51 ms, so 7.67.)
 struct WtSetup {
   bool zx, zy;  // kz is x, is y
   float sx, sy, sz;
