@@ -583,8 +583,9 @@ int ajg_scene_create_flat_ex(ajg_ctx* ctx, const float* tris,
   auto* s = new ajg_scene();
   s->ctx = ctx;
   // lights: the emitters' area lights first (default_scene.cpp:33-48), then
-  // the records as given; env records get the two mass flags of the 1x1
-  // Distribution2D (utility/distribution.h:40-60, 135-144)
+  // the records as given with what no hit changes (light records, scene.cuh);
+  // env records get the two mass flags of the 1x1 Distribution2D
+  // (utility/distribution.h:40-60, 135-144)
   const uint32_t nl_all = num_area + num_lights;
   s->host_lights.resize(12 * (size_t)nl_all);
   std::vector<float> emit_pts;
@@ -604,8 +605,15 @@ int ajg_scene_create_flat_ex(ajg_ctx* ctx, const float* tris,
       const float func_int = 0.f + w * (1.f / 1.f);
       r[10] = func_int > 0.f ? 1.f : 0.f;
       r[11] = func_int * func_int != 0.f ? 1.f : 0.f;
+      constexpr float inv_2_pi = 1.f / (2.f * kPi);
+      r[4] = r[9] / 180 * kPi * inv_2_pi;
     } else {
-      r[10] = r[11] = 0.f;
+      const float x = r[4], y = r[5], z = r[6];
+      const float inv = 1.f / std::sqrt(0.f + x * x + y * y + z * z);
+      r[8] = x * inv;
+      r[9] = y * inv;
+      r[10] = z * inv;
+      r[11] = -1.f / (std::copysign(1.f, r[10]) + r[10]);
     }
   }
   s->host_materials.resize(16 * (size_t)num_materials);

@@ -89,8 +89,11 @@ inline DeviceScene closest_view(const DeviceScene& s) {
   return c;
 }
 
-// Light record types ([12] floats, type in [0]): the two of the ABI, and the
-// area light of an emissive primitive:
+// Light record types ([12] floats, type in [0]): the two of the ABI -- a
+// directional light's unit direction in [8..10] and its frame's division in
+// [11], an environment's rotation as a share of a turn in [4], by the
+// samplers' own operations, so that no hit repeats them -- and the area light
+// of an emissive primitive:
 //   [1..3] radiance, [4] geometry (AJG_GEOM_*), [5] two-sided,
 //   [6] triangles (uint bits), [7] 1 / area, [8] the quad's (a,b,c) share of
 //   its area, [9] Geometry::Pdf (the same for every point of the surface),

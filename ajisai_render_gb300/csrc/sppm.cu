@@ -348,7 +348,7 @@ __device__ Emission sample_emit(const SppmArgs& a, const float* L,
     const float u0 = key_float(key, dim), u1 = key_float(key, dim + 1);
     dim += 2;
     const F3 r2l =
-        Frame(normalize3(mk3(L[4], L[5], L[6]))).to_world(uniform_cone(u0, u1, L[7]));
+        Frame(mk3(L[8], L[9], L[10]), L[11]).to_world(uniform_cone(u0, u1, L[7]));
     const float pdf_dir = uniform_cone_pdf(L[7]);
     const float radius = a.s.radius;
     float dx, dy;
@@ -369,9 +369,8 @@ __device__ Emission sample_emit(const SppmArgs& a, const float* L,
     dim += 2;
     if (L[10] == 0.f) return Emission{};  // the 1x1 distribution has no mass
     float pdf = 1.f;
-    constexpr float inv_2_pi = 1.f / (2.f * kPi);
     constexpr float two_pi = 2.f * kPi;
-    u -= L[9] / 180 * kPi * inv_2_pi;
+    u -= L[4];
     if (u > 1.f) u -= 1.f;
     if (u < 0.f) u += 1.f;
     const float phi = u * two_pi;
