@@ -356,10 +356,11 @@ inline int trace_grid(const void* fn, int threads) {
                           // votes (a lane leaves early with a leaf found or its
                           // ray done).  Any-hit ms of the Cornell box, the 1.3 M
                           // sphere and 16 batched jobs: 1 visit 1.77 / 24.9 /
-                          // 19.5, 2 1.81 / 24.5 / -, 3 1.70 / 24.5 / 18.9, 4
-                          // 1.80 / 25.0 / 19.1, 6 1.82 / 26.0 / 19.8.  Closest
-                          // hits, with their leaf tests in the visit: 1 visit
-                          // 20.2 ms, 2 20.6, 3 20.3, 4 20.7
+                          // 19.5 before the children were sorted by area;
+                          // since then 2 1.60 / 23.3 / 17.8, 3 1.45 / 23.3 /
+                          // 17.5, 4 1.54 / 23.5 / 17.7.  Closest hits, with
+                          // their leaf tests in the visit: 1 visit 20.2 ms, 2
+                          // 20.6, 3 20.3, 4 20.7
 #endif
 #ifndef AJG_LEAF_DEFER_CLOSEST
 #define AJG_LEAF_DEFER_CLOSEST 0  // the same for closest-hit queries over
