@@ -518,9 +518,9 @@ __global__ void k_deposit_sort(Deposits dp) {
 // unit of 32 points x 32 photons.  A lane holds one visible point and its
 // sums; the 32 photons sit in shared memory, read by all lanes at once for
 // the distance test; the photons a lane accepts are then evaluated one a
-// round, so that lanes with different photons share the rounds.  A warp's
-// units are consecutive, and a group of points keeps its sums over its run
-// of photons: one atomic add per point and run instead of one per pair.
+// round, so that lanes with different photons share the rounds.  A group of
+// points keeps its sums over a run of photons: one atomic add per point and
+// run instead of one per pair.
 // Bound by instruction issue (the distance tests and BSDF evaluations).  A
 // photon walking its entry's list by itself (the form before this) left
 // 2.8 of 32 threads active and added every pair atomically: 925 us a depth
@@ -529,9 +529,17 @@ __global__ void k_deposit_sort(Deposits dp) {
 // iterations; 512x512, radius 0.01, 2 M photons over 327,682 triangles:
 // 14.1 -> 10.8 ms for 4), 372 us with the points' BSDF terms prepared once.
 //
+// A unit costs from 32 distance tests a lane to 32 evaluations more, and dense
+// entries lie together, so a warp takes kRuns short runs spread over all units
+// rather than one share (which left half the warps of the box above waiting
+// for the rest: 4.6 ms, 4 runs 3.1, runs of one unit -- 8 and more -- 2.8; the
+// sphere, with few pairs a unit and more units, loses 10 to 20 us of 210).
+//
 // 8 blocks of 128 an SM (64 registers, 200 bytes of spills beside the BSDF's
-// prepared terms in local memory): 4.5 ms on the box above, 6 blocks 5.6,
-// 5 6.1, 4 without spills 7.0.  Only the Lambertian lobe prepared: 7.6.
+// prepared terms in local memory): 4.5 ms on the box above with one share
+// a warp, 6 blocks 5.6, 5 6.1, 4 without spills 7.0.  Only the Lambertian lobe
+// prepared: 7.6.
+constexpr uint32_t kRuns = 8;
 __global__ void __launch_bounds__(kThreads, 8)
     k_deposit(SppmArgs a, SppmPixels px, Grid g, Deposits dp) {
   __shared__ float4 s_rec[kThreads / 32][32 * 3];
@@ -540,91 +548,93 @@ __global__ void __launch_bounds__(kThreads, 8)
   const uint64_t n_warps = (uint64_t)gridDim.x * (kThreads / 32);
   const uint64_t wid = (uint64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
   const unsigned long long total = dp.units[kEntries];
-  // the warp's share [u, end); total * wid would overflow only beyond 2^50
-  // units
-  unsigned long long u = total / n_warps * wid + min((uint64_t)(total % n_warps), wid);
-  const unsigned long long end =
-      u + total / n_warps + (wid < total % n_warps ? 1 : 0);
-  if (u >= end) return;
-  uint32_t e = 0;  // the entry of unit u: the last with units[e] <= u
-  for (uint32_t hi = kEntries; hi - e > 1;) {
-    const uint32_t mid = (e + hi) >> 1;
-    if (dp.units[mid] <= u)
-      e = mid;
-    else
-      hi = mid;
-  }
-  while (u < end) {
-    // skip entries whose units end at or before u
-    for (;;) {
-      const uint32_t c = e + 1 + (uint32_t)lane;
-      const unsigned past =
-          __ballot_sync(kFull, c < kEntries && dp.units[c] <= u);
-      e += __popc(past);
-      if (past != kFull) break;
+  // the warps' runs of `run` units, dealt out in turn
+  const unsigned long long share = (total + n_warps - 1) / n_warps;
+  const unsigned long long run = (share + kRuns - 1) / kRuns;
+  for (unsigned long long u0 = wid * run; u0 < total; u0 += n_warps * run) {
+    unsigned long long u = u0;
+    const unsigned long long end = min(u0 + run, total);
+    // the entry of unit u: the last with units[e] <= u, 32 pivots a round
+    uint32_t e = 0;
+    for (uint32_t hi = kEntries; hi - e > 1;) {
+      const uint32_t step = (hi - e + 31) / 32;
+      const uint32_t c = e + step * ((uint32_t)lane + 1);
+      const unsigned past = __ballot_sync(kFull, c < hi && dp.units[c] <= u);
+      e += step * __popc(past);
+      hi = min(hi, e + step);
     }
-    const uint32_t i0 = g.offsets[e], i1 = min(g.offsets[e + 1], g.cap);
-    const uint32_t p0 = dp.offsets[e], p1 = dp.offsets[e + 1];
-    const uint32_t tiles = (p1 - p0 + 31) / 32;
-    const unsigned long long local = u - dp.units[e];
-    const uint32_t group = (uint32_t)(local / tiles);
-    const uint32_t t0 = (uint32_t)(local % tiles);
-    const uint32_t t1 = (uint32_t)min((unsigned long long)tiles, t0 + (end - u));
-    const uint32_t item = i0 + group * 32 + (uint32_t)lane;
-    const bool on = item < i1;
-    const float4 sp = on ? __ldg(&g.spheres[item]) : make_float4(0, 0, 0, 0);
-    Bsdf f;
-    F3 sum = mk3(0, 0, 0);
-    uint32_t pix = 0, m_sum = 0;
-    bool loaded = false;
-    for (uint32_t t = t0; t < t1; ++t) {
-      const uint32_t first = p0 + 32 * t;
-      const int cnt = (int)min(32u, p1 - first);
-      if (lane < cnt) {
-        const float4* r = dp.rec + 3 * (uint64_t)dp.sorted[first + lane];
-        tile[3 * lane] = r[0];
-        tile[3 * lane + 1] = r[1];
-        tile[3 * lane + 2] = r[2];
+    while (u < end) {
+      // skip entries whose units end at or before u
+      for (;;) {
+        const uint32_t c = e + 1 + (uint32_t)lane;
+        const unsigned past =
+            __ballot_sync(kFull, c < kEntries && dp.units[c] <= u);
+        e += __popc(past);
+        if (past != kFull) break;
       }
-      __syncwarp();
-      unsigned near = 0;
+      const uint32_t i0 = g.offsets[e], i1 = min(g.offsets[e + 1], g.cap);
+      const uint32_t p0 = dp.offsets[e], p1 = dp.offsets[e + 1];
+      const uint32_t tiles = (p1 - p0 + 31) / 32;
+      const unsigned long long local = u - dp.units[e];
+      const uint32_t group = (uint32_t)(local / tiles);
+      const uint32_t t0 = (uint32_t)(local % tiles);
+      const uint32_t t1 = (uint32_t)min((unsigned long long)tiles, t0 + (end - u));
+      const uint32_t item = i0 + group * 32 + (uint32_t)lane;
+      const bool on = item < i1;
+      const float4 sp = on ? __ldg(&g.spheres[item]) : make_float4(0, 0, 0, 0);
+      Bsdf f;
+      F3 sum = mk3(0, 0, 0);
+      uint32_t pix = 0, m_sum = 0;
+      bool loaded = false;
+      for (uint32_t t = t0; t < t1; ++t) {
+        const uint32_t first = p0 + 32 * t;
+        const int cnt = (int)min(32u, p1 - first);
+        if (lane < cnt) {
+          const float4* r = dp.rec + 3 * (uint64_t)dp.sorted[first + lane];
+          tile[3 * lane] = r[0];
+          tile[3 * lane + 1] = r[1];
+          tile[3 * lane + 2] = r[2];
+        }
+        __syncwarp();
+        unsigned near = 0;
 #pragma unroll 4
-      for (int j = 0; j < cnt; ++j) {
-        const F3 d = xyz(sp) - xyz(tile[3 * j]);
-        if (!(dot3(d, d) > sp.w)) near |= 1u << j;
-      }
-      if (!on) near = 0;
-      if (near && !loaded) {
-        pix = g.items[item];
-        const VisPointD v = px.vp[pix];
-        const uint32_t mat = __float_as_uint(v.pos.w);
-        f.prepare(a.s.materials + 16 * mat, __ldg(&a.s.mat_lum[mat].x), xyz(v.ng),
-                  xyz(v.ns), xyz(v.wr));
-        loaded = true;
-      }
-      while (__any_sync(kFull, near != 0)) {
-        if (near) {
-          const int j = __ffs(near) - 1;
-          near &= near - 1;
-          const float px_ = tile[3 * j].w;
-          const float4 q = tile[3 * j + 1];
-          const float wz = tile[3 * j + 2].x;
-          const F3 c = mk3(px_, q.x, q.y) * f.eval(mk3(q.z, q.w, wz));
-          if (isfinite(c.x) && isfinite(c.y) && isfinite(c.z)) {
-            sum = sum + c;
-            ++m_sum;
+        for (int j = 0; j < cnt; ++j) {
+          const F3 d = xyz(sp) - xyz(tile[3 * j]);
+          if (!(dot3(d, d) > sp.w)) near |= 1u << j;
+        }
+        if (!on) near = 0;
+        if (near && !loaded) {
+          pix = g.items[item];
+          const VisPointD v = px.vp[pix];
+          const uint32_t mat = __float_as_uint(v.pos.w);
+          f.prepare(a.s.materials + 16 * mat, __ldg(&a.s.mat_lum[mat].x), xyz(v.ng),
+                    xyz(v.ns), xyz(v.wr));
+          loaded = true;
+        }
+        while (__any_sync(kFull, near != 0)) {
+          if (near) {
+            const int j = __ffs(near) - 1;
+            near &= near - 1;
+            const float px_ = tile[3 * j].w;
+            const float4 q = tile[3 * j + 1];
+            const float wz = tile[3 * j + 2].x;
+            const F3 c = mk3(px_, q.x, q.y) * f.eval(mk3(q.z, q.w, wz));
+            if (isfinite(c.x) && isfinite(c.y) && isfinite(c.z)) {
+              sum = sum + c;
+              ++m_sum;
+            }
           }
         }
+        __syncwarp();
       }
-      __syncwarp();
+      if (m_sum) {
+        atomicAdd(&px.phi[pix].x, sum.x);
+        atomicAdd(&px.phi[pix].y, sum.y);
+        atomicAdd(&px.phi[pix].z, sum.z);
+        atomicAdd(&px.M[pix], m_sum);
+      }
+      u += t1 - t0;
     }
-    if (m_sum) {
-      atomicAdd(&px.phi[pix].x, sum.x);
-      atomicAdd(&px.phi[pix].y, sum.y);
-      atomicAdd(&px.phi[pix].z, sum.z);
-      atomicAdd(&px.M[pix], m_sum);
-    }
-    u += t1 - t0;
   }
 }
 
