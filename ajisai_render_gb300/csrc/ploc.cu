@@ -1107,10 +1107,17 @@ struct BuildMem {
 
 // The arrays only shading reads, copied in on the trace stream while the
 // tree is built (1,310,722 triangles: 58 of 105 MB, 330 us); done before the
-// build returns, whichever way it does.
+// build returns, whichever way it does.  Two of them lie in the kept scratch,
+// which the renders enqueued before may still be using on the context's
+// stream (ajg_render_device returns with its film there): the trace stream
+// waits for that stream as it was when the scratch was taken.
 struct ShadingCopy {
   ajg_ctx* ctx;
   bool started = false;
+  explicit ShadingCopy(ajg_ctx* c) : ctx(c) {
+    cudaEventRecord(ctx->ev_queue, ctx->stream);
+    cudaStreamWaitEvent(ctx->trace_stream, ctx->ev_queue, 0);
+  }
   void start(int32_t* d_mat, const int32_t* mat, int32_t* d_flags,
              const int32_t* flags, float* d_corner, const float* corner,
              uint64_t n) {
@@ -1276,6 +1283,7 @@ int build_scene(ajg_ctx* ctx, ajg_scene* s, const float* h_tris,
   if (!tmp.take(ctx, (uint64_t)(uintptr_t)temporaries(nullptr), st))
     return set_err(ctx, AJG_ERR_OOM, "device allocation failed (PLOC build)");
   temporaries(tmp.p);
+  ShadingCopy shading(ctx);
 
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
@@ -1348,7 +1356,6 @@ int build_scene(ajg_ctx* ctx, ajg_scene* s, const float* h_tris,
                        (int)sizeof(TailMem));
   const int g_nb = grid_for(n, kClusterThreads, kSMs * 8);
   const int g_pair = grid_for(n, kPairTile, kSMs * 8);
-  ShadingCopy shading{ctx};
   PlocState h{};
   int batch = n > kTail ? (int)std::ceil(std::log((double)n / kTail) / std::log(1.25)) + 1
                         : 0;

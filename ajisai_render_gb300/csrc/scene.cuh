@@ -396,9 +396,12 @@ namespace ajg {
 // kScratchKeep bytes for it, grown on demand and freed with the context: a
 // stream-ordered allocation whose memory went back to the system at the last
 // synchronisation costs about 100 us a buffer (a first 128x128 preview after
-// one: 789 -> 573 us; SPPM with 26 buffers, 10.8 -> 8.4 ms).  The block belongs to the call
-// that holds the context's mutex, and all its uses are ordered on the
-// context's stream.  A larger scratch, and one taken while the stream is
+// one: 789 -> 573 us; SPPM with 26 buffers, 10.8 -> 8.4 ms).  The block belongs
+// to the call that holds the context's mutex, and all its uses are ordered on
+// the context's stream; the calls before may still be using it there
+// (ajg_render_device does not wait), so a use on another stream waits for an
+// event recorded there once the scratch is taken, and the context's stream
+// for that use in turn.  A larger scratch, and one taken while the stream is
 // being captured (the graph then owns it), is allocated in stream order for
 // the call alone.
 constexpr uint64_t kScratchKeep = 4ull << 30;
