@@ -972,6 +972,7 @@ cudaError_t Scratch::take(ajg_ctx* ctx, uint64_t bytes, cudaStream_t st) {
     const cudaError_t e = cudaMallocAsync((void**)&p, bytes, st);
     own = st;
     owned = e == cudaSuccess;
+    if (!owned) cudaGetLastError();
     return e;
   }
   if (ctx->scratch.bytes < bytes) {

@@ -16,8 +16,9 @@
 //     deposit and samples the BSDF; roulette draws as the reference draws
 //     them;
 //   the deposits (AddPhoton: EvalAll at each visible point of the photon's
-//     entry within its radius) of all depths of an iteration at once: the records sorted by
-//     hash entry and joined entry by entry with the grid's visible points
+//     entry within its radius) of all depths of an iteration at once, or of
+//     the depths a record buffer holds (photon_plan.cuh): the records sorted
+//     by hash entry and joined entry by entry with the grid's visible points
 //     (k_deposit);
 //   the radius reduction and UpdatePixel (sppm.cpp:145-169).
 // Photon i of iteration k draws from path_key(photon_seed(seed), i, k).
@@ -27,6 +28,7 @@
 #include <string>
 #include <vector>
 
+#include "photon_plan.cuh"
 #include "shade.cuh"
 #include "trace.cuh"
 
@@ -36,8 +38,6 @@ namespace {
 constexpr uint32_t kEntries = 40960;   // VisiblePointSearcher(..., 40960)
 constexpr int kMaxCellsPerAxis = 4;    // a radius box spans <= 3 cells
 constexpr int kThreads = 128;
-constexpr uint64_t kDepositRecords = 1ull << 25;  // of a wave: 48 + 4 bytes each
-constexpr uint64_t kWavePhotons = 1ull << 21;  // waves of several iterations
 constexpr unsigned kFull = 0xffffffffu;
 
 int fail(ajg_ctx* ctx, int code, const std::string& m) {
@@ -817,33 +817,15 @@ int sppm_render(ajg_scene* sc, const ajg_camera& cam, const ajg_sppm_params& p,
     a.lpdf = table[0];
   }
 
-  // A photon wave holds an iteration's photons, in equal chunks of at most the
-  // context's wave size whose deposits (one per depth from 2 on) fit the record
-  // buffer -- or, as photons do not depend on the iterations before, those of
-  // several iterations, so that a wave of small ones still fills the GPU (12
-  // iterations x 100,000 photons of the emitter box, radius 0.1: 240 launches
-  // of rays and shading, 4.7 ms, became 20, 1.5 ms; 10.9 -> 7.5 ms a render).
+  // Photon waves (photon_plan).  As photons do not depend on the iterations
+  // before, a wave holds those of several, so that small ones still fill the
+  // GPU (12 iterations x 100,000 photons of the emitter box, radius 0.1: 240
+  // launches of rays and shading, 4.7 ms, became 20, 1.5 ms; 10.9 -> 7.5 ms a
+  // render).
   const uint64_t dep_depths = p.photon_max_depth > 1 ? p.photon_max_depth - 1 : 0;
-  uint64_t most = ctx->wave_paths;
-  if (dep_depths) most = std::min<uint64_t>(most, kDepositRecords / dep_depths);
-  uint64_t chunk = std::max<uint64_t>(
-      1, std::min<uint64_t>(p.photons_per_iteration, most));
-  const uint64_t n_chunks = (p.photons_per_iteration + chunk - 1) / chunk;
-  if (n_chunks) chunk = (p.photons_per_iteration + n_chunks - 1) / n_chunks;
-  uint64_t group = 1;  // iterations of a wave
-  if (n_chunks == 1) {
-    group = std::min<uint64_t>(std::min<uint64_t>(most, kWavePhotons) / chunk,
-                               p.iterations);
-    group = std::max<uint64_t>(group, 1);
-    const uint64_t waves = (p.iterations + group - 1) / group;
-    group = (p.iterations + waves - 1) / waves;
-  }
-  const uint64_t wave = chunk * group;  // photons
-  const uint64_t dep_cap = chunk * dep_depths;  // deposits of an iteration
-  // zeroed per wave: the depths' queue counters and the iterations' deposit
-  // counts
   const uint64_t n_depths = 2 * ((uint64_t)p.photon_max_depth + 2);
-  const uint64_t n_counts = n_depths + group;
+  PhotonPlan plan{};
+  uint64_t wave = 0, n_counts = 0;
   const uint32_t cap = (uint32_t)std::min<uint64_t>(8 * npix, 0xffffffffull);
 
   // the camera pass's wave arena first, then everything else
@@ -880,18 +862,28 @@ int sppm_render(ajg_scene* sc, const ajg_camera& cam, const ajg_sppm_params& p,
     qhits = carve<ajg_hit>(cur, wave);
     qcounts = carve<uint32_t>(cur, n_counts);
     dhist = carve<uint32_t>(cur, kEntries);
-    drec = carve<float4>(cur, 3 * dep_cap * group);
+    drec = carve<float4>(cur, 3 * plan.records * plan.group);
     doff = carve<uint32_t>(cur, kEntries + 1);
     dunits = carve<unsigned long long>(cur, kEntries + 1);
-    dsorted = carve<uint32_t>(cur, dep_cap);
+    dsorted = carve<uint32_t>(cur, plan.records);
     totals = carve<EntryVal>(cur, kEntryBlocks);
     if (want_film) d_out = carve<float4>(cur, npix);
     if (want_rad) d_rad = carve<float>(cur, 3 * npix);
     return cur;
   };
-  const uint64_t bytes = (uint64_t)(uintptr_t)layout(nullptr);
-  if (scratch.take(ctx, bytes, st) != cudaSuccess)
-    return fail(ctx, AJG_ERR_OOM, "device allocation failed (SPPM buffers)");
+  for (int tries = 0;; ++tries) {
+    plan = photon_plan(p.photons_per_iteration, p.iterations, p.photon_max_depth,
+                       ctx->wave_paths, tries);
+    wave = plan.chunk * plan.group;  // photons
+    // zeroed per wave: the depths' queue counters and the iterations' deposit
+    // counts
+    n_counts = n_depths + plan.group;
+    if (scratch.take(ctx, (uint64_t)(uintptr_t)layout(nullptr), st) == cudaSuccess)
+      break;
+    if (tries > 0 && plan.chunk == 1)
+      return fail(ctx, AJG_ERR_OOM, "device allocation failed (SPPM buffers)");
+  }
+  const uint64_t chunk = plan.chunk, group = plan.group;
   layout(scratch.p);
   *out_film = d_out;
   *out_rad = d_rad;
@@ -925,8 +917,18 @@ int sppm_render(ajg_scene* sc, const ajg_camera& cam, const ajg_sppm_params& p,
   dp.offsets = doff;
   dp.units = dunits;
   dp.sorted = dsorted;
-  dp.cap = (uint32_t)dep_cap;
+  dp.cap = (uint32_t)plan.records;
   const int gd = resident_grid((const void*)k_deposit, kThreads);
+  // Joins the recorded deposits of an iteration with its grid.
+  auto join = [&](const Deposits& d) {
+    const int gr = grid_for(plan.records, 256, gs);
+    cudaMemsetAsync(d.hist, 0, kEntries * sizeof(uint32_t), st);
+    k_deposit_enter<<<gr, 256, 0, st>>>(a, g, d);
+    k_entry_totals<true><<<kEntryBlocks, kEntryThreads, 0, st>>>(g, d, totals);
+    k_entry_scan<true><<<kEntryBlocks, kEntryThreads, 0, st>>>(g, d, totals);
+    k_deposit_sort<<<gr, 256, 0, st>>>(d);
+    k_deposit<<<gd, kThreads, 0, st>>>(a, px, g, d);
+  };
   // Traces photons [i0, i0 + m) of `iters` iterations from it0 on.
   auto trace = [&](uint32_t it0, uint32_t iters, uint64_t i0) {
     a.it0 = it0;
@@ -949,6 +951,11 @@ int sppm_render(ajg_scene* sc, const ajg_camera& cam, const ajg_sppm_params& p,
       });
       k_photon_shade<<<grid_for(n, kThreads, gs), kThreads, 0, st>>>(
           a, q, dp, depth, ctx->d_error);
+      // the record buffer may be full, and photons of a depth to come live
+      if (depth > 1 && depth < p.photon_max_depth && (depth - 1) % plan.depths == 0) {
+        join(dp);
+        cudaMemsetAsync(dp.count, 0, sizeof(uint32_t), st);
+      }
     }
     ctx->paths_total += n;
   };
@@ -964,15 +971,9 @@ int sppm_render(ajg_scene* sc, const ajg_camera& cam, const ajg_sppm_params& p,
         trace(it, std::min<uint32_t>((uint32_t)group, p.iterations - it), i0);
       if (!dep_depths) continue;
       Deposits own = dp;
-      own.rec += 3 * dep_cap * j;
+      own.rec += 3 * plan.records * j;
       own.count += j;
-      const int gr = grid_for(dep_cap, 256, gs);
-      cudaMemsetAsync(dp.hist, 0, kEntries * sizeof(uint32_t), st);
-      k_deposit_enter<<<gr, 256, 0, st>>>(a, g, own);
-      k_entry_totals<true><<<kEntryBlocks, kEntryThreads, 0, st>>>(g, own, totals);
-      k_entry_scan<true><<<kEntryBlocks, kEntryThreads, 0, st>>>(g, own, totals);
-      k_deposit_sort<<<gr, 256, 0, st>>>(own);
-      k_deposit<<<gd, kThreads, 0, st>>>(a, px, g, own);
+      join(own);
     }
     cudaMemsetAsync(bits, 0, sizeof(uint32_t), st);
     k_max_radius<<<grid_for(npix, 256, gs), 256, 0, st>>>(a, px, bits);
