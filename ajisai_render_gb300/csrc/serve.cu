@@ -6,8 +6,8 @@
 // (scenes + arena + films + result buffers), plans each wave from the
 // running jobs (one chunk per job and wave: a pixel range of the job's
 // current sample pass, or several whole passes of its window when they fit),
-// uploads the tables, launches the wave's bounce loop as one CUDA graph
-// (cached per bounce count and triangle test) and then the resolves and
+// uploads the tables, launches the wave's bounce loop (as one CUDA graph from
+// the third wave of its kind on, see graph_for) and then the resolves and
 // copies of the results that wave completes.  Up to `inflight_waves` waves
 // are queued ahead; results are handed over when their wave's event fires.
 //
@@ -155,7 +155,12 @@ struct Server {
   std::vector<char*> h_tables;  // pinned, one per in-flight slot + 1
   size_t table_bytes = 0;
   uint64_t wave_no = 0;
-  std::map<std::tuple<int, int, int, bool, bool, uint32_t>, cudaGraphExec_t> graphs;
+  // captured waves by what their launches depend on (see graph_for)
+  struct WaveGraph {
+    cudaGraphExec_t exec = nullptr;
+    int direct = 0;  // waves launched without it so far
+  };
+  std::map<std::tuple<int, int, int, bool, bool, uint32_t>, WaveGraph> graphs;
   std::deque<InFlight> inflight;
   std::vector<uint32_t*> err_words;  // pinned, recycled
   uint32_t* d_err = nullptr;
@@ -172,6 +177,7 @@ struct Server {
   int ensure_arena(int nt, uint64_t target_paths);
   cudaGraphExec_t graph_for(int bounces, int tri_test, int width, bool emit,
                             bool packets, uint32_t mat_mask);
+  void drop_graphs();
 };
 
 namespace {
@@ -197,8 +203,7 @@ int Server::ensure_arena(int nt, uint64_t target) {
   if (arena && nt <= NT && P == target) return AJG_OK;
   // a bigger light count needs a bigger arena: drain, then regrow
   while (!inflight.empty()) retire_oldest();
-  for (auto& g : graphs) cudaGraphExecDestroy(g.second);
-  graphs.clear();
+  drop_graphs();
   if (arena) cudaFree(arena);
   arena = nullptr;
   P = target;
@@ -220,27 +225,50 @@ int Server::ensure_arena(int nt, uint64_t target) {
   return AJG_OK;
 }
 
+void Server::drop_graphs() {
+  for (auto& g : graphs)
+    if (g.second.exec) cudaGraphExecDestroy(g.second.exec);
+  graphs.clear();
+}
+
+// The captured wave with these launches; null: launch them on the stream.
+// Capturing and instantiating one takes 0.35 to 0.6 ms, in the middle of
+// serving, and saves a small wave 0.05 to 0.15 ms (64x64x1 over the box 0.48
+// -> 0.42 ms, the material box 1.24 -> 1.09), so the first two waves of a
+// kind go as they are and the third is captured.
+constexpr int kDirectWaves = 2;
 cudaGraphExec_t Server::graph_for(int bounces, int tri_test, int width,
                                   bool emit, bool packets,
                                   uint32_t mat_mask) {
-  const auto key =
-      std::make_tuple(bounces, tri_test, width, emit, packets, mat_mask);
-  auto it = graphs.find(key);
-  if (it != graphs.end()) return it->second;
+  WaveGraph& kept =
+      graphs[std::make_tuple(bounces, tri_test, width, emit, packets, mat_mask)];
+  if (kept.exec) return kept.exec;
+  if (kept.direct < kDirectWaves) {
+    ++kept.direct;
+    return nullptr;
+  }
   prepare_mj_kernels();
   cudaGraph_t g = nullptr;
   cudaGraphExec_t ex = nullptr;
   if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) !=
-      cudaSuccess)
+      cudaSuccess) {
+    cudaGetLastError();
     return nullptr;
+  }
   enqueue_mj_wave(t, w, P, NT, bounces, tri_test, width, emit, mat_mask, d_ctr,
                   d_err, st, ctx->overlap ? ts : nullptr, ev_queue, ev_hits,
                   ctx->packet_camera, packets);
-  if (cudaStreamEndCapture(st, &g) != cudaSuccess || !g) return nullptr;
-  if (cudaGraphInstantiate(&ex, g, 0) != cudaSuccess) ex = nullptr;
+  if (cudaStreamEndCapture(st, &g) != cudaSuccess || !g) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (cudaGraphInstantiate(&ex, g, 0) != cudaSuccess) {
+    cudaGetLastError();
+    ex = nullptr;
+  }
   cudaGraphDestroy(g);
   if (ex) {
-    graphs[key] = ex;
+    kept.exec = ex;
     ++stats.graph_builds;
   }
   return ex;
@@ -551,8 +579,7 @@ bool Server::plan_and_launch() {
   cudaGraphExec_t g = graph_for(bounces, tri_test, width, emit, packets, mat_mask);
   if (g) {
     cudaGraphLaunch(g, st);
-  } else {  // capture unavailable: the same launches on the stream
-    cudaGetLastError();
+  } else {
     enqueue_mj_wave(t, w, P, NT, bounces, tri_test, width, emit, mat_mask, d_ctr,
                     d_err, st, ctx->overlap ? ts : nullptr, ev_queue, ev_hits,
                     ctx->packet_camera, packets);
@@ -795,7 +822,7 @@ void server_shutdown(ajg_ctx* ctx) {
   s->cv_work.notify_all();
   s->th.join();
   cudaStreamSynchronize(s->st);
-  for (auto& g : s->graphs) cudaGraphExecDestroy(g.second);
+  s->drop_graphs();
   for (char* h : s->h_tables) cudaFreeHost(h);
   for (uint32_t* e : s->err_words) cudaFreeHost(e);
   if (s->ring.base) cudaFreeHost(s->ring.base);

@@ -407,7 +407,8 @@ AJG_API int ajg_render_static(ajg_scene* scene, const ajg_camera* cam,
  * films resident, admits jobs as the HBM budget (ajg_config) allows, and
  * fills every wave of paths from many jobs at once: a wave carries chunks
  * (pixel range x sample range) of up to 1,024 jobs over their own scenes,
- * and its bounce loop is one CUDA graph launch.  Each pixel receives its
+ * and its bounce loop is one CUDA graph launch (the first two waves of a
+ * kind go launch by launch).  Each pixel receives its
  * samples in sample order, so a job's film is bit-identical to the same job
  * rendered alone (ajg_render) or in any mix.  Progressive results: every
  * `progress_spp` samples per pixel the job's window is resolved and
