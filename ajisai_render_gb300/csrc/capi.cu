@@ -210,10 +210,12 @@ template <class T>
 struct DevBuf {
   T* p = nullptr;
   cudaStream_t s = nullptr;
-  cudaError_t alloc(uint64_t count, cudaStream_t st) {
+  cudaError_t alloc(ajg_ctx* ctx, uint64_t count, cudaStream_t st) {
     s = st;
-    return cudaMallocAsync((void**)&p, count * sizeof(T) > 0 ? count * sizeof(T) : 16,
-                           st);
+    return device_malloc_async(ctx, (void**)&p, std::max<uint64_t>(count * sizeof(T), 16),
+                               st)
+               ? cudaSuccess
+               : cudaErrorMemoryAllocation;
   }
   ~DevBuf() {
     if (p) cudaFreeAsync(p, s);
@@ -650,9 +652,10 @@ int ajg_scene_create_flat_ex(ajg_ctx* ctx, const float* tris,
     return fail(ctx, AJG_ERR_OOM, "device allocation failed (scene tables)");
   }
   s->allocations.push_back(block);
-  s->info.device_bytes += n_mat * sizeof(float) + n_light * sizeof(float) +
-                          num_materials * sizeof(float4) + n_pts * sizeof(float) +
-                          (num_area ? n * sizeof(int32_t) : 0);
+  const uint64_t table_bytes = n_mat * sizeof(float) + n_light * sizeof(float) +
+                               num_materials * sizeof(float4) + n_pts * sizeof(float) +
+                               (num_area ? n * sizeof(int32_t) : 0);
+  s->info.device_bytes += table_bytes;
   layout(stage.data());
   std::memcpy(d_mat, s->host_materials.data(), n_mat * sizeof(float));
   if (nl_all)
@@ -677,6 +680,15 @@ int ajg_scene_create_flat_ex(ajg_ctx* ctx, const float* tris,
   s->d.env = env;
   int rc = build_scene(ctx, s, tris, corner_normals, tri_material, tri_flags,
                        n, world, o);
+  // The build's temporaries are in the kept scratch, which may be larger than
+  // they need: once more with it given back.
+  if (rc == AJG_ERR_OOM && scratch_drop(ctx)) {
+    for (; s->allocations.size() > 1; s->allocations.pop_back())
+      cudaFree(s->allocations.back());
+    s->info.device_bytes = table_bytes;
+    rc = build_scene(ctx, s, tris, corner_normals, tri_material, tri_flags, n,
+                     world, o);
+  }
   if (rc != AJG_OK) {
     std::string m = ctx->last_error;
     ajg_scene_release(s);
@@ -931,10 +943,10 @@ int ajg_bsdf_query(ajg_ctx* ctx, const ajg_material* materials,
   DevBuf<ajg_material> dm;
   DevBuf<float> dv, dout;
   DevBuf<int32_t> dop;
-  CK(dm.alloc(n, st), "bsdf_query");
-  CK(dv.alloc(15 * n, st), "bsdf_query");
-  CK(dout.alloc(8 * n, st), "bsdf_query");
-  CK(dop.alloc(n, st), "bsdf_query");
+  CK(dm.alloc(ctx, n, st), "bsdf_query");
+  CK(dv.alloc(ctx, 15 * n, st), "bsdf_query");
+  CK(dout.alloc(ctx, 8 * n, st), "bsdf_query");
+  CK(dop.alloc(ctx, n, st), "bsdf_query");
   // the device records: plastic's precomputed terms in the reserved floats
   std::vector<ajg_material> recs(materials, materials + n);
   for (uint64_t i = 0; i < n; ++i) {
@@ -969,8 +981,8 @@ int ajg_camera_rays(ajg_ctx* ctx, const ajg_camera* cam, const float* raster,
   cudaSetDevice(ctx->device);
   cudaStream_t st = ctx->stream;
   DevBuf<float> din, dout;
-  CK(din.alloc(4 * n, st), "camera_rays");
-  CK(dout.alloc(6 * n, st), "camera_rays");
+  CK(din.alloc(ctx, 4 * n, st), "camera_rays");
+  CK(dout.alloc(ctx, 6 * n, st), "camera_rays");
   cudaMemcpyAsync(din.p, raster, 4 * n * sizeof(float), cudaMemcpyHostToDevice, st);
   k_camera_rays<<<grid_for(n, 128), 128, 0, st>>>(*cam, din.p, n, dout.p);
   cudaMemcpyAsync(rays, dout.p, 6 * n * sizeof(float), cudaMemcpyDeviceToHost, st);

@@ -969,11 +969,9 @@ cudaError_t Scratch::take(ajg_ctx* ctx, uint64_t bytes, cudaStream_t st) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   cudaStreamIsCapturing(st, &cap);
   if (bytes > kScratchKeep || cap != cudaStreamCaptureStatusNone) {
-    const cudaError_t e = cudaMallocAsync((void**)&p, bytes, st);
     own = st;
-    owned = e == cudaSuccess;
-    if (!owned) cudaGetLastError();
-    return e;
+    owned = device_malloc_async(ctx, (void**)&p, bytes, st);
+    return owned ? cudaSuccess : cudaErrorMemoryAllocation;
   }
   if (ctx->scratch.bytes < bytes) {
     scratch_drop(ctx);
@@ -992,19 +990,43 @@ cudaError_t Scratch::take(ajg_ctx* ctx, uint64_t bytes, cudaStream_t st) {
 
 bool scratch_drop(ajg_ctx* ctx) {
   if (!ctx->scratch.ptr) return false;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(ctx->stream, &cap);
+  if (cap != cudaStreamCaptureStatusNone) return false;
   cudaStreamSynchronize(ctx->stream);
   cudaFree(ctx->scratch.ptr);
   ctx->scratch = Buffer{};
   return true;
 }
 
-bool device_malloc(ajg_ctx* ctx, void** p, uint64_t bytes) {
-  if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+bool scratch_yield(ajg_ctx* ctx) {
+  if (!ctx->mu.try_lock()) return false;
+  const bool dropped = scratch_drop(ctx);
+  ctx->mu.unlock();
+  return dropped;
+}
+
+template <class Alloc, class Drop>
+static bool alloc_or_drop(Alloc&& alloc, Drop&& drop, void** p) {
+  if (alloc() == cudaSuccess) return true;
   cudaGetLastError();
-  if (scratch_drop(ctx) && cudaMalloc(p, bytes) == cudaSuccess) return true;
+  if (drop() && alloc() == cudaSuccess) return true;
   cudaGetLastError();
   *p = nullptr;
   return false;
+}
+
+bool device_malloc(ajg_ctx* ctx, void** p, uint64_t bytes, bool locked) {
+  return alloc_or_drop(
+      [&] { return cudaMalloc(p, bytes); },
+      [&] { return locked ? scratch_drop(ctx) : scratch_yield(ctx); }, p);
+}
+
+bool device_malloc_async(ajg_ctx* ctx, void** p, uint64_t bytes, cudaStream_t st,
+                         bool locked) {
+  return alloc_or_drop(
+      [&] { return cudaMallocAsync(p, bytes, st); },
+      [&] { return locked ? scratch_drop(ctx) : scratch_yield(ctx); }, p);
 }
 
 int resident_grid(const void* fn, int threads, int carveout) {

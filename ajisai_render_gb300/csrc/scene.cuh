@@ -417,11 +417,18 @@ struct Scratch {
   }
 };
 // Frees the kept block (no call may be using it: the context's mutex is
-// held, before Scratch::take); false when there is none.
+// held, before Scratch::take); false when there is none, or the context's
+// stream is being captured.
 bool scratch_drop(ajg_ctx* ctx);
-// cudaMalloc, giving the kept scratch back first where memory is short
-// (conditions as for scratch_drop).
-bool device_malloc(ajg_ctx* ctx, void** p, uint64_t bytes);
+// The same for a thread that does not hold the mutex (the request loop):
+// false also while a call holds it.
+bool scratch_yield(ajg_ctx* ctx);
+// cudaMalloc and cudaMallocAsync, giving the kept scratch back where memory is
+// short: by scratch_drop, or where the mutex is not held (`locked` false) by
+// scratch_yield.
+bool device_malloc(ajg_ctx* ctx, void** p, uint64_t bytes, bool locked = true);
+bool device_malloc_async(ajg_ctx* ctx, void** p, uint64_t bytes, cudaStream_t st,
+                         bool locked = true);
 // The next `count` T of a scratch, 256-byte aligned, and their size there.
 template <class T>
 T* carve(char*& cur, uint64_t count) {

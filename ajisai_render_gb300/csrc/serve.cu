@@ -209,15 +209,8 @@ int Server::ensure_arena(int nt, uint64_t target) {
   P = target;
   NT = std::max(nt, NT > 0 ? NT : 3);
   arena_bytes = wave_bytes(P, NT, true);
-  bool ok = cudaMalloc(&arena, arena_bytes + counter_bytes(kMaxBounces)) == cudaSuccess;
-  if (!ok && ctx->mu.try_lock()) {  // the calls' kept scratch gives way
-    cudaGetLastError();
-    ok = scratch_drop(ctx) && cudaMalloc(&arena, arena_bytes + counter_bytes(kMaxBounces)) == cudaSuccess;
-    ctx->mu.unlock();
-  }
-  if (!ok) {
-    cudaGetLastError();
-    arena = nullptr;
+  if (!device_malloc(ctx, (void**)&arena, arena_bytes + counter_bytes(kMaxBounces),
+                     false)) {
     arena_bytes = 0;
     return AJG_ERR_OOM;
   }
@@ -328,7 +321,7 @@ bool Server::admit_locked() {
     }
     const uint64_t film_bytes = (uint64_t)j->npix * 32;
     void* film = nullptr;
-    if (cudaMallocAsync(&film, film_bytes, st) != cudaSuccess) {
+    if (!device_malloc_async(ctx, &film, film_bytes, st, false)) {
       pending.pop_front();
       end_job_locked(j, AJG_JOB_FAILED, AJG_ERR_OOM);
       continue;
@@ -339,7 +332,7 @@ bool Server::admit_locked() {
       j->out_dev = reinterpret_cast<float4*>(j->out_user_dev);
     } else {
       void* o = nullptr;
-      if (cudaMallocAsync(&o, (uint64_t)j->npix * 16, st) != cudaSuccess) {
+      if (!device_malloc_async(ctx, &o, (uint64_t)j->npix * 16, st, false)) {
         cudaFreeAsync(film, st);
         j->film = nullptr;
         pending.pop_front();
