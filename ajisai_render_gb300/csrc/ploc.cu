@@ -317,6 +317,7 @@ struct PlocState {
   uint32_t stuck;  // an iteration merged no pair
 };
 constexpr uint32_t kTail = 1024;
+constexpr uint32_t kMaxIterations = 100000;
 constexpr int kLevels = 64;  // levels of the wide collapse enqueued at most
 constexpr int kTailThreads = 1024;
 constexpr int kPairItems = 4;
@@ -1378,11 +1379,12 @@ int build_scene(ajg_ctx* ctx, ajg_scene* s, const float* h_tris,
     if (e != cudaSuccess)
       return set_err(ctx, AJG_ERR_CUDA,
                      std::string("PLOC build: ") + cudaGetErrorString(e));
+    if (h.iters > kMaxIterations)  // ended or not: the last batch and the
+                                   // tail do not stop at the limit
+      return set_err(ctx, AJG_ERR_DEVICE, "PLOC did not converge");
     if (h.stuck)
       return set_err(ctx, AJG_ERR_DEVICE, "PLOC iteration merged no pair");
     if (h.cnt == 1) break;
-    if (h.iters > 100000)
-      return set_err(ctx, AJG_ERR_DEVICE, "PLOC did not converge");
     batch = 8;
   }
   const uint32_t iters = h.iters;
