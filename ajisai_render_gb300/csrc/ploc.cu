@@ -331,22 +331,34 @@ __device__ __forceinline__ bool ploc_idle(const PlocState& s) {
   return s.cnt <= kTail || s.stuck;
 }
 
-// Nearest neighbour of box k within [s0, s1) of `box` (SoA, `stride` floats a
-// plane; ploc_aggregate.cpp:408-459): in ascending order with a strict
-// comparison.  0xffffffff: none.
-__device__ __forceinline__ uint32_t nearest(const float* box, uint32_t stride,
-                                            uint32_t k, uint32_t s0,
-                                            uint32_t s1) {
-  const F3 ilo = mk3(box[k], box[stride + k], box[2 * stride + k]);
-  const F3 ihi = mk3(box[3 * stride + k], box[4 * stride + k], box[5 * stride + k]);
+// A cluster's box in shared memory: lo.xy, (lo.z, hi.x), hi.yz.  Neighbouring
+// lanes' boxes are 6 words apart, so a half warp's 8-byte loads hit different
+// banks, and a candidate is three loads at constant offsets.  (A plane per
+// coordinate is six loads with an address each: 100,000 clusters of 33
+// candidates 12 -> 10.6 us, of 2,049 470 -> 405.)
+struct Box6 {
+  float2 a, b, c;
+  __device__ __forceinline__ F3 lo() const { return mk3(a.x, a.y, b.x); }
+  __device__ __forceinline__ F3 hi() const { return mk3(b.y, c.x, c.y); }
+};
+__device__ __forceinline__ Box6 box6(const PNode& n) {
+  return Box6{make_float2(n.a.x, n.a.y), make_float2(n.a.z, n.b.x),
+              make_float2(n.b.y, n.b.z)};
+}
+
+// Nearest neighbour of box k within [s0, s1) of `box`
+// (ploc_aggregate.cpp:408-459): in ascending order with a strict comparison.
+// 0xffffffff: none.
+__device__ __forceinline__ uint32_t nearest(const Box6* box, uint32_t k,
+                                            uint32_t s0, uint32_t s1) {
+  const F3 ilo = box[k].lo(), ihi = box[k].hi();
   float best = FLT_MAX;
   uint32_t bj = 0xffffffffu;
   for (uint32_t j = s0; j < s1; ++j) {
     if (j == k) continue;
+    const Box6 o = box[j];
     F3 lo, hi;
-    join(ilo, ihi, mk3(box[j], box[stride + j], box[2 * stride + j]),
-         mk3(box[3 * stride + j], box[4 * stride + j], box[5 * stride + j]), lo,
-         hi);
+    join(ilo, ihi, o.lo(), o.hi(), lo, hi);
     const float d = area(lo, hi);
     if (d < best) {
       best = d;
@@ -359,39 +371,34 @@ __device__ __forceinline__ uint32_t nearest(const float* box, uint32_t stride,
 __global__ void __launch_bounds__(kClusterThreads)
     k_neighbors(const PlocState* __restrict__ st, const PNode* __restrict__ a,
                 const PNode* __restrict__ b, int r, uint32_t* __restrict__ nb) {
-  extern __shared__ float sb[];
+  extern __shared__ Box6 sb[];
   const PlocState s = *st;
   if (ploc_idle(s)) return;
   const PNode* __restrict__ in = s.buf ? b : a;
-  const uint32_t stride = kClusterThreads + 2 * (uint32_t)r;
   for (uint32_t i0 = blockIdx.x * kClusterThreads; i0 < s.cnt;
        i0 += gridDim.x * kClusterThreads) {
     const uint32_t lo_idx = i0 > (uint32_t)r ? i0 - r : 0u;
     const uint32_t hi_idx = min(i0 + kClusterThreads + (uint32_t)r, s.cnt);
     __syncthreads();
-    for (uint32_t k = threadIdx.x; k < hi_idx - lo_idx; k += blockDim.x) {
-      const float4 lo = in[lo_idx + k].a, hi = in[lo_idx + k].b;
-      sb[k] = lo.x;
-      sb[stride + k] = lo.y;
-      sb[2 * stride + k] = lo.z;
-      sb[3 * stride + k] = hi.x;
-      sb[4 * stride + k] = hi.y;
-      sb[5 * stride + k] = hi.z;
-    }
+    for (uint32_t k = threadIdx.x; k < hi_idx - lo_idx; k += blockDim.x)
+      sb[k] = box6(in[lo_idx + k]);
     __syncthreads();
     const uint32_t i = i0 + threadIdx.x;
     if (i >= s.cnt) continue;
     const uint32_t s0 = i > (uint32_t)r ? i - r : 0u;
     const uint32_t s1 = min(i + (uint32_t)r + 1, s.cnt);
-    const uint32_t j = nearest(sb, stride, i - lo_idx, s0 - lo_idx, s1 - lo_idx);
+    const uint32_t j = nearest(sb, i - lo_idx, s0 - lo_idx, s1 - lo_idx);
     nb[i] = j == 0xffffffffu ? j : j + lo_idx;
   }
 }
 
-// mate[i]: the cluster i merges with, or i itself.
+// mate[i]: the cluster i merges with, or i itself; rank[i]: the merges of i's
+// tile up to and with i (a merge counts at its first cluster).
 __global__ void __launch_bounds__(kClusterThreads)
     k_pairs(PlocState* st, int cur, const uint32_t* __restrict__ nb,
-            uint32_t* __restrict__ mate, uint32_t* tile_sum, uint32_t* ticket) {
+            uint32_t* __restrict__ mate, uint16_t* __restrict__ rank,
+            uint32_t* tile_sum, uint32_t* ticket) {
+  __shared__ uint32_t s_count[kPairItems][kClusterThreads / 32];
   __shared__ uint32_t s_warp[kClusterThreads / 32];
   __shared__ uint32_t s_run;
   const PlocState s = st[cur];
@@ -401,27 +408,37 @@ __global__ void __launch_bounds__(kClusterThreads)
   }
   const uint32_t tiles = (s.cnt + kPairTile - 1) / kPairTile;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned le = 0xffffffffu >> (31 - lane);
   for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-    uint32_t c = 0;
+    uint32_t in_warp[kPairItems];
+    __syncthreads();
 #pragma unroll
     for (int k = 0; k < kPairItems; ++k) {
       const uint32_t i = t * kPairTile + k * kClusterThreads + threadIdx.x;
+      bool merges = false;
       if (i < s.cnt) {
         const uint32_t j = nb[i];
         const bool mutual = j != 0xffffffffu && nb[j] == i;
         mate[i] = mutual ? j : i;
-        c += mutual && i < j;
+        merges = mutual && i < j;
       }
+      const unsigned bal = __ballot_sync(0xffffffffu, merges);
+      in_warp[k] = __popc(bal & le);
+      if (lane == 0) s_count[k][warp] = __popc(bal);
     }
-    c = __reduce_add_sync(0xffffffffu, c);
     __syncthreads();
-    if (lane == 0) s_warp[warp] = c;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      uint32_t sum = 0;
-      for (int w = 0; w < kClusterThreads / 32; ++w) sum += s_warp[w];
-      tile_sum[t] = sum;
+    uint32_t run = 0;
+#pragma unroll
+    for (int k = 0; k < kPairItems; ++k) {
+      const uint32_t i = t * kPairTile + k * kClusterThreads + threadIdx.x;
+      uint32_t before = run;
+      for (int w = 0; w < kClusterThreads / 32; ++w) {
+        if (w < warp) before += s_count[k][w];
+        run += s_count[k][w];
+      }
+      if (i < s.cnt) rank[i] = (uint16_t)(before + in_warp[k]);
     }
+    if (threadIdx.x == 0) tile_sum[t] = run;
   }
   // the last block scans the tiles' merges in place (exclusive)
   __threadfence();
@@ -475,58 +492,38 @@ __device__ __forceinline__ PNode merged_node(const PNode& ni, const PNode& nj,
   return p;
 }
 
+// (A cluster's rank is read, not counted over the clusters up to its mate, which
+// is up to the search radius away.  100,000 clusters, counted: 78 us an
+// iteration at a radius of 1,024 and 15 at 16; read: 6 at both.)
 __global__ void __launch_bounds__(kClusterThreads)
     k_cluster(const PlocState* __restrict__ st, int cur, PNode* a, PNode* b,
               const uint32_t* __restrict__ mate,
+              const uint16_t* __restrict__ rank,
               const uint32_t* __restrict__ tile_sum, PNode* __restrict__ nodes,
               SahTable sah) {
-  __shared__ uint32_t s_warp[kPairItems][kClusterThreads / 32];
   const PlocState s = st[cur];
   if (ploc_idle(s)) return;
   const uint32_t first = st[cur ^ 1].end;  // this iteration's nodes start here
   if (st[cur ^ 1].stuck) return;
   const PNode* in = s.buf ? b : a;
   PNode* out = s.buf ? a : b;
-  const uint32_t tiles = (s.cnt + kPairTile - 1) / kPairTile;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned le = 0xffffffffu >> (31 - lane);
-  for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-    uint32_t m[kPairItems], in_warp[kPairItems];
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kPairItems; ++k) {
-      const uint32_t i = t * kPairTile + k * kClusterThreads + threadIdx.x;
-      m[k] = i < s.cnt ? mate[i] : i;
-      const unsigned bal = __ballot_sync(0xffffffffu, m[k] > i);
-      in_warp[k] = __popc(bal & le);
-      if (lane == 0) s_warp[k][warp] = __popc(bal);
-    }
-    __syncthreads();
-    uint32_t run = tile_sum[t];
-#pragma unroll
-    for (int k = 0; k < kPairItems; ++k) {
-      const uint32_t i = t * kPairTile + k * kClusterThreads + threadIdx.x;
-      uint32_t before = run;
-      for (int w = 0; w < kClusterThreads / 32; ++w) {
-        if (w < warp) before += s_warp[k][w];
-        run += s_warp[k][w];
-      }
-      if (i >= s.cnt) continue;
-      const uint32_t mi = before + in_warp[k];  // merges up to and with i
-      const uint32_t j = m[k];
-      if (j == i) {
-        out[i - mi] = in[i];
-      } else if (j > i) {
-        const uint32_t fc = first + (mi - 1) * 2;
-        uint32_t mj = mi;  // merges up to and with j (at most r further)
-        for (uint32_t k2 = i + 1; k2 <= j; ++k2) mj += mate[k2] > k2;
-        const PNode ni = in[i], nj = in[j];
-        out[j - mj] = merged_node(ni, nj, fc);
-        nodes[fc] = ni;
-        nodes[fc + 1] = nj;
-        sah_node(sah, fc, ni);
-        sah_node(sah, fc + 1, nj);
-      }
+  // merges up to and with cluster i
+  auto merges = [&](uint32_t i) { return tile_sum[i / kPairTile] + rank[i]; };
+  for (uint32_t i = blockIdx.x * kClusterThreads + threadIdx.x; i < s.cnt;
+       i += gridDim.x * kClusterThreads) {
+    const uint32_t j = mate[i];
+    if (j < i) continue;
+    const uint32_t mi = merges(i);
+    if (j == i) {
+      out[i - mi] = in[i];
+    } else {
+      const uint32_t fc = first + (mi - 1) * 2;
+      const PNode ni = in[i], nj = in[j];
+      out[j - merges(j)] = merged_node(ni, nj, fc);
+      nodes[fc] = ni;
+      nodes[fc + 1] = nj;
+      sah_node(sah, fc, ni);
+      sah_node(sah, fc + 1, nj);
     }
   }
 }
@@ -535,7 +532,7 @@ __global__ void __launch_bounds__(kClusterThreads)
 // shared memory, a barrier where the other kernels end.  Runs no more
 // iterations than there are clusters (each merges a pair or stops).
 struct TailMem {
-  float box[6][kTail];
+  Box6 box[kTail];
   int first[kTail], count[kTail];
   uint32_t nb[kTail], mi[kTail];
   uint32_t warp[kTailThreads / 32];
@@ -552,21 +549,15 @@ __global__ void __launch_bounds__(kTailThreads)
   const uint32_t tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
   auto put = [&](uint32_t k, const PNode& x) {
-    m.box[0][k] = x.a.x;
-    m.box[1][k] = x.a.y;
-    m.box[2][k] = x.a.z;
-    m.box[3][k] = x.b.x;
-    m.box[4][k] = x.b.y;
-    m.box[5][k] = x.b.z;
+    m.box[k] = box6(x);
     m.first[k] = __float_as_int(x.a.w);
     m.count[k] = __float_as_int(x.b.w);
   };
   auto get = [&](uint32_t k) {
+    const F3 lo = m.box[k].lo(), hi = m.box[k].hi();
     PNode x;
-    x.a = make_float4(m.box[0][k], m.box[1][k], m.box[2][k],
-                      __int_as_float(m.first[k]));
-    x.b = make_float4(m.box[3][k], m.box[4][k], m.box[5][k],
-                      __int_as_float(m.count[k]));
+    x.a = make_float4(lo.x, lo.y, lo.z, __int_as_float(m.first[k]));
+    x.b = make_float4(hi.x, hi.y, hi.z, __int_as_float(m.count[k]));
     return x;
   };
   for (uint32_t k = tid; k < s.cnt; k += kTailThreads) put(k, in[k]);
@@ -574,7 +565,7 @@ __global__ void __launch_bounds__(kTailThreads)
   while (s.cnt > 1) {
     for (uint32_t i = tid; i < s.cnt; i += kTailThreads) {
       const uint32_t s0 = i > (uint32_t)r ? i - r : 0u;
-      m.nb[i] = nearest(&m.box[0][0], kTail, i, s0, min(i + (uint32_t)r + 1, s.cnt));
+      m.nb[i] = nearest(m.box, i, s0, min(i + (uint32_t)r + 1, s.cnt));
     }
     __syncthreads();
     // merges up to and with each cluster (a thread holds kPer in a row)
@@ -1231,6 +1222,7 @@ int build_scene(ajg_ctx* ctx, ajg_scene* s, const float* h_tris,
 
   float* d_tris;
   int32_t *d_mat, *d_flags, *va, *vb, *owner = nullptr;
+  uint16_t* rank;
   uint32_t *ka, *kb, *hist, *scratch, *pos_of = nullptr, *acc, *nbr, *mate, *tile_sum,
       *flags = nullptr, *mi = nullptr, *choice = nullptr, *wc = nullptr;
   PNode *na, *nbuf;
@@ -1261,6 +1253,7 @@ int build_scene(ajg_ctx* ctx, ajg_scene* s, const float* h_tris,
     nbuf = carve<PNode>(cur, n);
     nbr = carve<uint32_t>(cur, n);
     mate = carve<uint32_t>(cur, n);
+    rank = carve<uint16_t>(cur, n);
     tile_sum = carve<uint32_t>(cur, (n + kPairTile - 1) / kPairTile);
     state = carve<PlocState>(cur, 2);
     if (!wide || hybrid) {
@@ -1348,7 +1341,7 @@ int build_scene(ajg_ctx* ctx, ajg_scene* s, const float* h_tris,
   const SahTable table{cost, choice};
   k_leaf_init<<<gb, 256, 0, st>>>(d_tris, perm, na, n);
   k_ploc_start<<<1, 1, 0, st>>>(state, (uint32_t)n, acc);
-  const size_t smem = (size_t)(kClusterThreads + 2 * r) * 6 * sizeof(float);
+  const size_t smem = (size_t)(kClusterThreads + 2 * r) * sizeof(Box6);
   if (smem > 48 * 1024)
     cudaFuncSetAttribute(k_neighbors,
                          cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1365,9 +1358,10 @@ int build_scene(ajg_ctx* ctx, ajg_scene* s, const float* h_tris,
     for (int k = 0; k < batch; ++k, ++it) {
       const int cur = (int)(it & 1);
       k_neighbors<<<g_nb, kClusterThreads, smem, st>>>(state + cur, na, nbuf, r, nbr);
-      k_pairs<<<g_pair, kClusterThreads, 0, st>>>(state, cur, nbr, mate, tile_sum, acc);
-      k_cluster<<<g_pair, kClusterThreads, 0, st>>>(state, cur, na, nbuf, mate,
-                                                    tile_sum, nodes, table);
+      k_pairs<<<g_pair, kClusterThreads, 0, st>>>(state, cur, nbr, mate, rank,
+                                                  tile_sum, acc);
+      k_cluster<<<g_nb, kClusterThreads, 0, st>>>(state, cur, na, nbuf, mate, rank,
+                                                  tile_sum, nodes, table);
     }
     k_cluster_tail<<<1, kTailThreads, sizeof(TailMem), st>>>(
         state, (int)(it & 1), na, nbuf, r, nodes, table);
