@@ -121,7 +121,7 @@ __device__ __forceinline__ bool mt_test(const RayQ& r, float4 A, float4 B,
 // sum and the scaled distance exactly: the sign test is symmetric, and t and
 // the barycentrics are the quotients, so the winding needs no axis swap.
 // (Six selects a vertex by the axes' numbers, and their comparisons: closest
-// hits of 853x479x16 paths over 9,002 triangles: 8.51 ms, so 7.67.)
+// hits of 853x479x16 paths over 108,014 triangles: 8.51 ms, so 7.67.)
 struct WtSetup {
   bool zx, zy;  // kz is x, is y
   float sx, sy, sz;
@@ -322,7 +322,7 @@ constexpr int trace_min_blocks() {
 // empty, so closest hits run beside any hits on one SM only if both ask for
 // the same; with 16 entries and each kernel's own size (164 and 100 KB) they
 // shared the chip by SMs.  16 entries and no request -> 8 entries and this
-// one: a 64x48x4 box 433 -> 424 us, 1024x1024x32 over 1.3 M triangles 63.3 ->
+// one: a 128x128x1 box 433 -> 424 us, 1024x1024x32 over 1.3 M triangles 63.3 ->
 // 62.5 ms, the material box 4.59 -> 4.49 ms, 16 batched jobs 50.7 -> 50.3 ms.
 // 64 KB holds too few blocks (+6% over the triangles), larger ones leave less
 // cache (132 KB +0.3%, 196 KB +2%); 4 entries spill too often (+1%); and the
