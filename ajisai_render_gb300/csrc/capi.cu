@@ -307,6 +307,8 @@ int ajg_destroy_context(ajg_ctx* ctx) {
   cudaStreamSynchronize(ctx->trace_stream);
   cudaEventDestroy(ctx->ev_queue);
   cudaEventDestroy(ctx->ev_hits);
+  for (cudaEvent_t e : ctx->ev_build)
+    if (e) cudaEventDestroy(e);
   cudaStreamDestroy(ctx->trace_stream);
   cudaStreamDestroy(ctx->stream);
   delete ctx;

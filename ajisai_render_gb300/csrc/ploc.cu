@@ -1128,6 +1128,28 @@ struct ShadingCopy {
   }
 };
 
+// The GPU time of a build: the spans between begin and end, which leave out the
+// copies in and the host's share (from pageable memory the copies of the
+// shading arrays hold the host, and the stream waits for both).
+struct BuildTimer {
+  ajg_ctx* ctx;
+  int n = 0;  // events recorded
+  explicit BuildTimer(ajg_ctx* c) : ctx(c) {
+    for (cudaEvent_t& e : ctx->ev_build)
+      if (!e) cudaEventCreate(&e);
+  }
+  void mark() { cudaEventRecord(ctx->ev_build[n++], ctx->stream); }
+  float ms() const {
+    float sum = 0.f;
+    for (int k = 0; k + 1 < n; k += 2) {
+      float t = 0.f;
+      cudaEventElapsedTime(&t, ctx->ev_build[k], ctx->ev_build[k + 1]);
+      sum += t;
+    }
+    return sum;
+  }
+};
+
 int set_err(ajg_ctx* ctx, int code, const std::string& msg) {
   ctx->last_error = msg;
   return code;
@@ -1280,13 +1302,11 @@ int build_scene(ajg_ctx* ctx, ajg_scene* s, const float* h_tris,
   temporaries(tmp.p);
   ShadingCopy shading(ctx);
 
-  cudaEvent_t e0, e1;
-  cudaEventCreate(&e0);
-  cudaEventCreate(&e1);
+  BuildTimer timer(ctx);
   cudaMemcpyAsync(d_tris, h_tris, n * 9 * sizeof(float),
                   cudaMemcpyHostToDevice, st);
   cudaMemsetAsync(ctx->d_error, 0, sizeof(uint32_t), st);
-  cudaEventRecord(e0, st);
+  timer.mark();
 
   // MortonEncoder (ploc_aggregate.cpp:61-66): grid = 1024 / size, offset =
   // -min * grid, all in float
@@ -1366,14 +1386,17 @@ int build_scene(ajg_ctx* ctx, ajg_scene* s, const float* h_tris,
     }
     k_cluster_tail<<<1, kTailThreads, sizeof(TailMem), st>>>(
         state, (int)(it & 1), na, nbuf, r, nodes, table);
-    if (!shading.started)  // beside the clustering
+    if (!shading.started) {  // beside the clustering
+      timer.mark();
       shading.start(d_mat, h_mat, d_flags, h_flags, corner, h_corner, n);
+    }
     cudaError_t e = cudaMemcpyAsync(&h, state + (it & 1), sizeof(h),
                                     cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess)
       return set_err(ctx, AJG_ERR_CUDA,
                      std::string("PLOC build: ") + cudaGetErrorString(e));
+    if (timer.n == 2) timer.mark();
     if (h.iters > kMaxIterations)  // ended or not: the last batch and the
                                    // tail do not stop at the limit
       return set_err(ctx, AJG_ERR_DEVICE, "PLOC did not converge");
@@ -1463,18 +1486,17 @@ int build_scene(ajg_ctx* ctx, ajg_scene* s, const float* h_tris,
                       cudaMemcpyDeviceToDevice, st);
   }
   if (width == 2) k_slot_tris<<<gb, 256, 0, st>>>(d_tris, perm, n, slot_tris);
+  timer.mark();
   cudaStreamWaitEvent(st, ctx->ev_queue, 0);
+  timer.mark();
   k_shade_data<<<gb, 256, 0, st>>>(d_tris, d_mat, d_flags, n, shade);
-  cudaEventRecord(e1, st);
+  timer.mark();
   cudaError_t ce = cudaStreamSynchronize(st);
   uint32_t derr = 0;
   if (ce == cudaSuccess)
     ce = cudaMemcpy(&derr, ctx->d_error, sizeof(uint32_t),
                     cudaMemcpyDeviceToHost);
-  float ms = 0.f;
-  cudaEventElapsedTime(&ms, e0, e1);
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
+  const float ms = timer.ms();
   if (ce != cudaSuccess)
     return set_err(ctx, AJG_ERR_CUDA,
                    std::string("PLOC build: ") + cudaGetErrorString(ce));

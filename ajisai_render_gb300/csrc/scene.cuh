@@ -337,6 +337,7 @@ struct ajg_ctx {
   // stream
   cudaStream_t trace_stream = nullptr;
   cudaEvent_t ev_queue = nullptr, ev_hits = nullptr;
+  cudaEvent_t ev_build[6] = {};  // a scene build's spans (made with the first)
   bool overlap = true;
   // single jobs without emitters over the plain 4-wide tree: the light terms
   // of bounce 0 whose shadow rays are traced as masked packets

@@ -225,7 +225,7 @@ typedef struct ajg_scene_info {
   uint64_t num_nodes;      /* 2n-1 PLOC nodes */
   uint64_t device_bytes;   /* resident bytes of the scene */
   uint32_t ploc_iterations;
-  float build_ms;          /* GPU time of the last PLOC build */
+  float build_ms;          /* GPU time of the last PLOC build (no copies in) */
   uint32_t bvh_width;      /* node width of the traversal tree */
   uint32_t bvh_node_bytes; /* bytes per traversal node */
   uint64_t bvh_nodes;      /* traversal nodes */
